@@ -175,7 +175,9 @@ int plan_beamform(rcabf_geometry *g, const rcabf_beamform_args *a, Plan &p, cons
         p.tiles_u = (int)((g->n_u + p.ts.tu - 1) / p.ts.tu);
         p.tiles_v = (int)((g->n_v + tile_v_extent - 1) / tile_v_extent);
         p.row_words = fused_row_words(p.fb);
-        p.slab_bytes = ((int64_t)(p.tc ? p.tc_rows : a->n_sample) * p.fb * es + 15) / 16 * 16;
+        p.slab_bytes = p.vb == 1 ? (a->n_sample + VBS_PAD_ROWS) * vbs_row_bytes(p.fb)
+                                 : (int64_t)(p.tc ? p.tc_rows : a->n_sample) * p.fb * es;
+        p.slab_bytes = (p.slab_bytes + 15) / 16 * 16;
         auto al = [](size_t x) { return (x + 255) / 256 * 256; };
         size_t off = 0;
         p.off_S = off;
@@ -186,8 +188,15 @@ int plan_beamform(rcabf_geometry *g, const rcabf_beamform_args *a, Plan &p, cons
         off += al((size_t)g->n_ele * p.tiles_u * p.tiles_z * sizeof(float2));
         p.off_txr = off;
         off += al((size_t)g->n_tx * p.tiles_v * p.tiles_z * sizeof(float2));
-        p.total = off;
         p.n_items = (int64_t)p.n_fb * p.tiles_z * p.tiles_u * p.tiles_v;
+        if (p.vb == 1) {   // streaming kernel: items per transmit range, its work counter
+            p.n_items *= p.n_split;
+            p.off_ctr = off;
+            off += al(sizeof(uint32_t));
+            p.off_part = off;
+            if (a->compound && p.n_split > 1) off += al((size_t)p.n_split * a->n_frame * g->n_pix * sizeof(float2));
+        }
+        p.total = off;
     };
 
     // Tensor-core kernel: FP16 slabs (BF16 slabs with hi + remainder weights),
@@ -251,59 +260,90 @@ int plan_beamform(rcabf_geometry *g, const rcabf_beamform_args *a, Plan &p, cons
         p.store = a->storage;
     }
 
-    // Voxel-blocked kernel: exact tables, a steering axis to block along,
-    // frames in pairs, and at most 2 rows of shift inside a block.  Its
-    // accumulators live in registers (vb = 1) or, for frame blocks of 8 and
-    // 16, in tensor memory (vb = 2).
+    // Voxel-blocked kernels: exact tables and a steering axis to block along.
+    //   vb = 1: register accumulators, windows streamed ahead by bulk copies.
+    //     The four voxels of a thread share their sample rows where a block
+    //     spreads over at most 2 of them (d = 1, 2); single frames and wider
+    //     spreads have every voxel read its own (d = 0).
+    //   vb = 2: accumulators in tensor memory, for frame blocks of 16 that
+    //     registers hold only with spills, at d = 1, 2.
     const int want_vb = force ? force->vb
                         : a->kernel == RCABF_KERNEL_FUSED_TMEM ? 2
                         : a->kernel == RCABF_KERNEL_FUSED_REGS ? 1
                                                                : 0;   // 0: the planner's choice
+    const bool named = !force && want_vb > 0;   // by name: row-sharing blocks of 2 frames or more only
     const bool vb_fb_ok = force ? force->vb >= 1
-                                : fb_req == 0 ? a->n_frame >= 2
-                                              : (fb_req == 2 || fb_req == 4 || fb_req == 8 || fb_req == 16);
-    if (g->mode == MODE_EXACT && vb_fb_ok && a->kernel != RCABF_KERNEL_FUSED_NOBLOCK) {
-        const int d = g->vb_shift(VB_BLOCK);
-        if (d >= 1 && d <= 2) {
-            const int tu = std::min(4, pow2_ceil(g->n_u));
-            const int tvb = 2;
-            TileShape vts{tu, tvb, VB_THREADS_HOST / (tu * tvb)};
-            if (force) {
-                if (force->ts.tu * force->ts.tv * force->ts.tz != VB_THREADS_HOST) return RCABF_ERR_UNSUPPORTED;
-                vts = force->ts;
+                                : fb_req == 0 ? (!named || a->n_frame >= 2)
+                                              : (fb_req == 2 || fb_req == 4 || fb_req == 8 || fb_req == 16 ||
+                                                 (!named && fb_req == 1));
+    const int shift = g->mode == MODE_EXACT && vb_fb_ok && a->kernel != RCABF_KERNEL_FUSED_NOBLOCK
+                          ? g->vb_shift(VB_BLOCK) : -1;
+    if (shift >= 1 && (shift <= 2 || !named)) {
+        const int tu = std::min(4, pow2_ceil(g->n_u));
+        const int tvb = 2;
+        TileShape vts{tu, tvb, VB_THREADS_HOST / (tu * tvb)};
+        if (force) {
+            if (force->ts.tu * force->ts.tv * force->ts.tz != VB_THREADS_HOST) return RCABF_ERR_UNSUPPORTED;
+            vts = force->ts;
+        }
+        const int rows = g->window_rows(TileShape{vts.tu, vts.tv * VB_BLOCK, vts.tz});
+        // streaming kernel: a grid of few tiles is split by transmits until
+        // there are two items per resident CTA (a number that depends on the
+        // grid alone, not on frames: the split sets the order of the sums)
+        const int64_t tiles = ((g->n_z + vts.tz - 1) / vts.tz) * ((g->n_u + vts.tu - 1) / vts.tu) *
+                              ((g->n_v + vts.tv * VB_BLOCK - 1) / (vts.tv * VB_BLOCK));
+        const int split = !a->compound ? g->n_tx
+                          : named ? 1
+                                  : (int)std::min<int64_t>(g->n_tx, (VBS_MIN_ITEMS + tiles - 1) / tiles);
+        auto fits = [&](int vb, int d, int fb) {   // the largest window of the acquisition in its staging buffer
+            const int need = (int)std::min<int64_t>(rows + std::max(d, 1), a->n_sample + d);
+            if (vb == 1)
+                return a->n_sample <= VBS_MAX_SAMPLES && vbs_chunk_records(fb, need) >= 1;
+            return need <= std::min<int>((int)(VB_SMEM_BUDGET / ((size_t)fused_stages(p.store) * fused_row_words(fb) * 4)),
+                                         vb_stage_rows_cap(p.store, fb));
+        };
+        auto pick = [&](int vb, int d) {   // the frame block, 0: none
+            if (vb == 2 && d == 0) return 0;
+            for (int c : {16, 8, 4, 2, 1}) {
+                if (d > 0 && c == 1) continue;
+                if (force ? c != force->fb : fb_req > 0 && c != fb_req) continue;
+                // the planner's choice: at most the frame count rounded up to a
+                // power of two (a block more than half empty costs more than
+                // the setup it saves); a store asked for by name may pad to 2x
+                const int64_t lim = want_vb ? 2 * a->n_frame : pow2_ceil(a->n_frame);
+                if (!force && fb_req == 0 && c > lim) continue;
+                // register accumulators: blocks of 8 at most (16 spill), but by name,
+                // and where every frame block has to keep one order of sums
+                if (vb == 1 && c == 16 && !want_vb && !(fb_req == 16 && (split > 1 || d == 0))) continue;
+                if (fits(vb, d, c)) return c;
             }
-            const int need = (int)std::min<int64_t>(
-                g->window_rows(TileShape{vts.tu, vts.tv * VB_BLOCK, vts.tz}) + d, a->n_sample);
-            auto pick_fb = [&](int tm) {   // the largest frame block whose window fits
-                for (int c : {16, 8, 4, 2}) {
-                    if (force && c != force->fb) continue;
-                    if (!force && fb_req > 0 && c != fb_req) continue;
-                    // the planner's choice: at most the frame count rounded up to a
-                    // power of two (a block more than half empty costs more than
-                    // the setup it saves: per item t ~ setup + FB x frame cost,
-                    // setup ~ 13 frames); a store asked for by name may pad to 2x
-                    const int64_t lim = want_vb ? 2 * a->n_frame : pow2_ceil(a->n_frame);
-                    if (!force && fb_req == 0 && c > lim) continue;
-                    const int cap = std::min<int>((int)(VB_SMEM_BUDGET / ((size_t)fused_stages(p.store) *
-                                                                           fused_row_words(c) * 4)),
-                                                  vb_stage_rows_cap(p.store, c));
-                    if (cap >= need) return c;
-                }
-                return 0;
-            };
-            int tm = want_vb == 2 ? 1 : want_vb == 1 ? 0 : VB_TMEM_DEFAULT;
-            int fb = pick_fb(tm);
-            if (!fb && tm && want_vb == 0) fb = pick_fb(tm = 0);   // blocks below 8 frames: registers
-            if (fb) {
-                p.vb = tm ? 2 : 1;
-                p.d = d;
-                p.fb = fb;
-                p.ts = vts;
-                layout(vts.tv * VB_BLOCK);
-                p.wmax = need;
-                p.smem = vb_smem_bytes(p.store, p.wmax, p.row_words, tm ? kind_taps(g->kind) + d : 0);
+            return 0;
+        };
+        const bool single = force ? force->fb == 1 : fb_req == 1 || (fb_req == 0 && a->n_frame == 1);
+        int vb = 0, d = shift <= 2 && !single ? shift : 0, fb = 0;
+        if (want_vb) {
+            fb = pick(vb = want_vb, d);
+            if (!fb && want_vb == 1 && a->n_sample > VBS_MAX_SAMPLES && d) fb = pick(vb = 2, d);   // the same bits
+        } else {
+            fb = pick(vb = 1, d);
+            if (!fb) fb = pick(vb = 2, d);
+        }
+        if (fb) {
+            p.vb = vb;
+            p.d = d;
+            p.fb = fb;
+            p.ts = vts;
+            p.wmax = (int)std::min<int64_t>(rows + std::max(d, 1), a->n_sample + d);
+            if (vb == 1) p.n_split = split;
+            layout(vts.tv * VB_BLOCK);
+            if (p.n_items < INT32_MAX) {
+                p.smem = vb == 1 ? vbs_smem_bytes(fb, p.wmax)
+                                 : vb_smem_bytes(p.store, p.wmax, p.row_words, kind_taps(g->kind) + d);
                 return RCABF_OK;
             }
+            p = Plan{};
+            p.kernel = RCABF_KERNEL_FUSED;
+            p.store = a->storage;
         }
     }
     if (want_vb) return RCABF_ERR_UNSUPPORTED;
@@ -329,34 +369,69 @@ int plan_beamform(rcabf_geometry *g, const rcabf_beamform_args *a, Plan &p, cons
     return RCABF_OK;
 }
 
+// Replaces the planner's own choice of the streaming kernel by one with a
+// smaller workspace, where there is one: slabs in the storage type, staged by
+// the voxel-blocked kernel with tensor-memory accumulators or by the
+// one-voxel-per-thread kernel.  Sets a.kernel to it.
+void plan_compact(rcabf_geometry *g, rcabf_beamform_args &a, Plan &p)
+{
+    if (a.kernel != RCABF_KERNEL_AUTO && a.kernel != RCABF_KERNEL_FUSED) return;
+    rcabf_beamform_args c = a;
+    for (int32_t k : {RCABF_KERNEL_FUSED_TMEM, RCABF_KERNEL_FUSED_NOBLOCK}) {
+        Plan q;
+        c.kernel = k;
+        if (plan_beamform(g, &c, q) == RCABF_OK && q.kernel == RCABF_KERNEL_FUSED && q.total < p.total) {
+            p = q;
+            a.kernel = k;
+            return;
+        }
+    }
+}
+
 static void mark(const rcabf_beamform_args *a, int i, cudaStream_t st)
 {
     if (a->stage_events && a->stage_events[i]) cudaEventRecord((cudaEvent_t)a->stage_events[i], st);
 }
 
 // Fills the per-job descriptor and launches the job's ingest and range kernels.
+// (the streaming kernel's: one launch that also writes the mask.)
 int stage_job(rcabf_geometry *g, const rcabf_beamform_args *a, const Plan &p, FusedJob &J, cudaStream_t st,
               const rcabf_beamform_args *marks = nullptr)
 {
     char *ws = reinterpret_cast<char *>(a->workspace);
+    const bool stream = p.vb == 1;
     IngestParams ip{};
     ip.iq = a->iq; ip.iq_dtype = a->iq_dtype; ip.n_sample = (int)a->n_sample; ip.n_ele = g->n_ele;
     ip.n_tx = g->n_tx; ip.n_frame = a->n_frame; ip.fb = p.fb; ip.n_fb = p.n_fb;
     ip.S = ws + p.off_S; ip.slab_bytes = p.slab_bytes; ip.n_rows = p.tc ? p.tc_rows : 0;
     ip.S2 = p.tc ? ws + p.off_S + (size_t)g->n_tx * g->n_ele * p.n_fb * p.slab_bytes : nullptr;
-    cudaError_t ce = launch_ingest(ip, p.store, st);
-    if (ce != cudaSuccess) return cuda_fail(ce, "ingest launch");
-    if (marks) mark(marks, 1, st);
+    cudaError_t ce = cudaSuccess;
+    if (!stream) {
+        if ((ce = launch_ingest(ip, p.store, st)) != cudaSuccess) return cuda_fail(ce, "ingest launch");
+        if (marks) mark(marks, 1, st);
+    }
     RangeParams rr{};
     rr.tab = g->rx_tab; rr.out = reinterpret_cast<float2 *>(ws + p.off_rxr); rr.rows = g->n_ele;
     rr.n_a = g->n_u; rr.n_z = g->n_z; rr.ta = p.ts.tu; rr.tz = p.ts.tz; rr.tiles_a = p.tiles_u;
     rr.tiles_z = p.tiles_z; rr.mode = g->mode; rr.is_rx = 1;
-    if ((ce = launch_range(rr, st)) != cudaSuccess) return cuda_fail(ce, "rx range launch");
     RangeParams tr = rr;
     tr.tab = g->tx_tab; tr.out = reinterpret_cast<float2 *>(ws + p.off_txr); tr.rows = g->n_tx;
     tr.n_a = g->n_v; tr.ta = p.vb ? p.ts.tv * VB_BLOCK : p.ts.tv; tr.tiles_a = p.tiles_v; tr.is_rx = 0;
-    if ((ce = launch_range(tr, st)) != cudaSuccess) return cuda_fail(ce, "tx range launch");
-    g_launches += 3;
+    if (stream) {
+        PrepParams pp{};
+        pp.ingest = ip;
+        pp.ingest.n_rows = (int)a->n_sample + VBS_PAD_ROWS;
+        pp.rx = rr; pp.tx = tr; pp.g = g->dev(); pp.mask = a->mask;
+        pp.compound = a->compound ? 1 : 0; pp.accumulate = a->accumulate ? 1 : 0;
+        pp.counter = reinterpret_cast<uint32_t *>(ws + p.off_ctr);
+        if ((ce = launch_prep(pp, p.store, st)) != cudaSuccess) return cuda_fail(ce, "preparation launch");
+        if (marks) mark(marks, 1, st);
+        g_launches += 1;
+    } else {
+        if ((ce = launch_range(rr, st)) != cudaSuccess) return cuda_fail(ce, "rx range launch");
+        if ((ce = launch_range(tr, st)) != cudaSuccess) return cuda_fail(ce, "tx range launch");
+        g_launches += 3;
+    }
     if (marks) mark(marks, 2, st);
 
     J = FusedJob{};
@@ -370,6 +445,29 @@ int stage_job(rcabf_geometry *g, const rcabf_beamform_args *a, const Plan &p, Fu
     J.compound = a->compound ? 1 : 0; J.accumulate = a->accumulate ? 1 : 0;
     J.tiles_z = p.tiles_z; J.tiles_u = p.tiles_u; J.tiles_v = p.tiles_v;
     J.tu = p.ts.tu; J.tv = p.ts.tv; J.tz = p.ts.tz;
+    J.n_split = p.n_split;
+    J.partial = reinterpret_cast<float2 *>(ws + p.off_part);
+    return RCABF_OK;
+}
+
+// After the streaming kernel: the sums of a job's transmit ranges into its output.
+static int finish_job(const rcabf_geometry *g, const rcabf_beamform_args *a, const Plan &p, const FusedJob &J,
+                      cudaStream_t st)
+{
+    if (p.vb != 1 || !a->compound || p.n_split <= 1) return RCABF_OK;
+    const cudaError_t e = launch_vbs_reduce(J.out, J.partial, a->n_frame * g->n_pix, p.n_split, J.accumulate, st);
+    if (e != cudaSuccess) return cuda_fail(e, "transmit range sum launch");
+    g_launches += 1;
+    return RCABF_OK;
+}
+
+// The mask, where no earlier launch of the plan has written it.
+static int finish_mask(const rcabf_geometry *g, const rcabf_beamform_args *a, const Plan &p, cudaStream_t st)
+{
+    if (!a->mask || p.vb == 1) return RCABF_OK;
+    const cudaError_t e = launch_mask(g->dev(), a->mask, a->compound ? 1 : 0, a->accumulate ? 1 : 0, st);
+    if (e != cudaSuccess) return cuda_fail(e, "mask kernel launch");
+    g_launches += 1;
     return RCABF_OK;
 }
 
@@ -377,21 +475,23 @@ int stage_job(rcabf_geometry *g, const rcabf_beamform_args *a, const Plan &p, Fu
 // shared memory (sets the kernel's shared-memory limit on first use).
 static int resident_ctas(const rcabf_geometry *g0, const Plan &p, size_t smem, DeviceState *ds, int &occ)
 {
-    // variant: (mode, or 2 vb + row shift for the voxel-blocked kernels; kind; fb; store)
-    const std::array<int64_t, 4> var{p.vb ? 2 * p.vb + p.d : g0->mode, g0->kind, p.fb, p.store};
+    // variant: (mode, or 4 vb + row shift for the voxel-blocked kernels; kind; fb; store)
+    const std::array<int64_t, 4> var{p.vb ? 4 * p.vb + p.d : g0->mode, g0->kind, p.fb, p.store};
     const std::array<int64_t, 5> key{var[0], var[1], var[2], var[3], (int64_t)smem};
     std::lock_guard<std::mutex> lk(ds->mu);
     auto lim = ds->smem_limit.find(var);
     if (lim == ds->smem_limit.end() || lim->second < smem) {
-        const cudaError_t pe = p.vb ? prepare_fused_vb(g0->kind, p.d, p.vb == 2, p.fb, p.store, smem)
-                                    : prepare_fused(g0->mode, g0->kind, p.fb, p.store, smem);
+        const cudaError_t pe = p.vb == 2   ? prepare_fused_vb(g0->kind, p.d, p.fb, p.store, smem)
+                               : p.vb == 1 ? prepare_fused_vbs(g0->kind, p.d, p.fb, p.store, smem)
+                                           : prepare_fused(g0->mode, g0->kind, p.fb, p.store, smem);
         if (pe != cudaSuccess) return cuda_fail(pe, "fused kernel shared-memory attribute");
         ds->smem_limit[var] = smem;
     }
     auto oc = ds->occ.find(key);
     if (oc == ds->occ.end()) {
-        const int o = p.vb ? fused_vb_occupancy(g0->kind, p.d, p.vb == 2, p.fb, p.store, smem)
-                           : fused_occupancy(g0->mode, g0->kind, p.fb, p.store, smem);
+        const int o = p.vb == 2   ? fused_vb_occupancy(g0->kind, p.d, p.fb, p.store, smem)
+                      : p.vb == 1 ? fused_vbs_occupancy(g0->kind, p.d, p.fb, p.store, smem)
+                                  : fused_occupancy(g0->mode, g0->kind, p.fb, p.store, smem);
         oc = ds->occ.emplace(key, o).first;
     }
     occ = std::max(1, oc->second);
@@ -413,16 +513,18 @@ int launch_fused_jobs(rcabf_geometry *g0, FusedParams &prm, const Plan &p, cudaS
         }
         return RCABF_OK;
     }
-    const size_t smem = p.vb ? vb_smem_bytes(p.store, prm.wmax, prm.row_words,
-                                             p.vb == 2 ? kind_taps(g0->kind) + p.d : 0)
-                             : fused_smem_bytes(g0->mode, g0->kind, p.store, prm.wmax, prm.row_words);
+    const size_t smem = p.vb == 2   ? vb_smem_bytes(p.store, prm.wmax, prm.row_words, kind_taps(g0->kind) + p.d)
+                        : p.vb == 1 ? vbs_smem_bytes(p.fb, prm.wmax)
+                                    : fused_smem_bytes(g0->mode, g0->kind, p.store, prm.wmax, prm.row_words);
+    if (p.vb == 1) prm.krec = vbs_chunk_records(p.fb, prm.wmax);
     int occ = 0;
     const int so = resident_ctas(g0, p, smem, ds, occ);
     if (so != RCABF_OK) return so;
     const int64_t grid = std::min<int64_t>(prm.n_items, (int64_t)ds->n_sm * occ);
     if (grid <= 0) return RCABF_OK;
-    const cudaError_t le = p.vb ? launch_fused_vb(g0->kind, p.d, p.vb == 2, p.fb, p.store, prm, (int)grid, smem, st)
-                                : launch_fused(g0->mode, g0->kind, p.fb, p.store, prm, (int)grid, smem, st);
+    const cudaError_t le = p.vb == 2   ? launch_fused_vb(g0->kind, p.d, p.fb, p.store, prm, (int)grid, smem, st)
+                           : p.vb == 1 ? launch_fused_vbs(g0->kind, p.d, p.fb, p.store, prm, (int)grid, smem, st)
+                                       : launch_fused(g0->mode, g0->kind, p.fb, p.store, prm, (int)grid, smem, st);
     if (le != cudaSuccess) return cuda_fail(le, "fused kernel launch");
     g_launches += 1;
     return RCABF_OK;
@@ -485,14 +587,12 @@ static int beamform_planned(rcabf_geometry *g, const rcabf_beamform_args *a, con
         prm.wmax = p.wmax;
         prm.row_words = p.row_words;
         prm.n_items = p.n_items;
+        prm.counter = reinterpret_cast<uint32_t *>(static_cast<char *>(a->workspace) + p.off_ctr);
         if ((s = launch_fused_jobs(g, prm, p, st)) != RCABF_OK) return s;
+        if ((s = finish_job(g, a, p, prm.jobs[0], st)) != RCABF_OK) return s;
     }
     mark(a, 3, st);
-    if (a->mask) {
-        const cudaError_t me = launch_mask(g->dev(), a->mask, a->compound ? 1 : 0, a->accumulate ? 1 : 0, st);
-        if (me != cudaSuccess) return cuda_fail(me, "mask kernel launch");
-        g_launches += 1;
-    }
+    if ((s = finish_mask(g, a, p, st)) != RCABF_OK) return s;
     mark(a, 4, st);
     return RCABF_OK;
 }
@@ -541,6 +641,10 @@ int beamform_noalloc(rcabf_geometry *g, const rcabf_beamform_args *a, cudaStream
         snprintf(g_last_err, sizeof(g_last_err), "noalloc: the plan is the plain kernel; this entry runs the fused kernel only");
         return RCABF_ERR_UNSUPPORTED;
     }
+    // the streaming kernel's FP32 slabs are up to three times the channel
+    // data in storage type: where they do not fit, the kernels that stage it
+    rcabf_beamform_args b = *a;
+    if (p.vb == 1 && p.total > RCABF_NOALLOC_WORKSPACE_BYTES) plan_compact(g, b, p);
     if (p.total > RCABF_NOALLOC_WORKSPACE_BYTES) {
         snprintf(g_last_err, sizeof(g_last_err),
                  "noalloc: the plan needs %zu workspace bytes; the static workspace holds %zu", p.total,
@@ -549,7 +653,6 @@ int beamform_noalloc(rcabf_geometry *g, const rcabf_beamform_args *a, cudaStream
     }
     NoallocRegion r;
     if ((s = noalloc_setup(g->device, r, true)) != RCABF_OK) return s;
-    rcabf_beamform_args b = *a;
     b.workspace = r.ws;
     b.workspace_bytes = RCABF_NOALLOC_WORKSPACE_BYTES;
     if ((s = check_ptrs(&b, p)) != RCABF_OK) return s;
@@ -562,13 +665,11 @@ int beamform_noalloc(rcabf_geometry *g, const rcabf_beamform_args *a, cudaStream
     prm.row_words = p.row_words;
     prm.n_items = p.n_items;
     prm.err_count = r.err;
+    prm.counter = reinterpret_cast<uint32_t *>(static_cast<char *>(b.workspace) + p.off_ctr);
     if ((s = launch_fused_jobs(g, prm, p, st)) != RCABF_OK) return s;
+    if ((s = finish_job(g, &b, p, prm.jobs[0], st)) != RCABF_OK) return s;
     mark(&b, 3, st);
-    if (b.mask) {
-        const cudaError_t me = launch_mask(g->dev(), b.mask, b.compound ? 1 : 0, b.accumulate ? 1 : 0, st);
-        if (me != cudaSuccess) return cuda_fail(me, "mask kernel launch");
-        g_launches += 1;
-    }
+    if ((s = finish_mask(g, &b, p, st)) != RCABF_OK) return s;
     mark(&b, 4, st);
     return RCABF_OK;
 }
@@ -899,6 +1000,7 @@ int rcabf_beamform_batch(int n, const rcabf_geometry *const *gs, const rcabf_bea
     if (!g0) return RCABF_ERR_BAD_HANDLE;
     FusedParams prm{};
     Plan p0;
+    std::vector<Plan> plans((size_t)n);
     int64_t items = 0;
     int wmax = 0;
     for (int i = 0; i < n; ++i) {
@@ -915,6 +1017,7 @@ int rcabf_beamform_batch(int n, const rcabf_geometry *const *gs, const rcabf_bea
         if (s != RCABF_OK) return s;
         if ((s = check_ptrs(&as[i], p)) != RCABF_OK) return s;
         if (i == 0) p0 = p;
+        plans[i] = p;
         // one launch = one kernel variant: every job fused, same frame block
         if (p.kernel != RCABF_KERNEL_FUSED || p.fb != p0.fb || p.vb != p0.vb || p.d != p0.d)
             return RCABF_ERR_UNSUPPORTED;
@@ -923,17 +1026,17 @@ int rcabf_beamform_batch(int n, const rcabf_geometry *const *gs, const rcabf_bea
         prm.jobs[i].item_begin = items;
         items += p.n_items;
     }
+    if (p0.vb == 1 && items >= INT32_MAX) return RCABF_ERR_UNSUPPORTED;
     prm.n_jobs = n;
     prm.wmax = wmax;
     prm.row_words = p0.row_words;
     prm.n_items = items;
+    prm.counter = reinterpret_cast<uint32_t *>(static_cast<char *>(as[0].workspace) + p0.off_ctr);
     int s = launch_fused_jobs(g0, prm, p0, st);
     if (s != RCABF_OK) return s;
     for (int i = 0; i < n; ++i) {
-        if (!as[i].mask) continue;
-        const cudaError_t me = launch_mask(gs[i]->dev(), as[i].mask, as[i].compound ? 1 : 0, as[i].accumulate ? 1 : 0, st);
-        if (me != cudaSuccess) return cuda_fail(me, "mask kernel launch");
-        g_launches += 1;
+        if ((s = finish_job(gs[i], &as[i], plans[i], prm.jobs[i], st)) != RCABF_OK) return s;
+        if ((s = finish_mask(gs[i], &as[i], plans[i], st)) != RCABF_OK) return s;
     }
     return RCABF_OK;
 }

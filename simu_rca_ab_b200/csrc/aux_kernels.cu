@@ -137,10 +137,9 @@ cudaError_t launch_range(const RangeParams &p, cudaStream_t st)
 // (pixel, tx) (RCA.cu:247-250, 301-304), summed over transmits when
 // compounding (RCA.m:696).
 // ------------------------------------------------------------------------
-__global__ void mask_kernel(const DevGeom g, float *mask, int compound, int accumulate)
+__device__ __forceinline__ void mask_voxel(const DevGeom &g, float *mask, int compound, int accumulate, int64_t v)
 {
     const int64_t n_vox = g.n_z * g.n_u * g.n_v;
-    const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= n_vox) return;
     const int64_t iz = v % g.n_z, iu = (v / g.n_z) % g.n_u, iv = v / (g.n_z * g.n_u);
     const int64_t rxkey = iu * g.n_z + iz, txkey = iv * g.n_z + iz;
@@ -148,9 +147,12 @@ __global__ void mask_kernel(const DevGeom g, float *mask, int compound, int accu
     const float a = g.apod_sum[rxkey];
     float total = 0.0f;
     for (int tx = 0; tx < g.n_tx; ++tx) {
-        const float4 t = g.tx_tab[(int64_t)tx * g.n_v * g.n_z + txkey];
-        bool cone = ((g.mode == MODE_EXACT) ? t.w : t.y) != 0.0f;
-        if (g.cone_u) cone = cone && g.cone_u[(int64_t)tx * g.n_u * g.n_z + rxkey] != 0;
+        bool cone = true;   // with no cone table the transmit mask is off: every table entry is inside
+        if (g.cone_u) {
+            const float4 t = g.tx_tab[(int64_t)tx * g.n_v * g.n_z + txkey];
+            cone = ((g.mode == MODE_EXACT) ? t.w : t.y) != 0.0f &&
+                   g.cone_u[(int64_t)tx * g.n_u * g.n_z + rxkey] != 0;
+        }
         const float m = cone ? a : 0.0f;
         if (compound) {
             total = __fadd_rn(total, m);
@@ -162,10 +164,157 @@ __global__ void mask_kernel(const DevGeom g, float *mask, int compound, int accu
     if (compound) mask[pix] = accumulate ? mask[pix] + total : total;
 }
 
+__global__ void mask_kernel(const DevGeom g, float *mask, int compound, int accumulate)
+{
+    mask_voxel(g, mask, compound, accumulate, (int64_t)blockIdx.x * blockDim.x + threadIdx.x);
+}
+
 cudaError_t launch_mask(const DevGeom &g, float *mask, int compound, int accumulate, cudaStream_t st)
 {
     const int64_t n = g.n_z * g.n_u * g.n_v;
     mask_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(g, mask, compound, accumulate);
+    return cudaGetLastError();
+}
+
+// ------------------------------------------------------------------------
+// Everything the streaming kernel needs before it starts, in one launch of
+// independent blocks: channel data -> FP32 slab rows (rounded through the
+// storage type, in the layout they are staged in: das_common.cuh's frame
+// pairs as (re, re, im, im), padded rows, zero rows past the record), the two
+// window range tables, the mask, and a zeroed work counter.  A call on a
+// small grid is bound by launches and by the range kernel's few threads
+// (10-17 us each for one thread per table entry on the 64 x 64 x 128 grid);
+// here 16 lanes share an entry and all parts run at once.
+// ------------------------------------------------------------------------
+constexpr int PREP_THREADS = 256;
+constexpr int RANGE_LANES = 16;
+
+template <int STORE, int IQ>
+__device__ __forceinline__ void prep_ingest(const IngestParams &p, int64_t i)
+{
+    const int rows = p.n_rows;
+    const int n = (int)(i % rows);
+    const int64_t q = i / rows;                       // (tx, ele), frame block
+    const int fb = (int)(q % p.n_fb);
+    const int64_t te = q / p.n_fb;
+    if (te >= (int64_t)p.n_tx * p.n_ele) return;
+    const int FB = p.fb;
+    char *row = reinterpret_cast<char *>(p.S) + (te * p.n_fb + fb) * p.slab_bytes + (int64_t)n * vbs_row_bytes(FB);
+    const int64_t f0 = (int64_t)fb * FB, frame = (int64_t)p.n_tx * p.n_ele * p.n_sample;
+    const int64_t src = te * p.n_sample + n;
+    auto sample = [&](int64_t f) {
+        if (n >= p.n_sample || f >= p.n_frame) return make_float2(0.f, 0.f);
+        return to_f2(from_f2<STORE>(load_iq<IQ>(p.iq, f * frame + src)));
+    };
+    if (FB == 1) {
+        *reinterpret_cast<float2 *>(row) = sample(f0);
+        return;
+    }
+#pragma unroll 4
+    for (int k = 0; k < FB; k += 2) {
+        const float2 a = sample(f0 + k), b = sample(f0 + k + 1);
+        *reinterpret_cast<float4 *>(row + 8 * k) = make_float4(a.x, b.x, a.y, b.y);
+    }
+}
+
+// one table entry per RANGE_LANES lanes
+__device__ __forceinline__ void prep_range(const RangeParams &p, int64_t i, int lane)
+{
+    const int64_t n_out = p.rows * p.tiles_a * p.tiles_z;
+    float lo = __int_as_float(0x7f800000), hi = -lo;
+    if (i < n_out) {
+        const int tzi = (int)(i % p.tiles_z);
+        const int tai = (int)((i / p.tiles_z) % p.tiles_a);
+        const float4 *tab = p.tab + i / ((int64_t)p.tiles_z * p.tiles_a) * p.n_a * p.n_z;
+        const int nz = (int)min((int64_t)p.tz, p.n_z - (int64_t)tzi * p.tz);
+        const int na = (int)min((int64_t)p.ta, p.n_a - (int64_t)tai * p.ta);
+        for (int k = lane; k < na * nz; k += RANGE_LANES) {
+            const float4 e = __ldg(&tab[((int64_t)tai * p.ta + k / nz) * p.n_z + (int64_t)tzi * p.tz + k % nz]);
+            if (!p.is_rx || e.w > 0.0f) { lo = fminf(lo, e.x); hi = fmaxf(hi, e.x); }
+        }
+    }
+#pragma unroll
+    for (int d = RANGE_LANES / 2; d > 0; d >>= 1) {
+        lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, d));
+        hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, d));
+    }
+    if (lane == 0 && i < n_out) p.out[i] = make_float2(lo, hi);
+}
+
+template <int STORE, int IQ>
+__global__ void __launch_bounds__(PREP_THREADS) prep_kernel(const __grid_constant__ PrepParams p)
+{
+    int64_t b = blockIdx.x;
+    if (b == 0 && threadIdx.x == 0) *p.counter = 0u;
+    if (b < p.blocks_rx + p.blocks_tx) {
+        const bool rx = b < p.blocks_rx;
+        if (!rx) b -= p.blocks_rx;
+        prep_range(rx ? p.rx : p.tx, (b * PREP_THREADS + threadIdx.x) / RANGE_LANES, threadIdx.x % RANGE_LANES);
+        return;
+    }
+    b -= p.blocks_rx + p.blocks_tx;
+    if (b < p.blocks_mask) {
+        mask_voxel(p.g, p.mask, p.compound, p.accumulate, b * PREP_THREADS + threadIdx.x);
+        return;
+    }
+    prep_ingest<STORE, IQ>(p.ingest, (b - p.blocks_mask) * PREP_THREADS + threadIdx.x);
+}
+
+template <int STORE>
+static void launch_prep_store(const PrepParams &p, unsigned blocks, cudaStream_t st)
+{
+    switch (p.ingest.iq_dtype) {
+    case 0: prep_kernel<STORE, 0><<<blocks, PREP_THREADS, 0, st>>>(p); break;
+    case 1: prep_kernel<STORE, 1><<<blocks, PREP_THREADS, 0, st>>>(p); break;
+    case 2: prep_kernel<STORE, 2><<<blocks, PREP_THREADS, 0, st>>>(p); break;
+    default: prep_kernel<STORE, 3><<<blocks, PREP_THREADS, 0, st>>>(p); break;
+    }
+}
+
+cudaError_t launch_prep(PrepParams &p, int store, cudaStream_t st)
+{
+    auto blocks = [](int64_t n) { return (n + PREP_THREADS - 1) / PREP_THREADS; };
+    p.blocks_rx = blocks(p.rx.rows * p.rx.tiles_a * p.rx.tiles_z * RANGE_LANES);
+    p.blocks_tx = blocks(p.tx.rows * p.tx.tiles_a * p.tx.tiles_z * RANGE_LANES);
+    p.blocks_mask = p.mask ? blocks(p.g.n_z * p.g.n_u * p.g.n_v) : 0;
+    const int64_t n = p.blocks_rx + p.blocks_tx + p.blocks_mask +
+                      blocks((int64_t)p.ingest.n_tx * p.ingest.n_ele * p.ingest.n_fb * p.ingest.n_rows);
+    if (n > INT32_MAX || p.ingest.iq_dtype < 0 || p.ingest.iq_dtype > 3) return cudaErrorInvalidValue;
+    switch (store) {
+    case ST_F32: launch_prep_store<ST_F32>(p, (unsigned)n, st); break;
+    case ST_F16: launch_prep_store<ST_F16>(p, (unsigned)n, st); break;
+    case ST_BF16: launch_prep_store<ST_BF16>(p, (unsigned)n, st); break;
+    default: return cudaErrorInvalidValue;
+    }
+    return cudaGetLastError();
+}
+
+// ------------------------------------------------------------------------
+// out[f][pix] (+)= sum over splits of part[split][f][pix], in split order:
+// the transmit ranges of a grid too small to fill the GPU with whole items.
+__global__ void __launch_bounds__(256) vbs_reduce_kernel(float2 *__restrict__ out, const float2 *__restrict__ part,
+                                                         int64_t n, int n_split, int accumulate)
+{
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    float2 a = part[i];
+    for (int s = 1; s < n_split; ++s) {
+        const float2 b = part[(int64_t)s * n + i];
+        a.x += b.x;
+        a.y += b.y;
+    }
+    if (accumulate) {
+        const float2 q = out[i];
+        a.x += q.x;
+        a.y += q.y;
+    }
+    out[i] = a;
+}
+
+cudaError_t launch_vbs_reduce(float2 *out, const float2 *partial, int64_t n, int n_split, int accumulate,
+                              cudaStream_t st)
+{
+    vbs_reduce_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(out, partial, n, n_split, accumulate);
     return cudaGetLastError();
 }
 

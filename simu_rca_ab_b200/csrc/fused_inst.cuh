@@ -97,6 +97,7 @@ static cudaError_t plain_iq(const PlainParams &p, cudaStream_t st)
 
 // ---- voxel-blocked kernel (fused_vb_kernel.cuh) ----
 #include "fused_vb_kernel.cuh"
+#include "fused_vbs_kernel.cuh"
 
 namespace rcabf {
 
@@ -128,50 +129,79 @@ static cudaError_t tmem_kernel_occupancy(K k, int threads, size_t smem, int cols
     return cudaSuccess;
 }
 
-template <int KIND, int FB, int STORE, int D, bool TM>
+template <int KIND, int FB, int STORE, int D>
 static cudaError_t vb_do(const FusedParams *p, int grid, size_t smem, cudaStream_t st, int what, int *occ)
 {
-    auto k = fused_vb_kernel<KIND, FB, STORE, D, TM>;
+    auto k = fused_vb_kernel<KIND, FB, STORE, D>;
     if (what == 1) return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (what == 2) {
-        if constexpr (TM) return tmem_kernel_occupancy(k, VB_THREADS, smem, vb_tmem_cols_host(FB), occ);
-        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, k, VB_THREADS, smem);
-    }
+    if (what == 2) return tmem_kernel_occupancy(k, VB_THREADS, smem, vb_tmem_cols_host(FB), occ);
     k<<<grid, VB_THREADS, smem, st>>>(*p);
     return cudaGetLastError();
 }
 
-// tm: accumulators in tensor memory (32 to 128 columns per CTA)
+// accumulators in tensor memory: 32 to 128 columns per CTA
 template <int KIND, int STORE, int D>
-static cudaError_t vb_fb(int tm, int fb, const FusedParams *p, int grid, size_t smem, cudaStream_t st, int what,
-                         int *occ)
+static cudaError_t vb_fb(int fb, const FusedParams *p, int grid, size_t smem, cudaStream_t st, int what, int *occ)
 {
-    if (tm) {
-        switch (fb) {
-        case 2: return vb_do<KIND, 2, STORE, D, true>(p, grid, smem, st, what, occ);
-        case 4: return vb_do<KIND, 4, STORE, D, true>(p, grid, smem, st, what, occ);
-        case 8: return vb_do<KIND, 8, STORE, D, true>(p, grid, smem, st, what, occ);
-        case 16: return vb_do<KIND, 16, STORE, D, true>(p, grid, smem, st, what, occ);
-        default: return cudaErrorInvalidValue;
-        }
-    }
     switch (fb) {
-    case 2: return vb_do<KIND, 2, STORE, D, false>(p, grid, smem, st, what, occ);
-    case 4: return vb_do<KIND, 4, STORE, D, false>(p, grid, smem, st, what, occ);
-    case 8: return vb_do<KIND, 8, STORE, D, false>(p, grid, smem, st, what, occ);
-    case 16: return vb_do<KIND, 16, STORE, D, false>(p, grid, smem, st, what, occ);
+    case 2: return vb_do<KIND, 2, STORE, D>(p, grid, smem, st, what, occ);
+    case 4: return vb_do<KIND, 4, STORE, D>(p, grid, smem, st, what, occ);
+    case 8: return vb_do<KIND, 8, STORE, D>(p, grid, smem, st, what, occ);
+    case 16: return vb_do<KIND, 16, STORE, D>(p, grid, smem, st, what, occ);
     default: return cudaErrorInvalidValue;
     }
 }
 
 template <int KIND, int D>
-static cudaError_t vb_store(int tm, int store, int fb, const FusedParams *p, int grid, size_t smem,
-                            cudaStream_t st, int what, int *occ)
+static cudaError_t vb_store(int store, int fb, const FusedParams *p, int grid, size_t smem, cudaStream_t st, int what,
+                            int *occ)
 {
     switch (store) {
-    case ST_F32: return vb_fb<KIND, ST_F32, D>(tm, fb, p, grid, smem, st, what, occ);
-    case ST_F16: return vb_fb<KIND, ST_F16, D>(tm, fb, p, grid, smem, st, what, occ);
-    case ST_BF16: return vb_fb<KIND, ST_BF16, D>(tm, fb, p, grid, smem, st, what, occ);
+    case ST_F32: return vb_fb<KIND, ST_F32, D>(fb, p, grid, smem, st, what, occ);
+    case ST_F16: return vb_fb<KIND, ST_F16, D>(fb, p, grid, smem, st, what, occ);
+    case ST_BF16: return vb_fb<KIND, ST_BF16, D>(fb, p, grid, smem, st, what, occ);
+    default: return cudaErrorInvalidValue;
+    }
+}
+
+// ---- streaming voxel-blocked kernel (fused_vbs_kernel.cuh) ----
+template <int KIND, int FB, int DEG, int D>
+static cudaError_t vbs_do(const FusedParams *p, int grid, size_t smem, cudaStream_t st, int what, int *occ)
+{
+    auto k = fused_vbs_kernel<KIND, FB, DEG, D>;
+    if (what == 1) return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (what == 2) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, k, VS_THREADS, smem);
+    k<<<grid, VS_THREADS, smem, st>>>(*p);
+    return cudaGetLastError();
+}
+
+template <int KIND, int DEG>
+static cudaError_t vbs_fb(int d, int fb, const FusedParams *p, int grid, size_t smem, cudaStream_t st, int what,
+                          int *occ)
+{
+    switch (d * 100 + fb) {
+    case 102: return vbs_do<KIND, 2, DEG, 1>(p, grid, smem, st, what, occ);
+    case 104: return vbs_do<KIND, 4, DEG, 1>(p, grid, smem, st, what, occ);
+    case 108: return vbs_do<KIND, 8, DEG, 1>(p, grid, smem, st, what, occ);
+    case 116: return vbs_do<KIND, 16, DEG, 1>(p, grid, smem, st, what, occ);
+    case 202: return vbs_do<KIND, 2, DEG, 2>(p, grid, smem, st, what, occ);
+    case 204: return vbs_do<KIND, 4, DEG, 2>(p, grid, smem, st, what, occ);
+    case 208: return vbs_do<KIND, 8, DEG, 2>(p, grid, smem, st, what, occ);
+    case 216: return vbs_do<KIND, 16, DEG, 2>(p, grid, smem, st, what, occ);
+    default: return cudaErrorInvalidValue;
+    }
+}
+
+// every voxel its own rows: degree-8 weights whatever the storage
+template <int KIND>
+static cudaError_t vbs_own_rows(int fb, const FusedParams *p, int grid, size_t smem, cudaStream_t st, int what, int *occ)
+{
+    switch (fb) {
+    case 1: return vbs_do<KIND, 1, 8, 0>(p, grid, smem, st, what, occ);
+    case 2: return vbs_do<KIND, 2, 8, 0>(p, grid, smem, st, what, occ);
+    case 4: return vbs_do<KIND, 4, 8, 0>(p, grid, smem, st, what, occ);
+    case 8: return vbs_do<KIND, 8, 8, 0>(p, grid, smem, st, what, occ);
+    case 16: return vbs_do<KIND, 16, 8, 0>(p, grid, smem, st, what, occ);
     default: return cudaErrorInvalidValue;
     }
 }
@@ -180,11 +210,18 @@ static cudaError_t vb_store(int tm, int store, int fb, const FusedParams *p, int
 
 #define RCABF_VB_TU(KIND, NAME)                                                                      \
     namespace rcabf {                                                                                \
-    cudaError_t vb_entry_##NAME(int d, int tm, int store, int fb, const FusedParams *p, int grid,    \
+    cudaError_t vb_entry_##NAME(int d, int store, int fb, const FusedParams *p, int grid,            \
                                 size_t smem, cudaStream_t st, int what, int *occ)                    \
     {                                                                                                \
-        if (d == 1) return vb_store<KIND, 1>(tm, store, fb, p, grid, smem, st, what, occ);           \
-        if (d == 2) return vb_store<KIND, 2>(tm, store, fb, p, grid, smem, st, what, occ);           \
+        if (d == 1) return vb_store<KIND, 1>(store, fb, p, grid, smem, st, what, occ);               \
+        if (d == 2) return vb_store<KIND, 2>(store, fb, p, grid, smem, st, what, occ);               \
         return cudaErrorInvalidValue;                                                                \
+    }                                                                                                \
+    cudaError_t vbs_entry_##NAME(int d, int store, int fb, const FusedParams *p, int grid,           \
+                                 size_t smem, cudaStream_t st, int what, int *occ)                   \
+    {                                                                                                \
+        if (d == 0) return vbs_own_rows<KIND>(fb, p, grid, smem, st, what, occ);                     \
+        if (store == ST_F32) return vbs_fb<KIND, VbWeightDeg<ST_F32>::value>(d, fb, p, grid, smem, st, what, occ); \
+        return vbs_fb<KIND, VbWeightDeg<ST_F16>::value>(d, fb, p, grid, smem, st, what, occ);        \
     }                                                                                                \
     }

@@ -24,9 +24,10 @@
 // sample rounding is well above the degree-6 weight error of <= 8e-5), each
 // mirrored pair of taps from one even and one odd chain.
 //
-// TM variant: the 2 x VB x FB accumulator words of a thread (128 at FB = 16,
-// half the register file a thread can have) live in tensor memory instead
-// of registers.  Per frame pair the warp loads the 16 words of the pair
+// The 2 x VB x FB accumulator words of a thread (128 at FB = 16, half the
+// register file a thread can have) live in tensor memory instead of
+// registers (frame blocks that registers hold run on the streaming kernel,
+// fused_vbs_kernel.cuh, which gives the same bits).  Per frame pair the warp loads the 16 words of the pair
 // (VB voxels x 2 frames x re/im) from its own TMEM lanes, adds the step's
 // terms and stores them back; a thread then fits in 128 registers instead of
 // 255 (with spills), so four CTAs share an SM (16 warps instead of 8, all 512
@@ -193,12 +194,12 @@ __device__ __forceinline__ void vb_unpack(float w0, float w1, float w2, float w3
     else { f0 = make_float2(w0, w1); f1 = make_float2(w2, w3); }
 }
 
-template <int KIND, int FB, int STORE, int D, bool TM>
-__global__ void __launch_bounds__(VB_THREADS, TM ? VB_TM_MIN_BLOCKS : VB_MIN_BLOCKS)
+template <int KIND, int FB, int STORE, int D>
+__global__ void __launch_bounds__(VB_THREADS, VB_TM_MIN_BLOCKS)
 fused_vb_kernel(const __grid_constant__ FusedParams prm)
 {
     static_assert(FB % 2 == 0, "frames are processed in pairs");
-    static_assert(!TM || VB == 4, "a TMEM access moves the 16 words of VB = 4 voxels x one frame pair");
+    static_assert(VB == 4, "a TMEM access moves the 16 words of VB = 4 voxels x one frame pair");
     using T = typename StoreT<STORE>::T;
     using KT = KindTraits<KIND>;
     constexpr int TAPS = KT::TAPS;
@@ -221,8 +222,8 @@ fused_vb_kernel(const __grid_constant__ FusedParams prm)
     {
         unsigned dyn;
         asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn));
-        // (TM: R rows of zeros follow the stages)
-        if (dyn < (unsigned)(NST * stage_bytes + (TM ? R * STRIDE : 0)) || prm.row_words * 4 != STRIDE ||
+        // R rows of zeros follow the stages
+        if (dyn < (unsigned)(NST * stage_bytes + R * STRIDE) || prm.row_words * 4 != STRIDE ||
             (!ASYNC && prm.wmax * CPR > SREGS * VB_THREADS)) {
             if (tid == 0) atomicAdd(prm.err_count, 1ull);
             return;
@@ -230,12 +231,12 @@ fused_vb_kernel(const __grid_constant__ FusedParams prm)
     }
     unsigned char *stages = smem;
 
-    // TM: warp 0 allocates the CTA's columns; each warp addresses the 32
+    // warp 0 allocates the CTA's columns; each warp addresses the 32
     // lanes of its quadrant, each thread its own lane
     constexpr uint32_t TCOLS = (uint32_t)vb_tmem_cols_host(FB);
     uint32_t tlane = 0;
-    const int zero_off = NST * stage_bytes;   // TM: offset of R staged rows of zeros
-    if constexpr (TM) {
+    const int zero_off = NST * stage_bytes;   // offset of R staged rows of zeros
+    {
         __shared__ uint32_t tbase;
         for (int i = tid; i < R * STRIDE / 16; i += VB_THREADS)
             *reinterpret_cast<float4 *>(smem + zero_off + 16 * i) = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -276,12 +277,7 @@ fused_vb_kernel(const __grid_constant__ FusedParams prm)
         const int n_steps = g.n_tx * g.n_ele;
         const char *S = reinterpret_cast<const char *>(J.S);
 
-        float2 acc[VB][FB];
-#pragma unroll
-        for (int v = 0; v < VB; ++v)
-#pragma unroll
-            for (int f = 0; f < FB; ++f) acc[v][f] = make_float2(0.f, 0.f);
-        // TM: words [16 p, 16 p + 16) of a lane hold frames 2p, 2p + 1 of
+        // accumulators: words [16 p, 16 p + 16) of a lane hold frames 2p, 2p + 1 of
         // its voxels: voxel v at 4 v + the staged layout (VbPlanar: re 2p,
         // re 2p+1, im 2p, im 2p+1; else re 2p, im 2p, re 2p+1, im 2p+1)
         auto tm_zero = [&]() {
@@ -292,26 +288,21 @@ fused_vb_kernel(const __grid_constant__ FusedParams prm)
 #pragma unroll
             for (int c = 0; c < FB; c += 2) tmem_st16(tlane + (uint32_t)(c * 8), z);
         };
-        // per-voxel, per-frame output of the accumulators (TM: read back
-        // from the lane's words), optionally added to what `out` holds
+        // per-voxel, per-frame output of the accumulators (read back from
+        // the lane's words), optionally added to what `out` holds
         auto emit = [&](int64_t frame_stride, int64_t frame_off) {
 #pragma unroll
             for (int c = 0; c < FB; c += 2) {
                 float2 a[VB][2];
-                if constexpr (TM) {
-                    uint32_t w[16];
-                    __syncwarp();
-                    tmem_wait_st();
-                    tmem_ld16(tlane + (uint32_t)(c * 8), w);
-                    tmem_wait_ld16(w);
+                uint32_t w[16];
+                __syncwarp();
+                tmem_wait_st();
+                tmem_ld16(tlane + (uint32_t)(c * 8), w);
+                tmem_wait_ld16(w);
 #pragma unroll
-                    for (int v = 0; v < VB; ++v)
-                        vb_unpack<PL>(__uint_as_float(w[4 * v]), __uint_as_float(w[4 * v + 1]),
-                                      __uint_as_float(w[4 * v + 2]), __uint_as_float(w[4 * v + 3]), a[v][0], a[v][1]);
-                } else {
-#pragma unroll
-                    for (int v = 0; v < VB; ++v) { a[v][0] = acc[v][c]; a[v][1] = acc[v][c + 1]; }
-                }
+                for (int v = 0; v < VB; ++v)
+                    vb_unpack<PL>(__uint_as_float(w[4 * v]), __uint_as_float(w[4 * v + 1]),
+                                  __uint_as_float(w[4 * v + 2]), __uint_as_float(w[4 * v + 3]), a[v][0], a[v][1]);
 #pragma unroll
                 for (int v = 0; v < VB; ++v) {
                     if (v < nvv) {
@@ -329,7 +320,7 @@ fused_vb_kernel(const __grid_constant__ FusedParams prm)
                 }
             }
         };
-        if constexpr (TM) tm_zero();
+        tm_zero();
 
         // Transmit order rotated per tile: a hash of the tile picks the
         // quarter of the transmits the item starts from, so CTAs that share
@@ -464,52 +455,7 @@ fused_vb_kernel(const __grid_constant__ FusedParams prm)
                 }
             }
 
-            if constexpr (!TM) {
-                if (!wA.skip && cone_bits != 0 && e.w > 0.0f) {
-                    const float ab = ab_value(g, tx, rx);
-                    const float2 abp = ab_phasor(g, tx, rx);
-                    // sample index of each voxel; rows are shared from the lowest
-                    float fl[VB], dd[VB];
-                    bool ok[VB];
-                    float base = 3.0e38f;
-#pragma unroll
-                    for (int v = 0; v < VB; ++v) {
-                        const float idx = __fadd_rn(__fadd_rn(txi[v], e.x), ab);
-                        fl[v] = floorf(idx);
-                        dd[v] = idx - fl[v];
-                        ok[v] = ((cone_bits >> v) & 1u) && fl[v] >= (float)KT::LO &&
-                                fl[v] < (float)(J.n_sample - 1 - KT::HI);
-                        if (ok[v]) base = fminf(base, fl[v]);
-                    }
-                    if (base < 2.0e38f) {
-                        float ws[VB][R];
-                        float2 P[VB];
-                        vb_terms<KIND, D, VbWeightDeg<STORE>::value>(prm, fl, dd, ok, base, txr, txq, e, abp, ws, P);
-                        const int row0 = (int)base - KT::LO - wA.lo;
-                        if (row0 < 0 || row0 + R > wA.count || wA.overflow) {
-                            atomicAdd(prm.err_count, 1ull);   // never expected: window bound violated
-                        } else {
-                            const char *rows = reinterpret_cast<const char *>(stages) +
-                                               (s % NST) * stage_bytes + row0 * STRIDE;
-#pragma unroll
-                            for (int c = 0; c < FB; c += 2) {
-                                float2 lo[VB], hi[VB];
-                                vb_pair_sums<R, STRIDE>(rows + c * 8, ws, lo, hi);
-#pragma unroll
-                                for (int v = 0; v < VB; ++v) {
-                                    float2 t0, t1;   // interpolated (re, im) of frames c, c + 1
-                                    vb_unpack<PL>(lo[v].x, lo[v].y, hi[v].x, hi[v].y, t0, t1);
-                                    float2 &a0 = acc[v][c], &a1 = acc[v][c + 1];
-                                    a0.x = fmaf(P[v].x, t0.x, fmaf(-P[v].y, t0.y, a0.x));
-                                    a0.y = fmaf(P[v].x, t0.y, fmaf(P[v].y, t0.x, a0.y));
-                                    a1.x = fmaf(P[v].x, t1.x, fmaf(-P[v].y, t1.y, a1.x));
-                                    a1.y = fmaf(P[v].x, t1.y, fmaf(P[v].y, t1.x, a1.y));
-                                }
-                            }
-                        }
-                    }
-                }
-            } else {
+            {
                 // every lane computes its terms (lanes without voxels carry
                 // zeros); the warp accumulates when any lane contributes
                 const bool act = !wA.skip && cone_bits != 0 && e.w > 0.0f;
@@ -590,14 +536,7 @@ fused_vb_kernel(const __grid_constant__ FusedParams prm)
 
             if (rx == g.n_ele - 1 && !J.compound) {   // per-transmit output
                 emit((int64_t)g.n_tx * g.n_pix, (int64_t)tx * g.n_pix);
-                if constexpr (TM) {
-                    tm_zero();
-                } else {
-#pragma unroll
-                    for (int v = 0; v < VB; ++v)
-#pragma unroll
-                        for (int f = 0; f < FB; ++f) acc[v][f] = make_float2(0.f, 0.f);
-                }
+                tm_zero();
             }
 
             if constexpr (!ASYNC) {
@@ -616,7 +555,7 @@ fused_vb_kernel(const __grid_constant__ FusedParams prm)
 
         if (J.compound) emit(g.n_pix, 0);
     }
-    if constexpr (TM) {
+    {
         // every load was waited for; the last stores complete before the free
         __syncwarp();
         tmem_wait_st();

@@ -1,0 +1,613 @@
+// Persistent delay-and-sum kernel for few frames (sm_100a, EXACT tables,
+// rectilinear grids): register accumulators, sample windows streamed by bulk
+// copies several (tx, rx) steps ahead.
+//
+// A thread owns 4 voxels along v (the transmit-steering axis) and the
+// FB frames of a block, as in the tensor-memory variant (fused_vb_kernel.cuh),
+// whose arithmetic it keeps operation for operation: the two give the same
+// bits.  With few frames per block the per-step work around the frame sums
+// sets the pace, and this kernel is built around that:
+//   - one elected warp scans the steps 32 at a time, drops the ones whose
+//     window is empty for the tile, and issues the others' windows as bulk
+//     copies (cp.async.bulk, one per step: the ingest writes slabs as FP32
+//     rows already padded to the shared-memory stride) in chunks of up to
+//     `krec` steps, three chunks in flight; no thread copies rows, converts
+//     samples or computes windows, and there is no CTA barrier in the loop
+//     (a full / empty mbarrier pair per chunk);
+//   - the weights of voxel pairs are formed with packed FP32 operations
+//     (fma.rn.f32x2: the scalar chain on each half);
+//   - work items are handed out by an atomic counter, deepest tiles first
+//     (the f-number leaves shallow tiles with few active steps, so a fixed
+//     assignment leaves SMs idle at the end), and the scan runs on into the
+//     next item while the current one is computed.
+//
+// Measured (B200, against the barrier-per-step kernels it replaced): 8 frames,
+// 128 x 128 x 256, two orientations 257 -> 152 ms; 4 frames of a 256-element
+// probe 361 -> 252 ms; 20 frames, 97 x 95 x 159 47.3 -> 31.0 ms; one frame, 64 x
+// 64 x 128 9.38 -> 1.60 ms; one frame, 32 x 32 x 64, 4 transmits 455 -> 115 us.
+// What bounds it: instruction issue (64 % of the cycles for one frame, 337
+// instructions per warp and active step, about 140 of them on weights).
+//
+// D >= 1: the four voxels share TAPS + D staged rows (weights shifted to each
+// voxel's first row, zeros elsewhere): one 16-byte load feeds 16 FMAs.
+// D = 0: every voxel reads its own TAPS rows.  Single frames, whose two FMAs
+// per row leave the loads cheap, and grids whose steering step spreads a
+// block over more than two rows.
+#pragma once
+
+#include "das_common.cuh"
+#include "poly_weights.cuh"
+#include "tc_common.cuh"
+
+namespace rcabf {
+
+// Chunks of steps in flight, and most steps of a chunk.
+constexpr int VS_STAGES = 3;
+constexpr int VS_MAXREC = VBS_MAX_RECORDS;
+constexpr int VS_THREADS = VB_THREADS_HOST;
+constexpr int VS_WARPS = VS_THREADS / 32;
+// 1.5 x 2^23: adding it rounding down leaves floor(x) in the low mantissa
+// bits for |x| < 2^22 (the planner bounds the record length by VBS_MAX_SAMPLES)
+constexpr float VS_MAGIC = 12582912.0f;
+constexpr int VS_MAGIC_BITS = 0x4B400000;
+
+// CTAs per SM the registers are budgeted for: 2 x 4 x FB accumulators, the
+// weights and the per-voxel transmit state.
+constexpr int vs_min_blocks(int fb) { return fb >= 8 ? 2 : fb >= 4 ? 3 : 4; }
+
+// One step of a chunk: staged rows [lo, lo + count) of (tx, rx).
+struct __align__(16) VsRec {
+    int32_t lo, count, tx, rx;
+};
+// One chunk: n records of work item `item` (-1: no more items), `last` the
+// item's last chunk.
+struct __align__(16) VsChunkInfo {
+    int32_t item, n, last, pad;
+};
+
+// Bulk copy global -> shared, completion counted in bytes on an mbarrier
+// (both addresses 16-byte aligned, size a multiple of 16).
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_t bytes, uint64_t *bar)
+{
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+                 "l"(src), "r"(bytes), "r"(smem_u32(bar))
+                 : "memory");
+}
+
+__device__ __forceinline__ float2 ld_shared_f2(uint32_t a)
+{
+    float2 v;
+    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ float4 ld_shared_f4(uint32_t a)
+{
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a));
+    return v;
+}
+
+// Work item -> frame block, transmit range and tile.  Tiles in depth-slowest
+// order, deepest first.
+struct VsItem {
+    int job, fb, split, tu, tv, tz, tx0, n_tx;
+};
+__device__ __forceinline__ VsItem vs_item(const FusedParams &prm, int item)
+{
+    VsItem w;
+    w.job = 0;
+    while (w.job + 1 < prm.n_jobs && prm.jobs[w.job + 1].item_begin <= item) ++w.job;
+    const FusedJob &J = prm.jobs[w.job];
+    uint32_t r = (uint32_t)(item - J.item_begin);
+    w.tu = (int)(r % (uint32_t)J.tiles_u);
+    r /= (uint32_t)J.tiles_u;
+    w.tv = (int)(r % (uint32_t)J.tiles_v);
+    r /= (uint32_t)J.tiles_v;
+    w.split = (int)(r % (uint32_t)J.n_split);
+    r /= (uint32_t)J.n_split;
+    w.fb = (int)(r % (uint32_t)J.n_fb);
+    w.tz = J.tiles_z - 1 - (int)(r / (uint32_t)J.n_fb);
+    w.tx0 = (int)((int64_t)w.split * J.g.n_tx / J.n_split);
+    w.n_tx = (int)((int64_t)(w.split + 1) * J.g.n_tx / J.n_split) - w.tx0;
+    return w;
+}
+
+// Scan state of a CTA, uniform over the scanning warp: the item scanned, the
+// one after it (fetched ahead), its steps, the first step of the next batch
+// of 32, the rotation of its step order, and the lanes of the current batch
+// whose step is still to be issued.
+struct VsScan {
+    int item, next, steps, base, rot;
+    unsigned mask;
+    VsItem it;
+};
+
+template <int KIND, int FB, int DEG, int D>
+__global__ void __launch_bounds__(VS_THREADS, vs_min_blocks(FB)) fused_vbs_kernel(const __grid_constant__ FusedParams prm)
+{
+    static_assert(VB_BLOCK == 4, "weights are formed for two pairs of voxels");
+    static_assert(FB == 1 || FB % 2 == 0, "frames are processed in pairs");
+    static_assert(FB >= 2 || D == 0, "single frames: each voxel reads its own rows");
+    using KT = KindTraits<KIND>;
+    constexpr int VB = VB_BLOCK;
+    constexpr int TAPS = KT::TAPS;
+    constexpr int R = TAPS + D;                  // rows a thread reads per step and block (D = 0: per voxel)
+    constexpr int STRIDE = vbs_row_bytes(FB);
+    constexpr int NP = FB == 1 ? 1 : FB / 2;     // frame pairs
+
+    extern __shared__ __align__(128) unsigned char smem[];
+    __shared__ uint64_t full[VS_STAGES], empty[VS_STAGES];
+    __shared__ VsRec recs[VS_STAGES][VS_MAXREC];
+    __shared__ VsChunkInfo info[VS_STAGES];
+    __shared__ VsScan scan_s;
+    __shared__ float4 scan_rng[32];              // per lane: receive, transmit table ranges of the next batch
+    __shared__ int scan_lo[32], scan_cnt[32];    // per lane: window of its step of the current batch
+    __shared__ volatile int abort_s;
+    __shared__ __align__(16) float zeros[D == 0 ? TAPS * STRIDE / 4 : 4];   // TAPS rows of zeros
+
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const uint32_t slot_bytes = (uint32_t)vbs_slot_bytes(FB, prm.wmax);
+    const int krec = prm.krec;
+    {
+        unsigned dyn;
+        asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn));
+        if (krec < 1 || krec > VS_MAXREC || dyn < VS_STAGES * (unsigned)krec * slot_bytes) {
+            if (tid == 0) atomicAdd(prm.err_count, 1ull);
+            return;
+        }
+    }
+    if (tid == 0) {
+        for (int i = 0; i < VS_STAGES; ++i) {
+            mbar_init(&full[i], 1);
+            mbar_init(&empty[i], VS_WARPS);
+        }
+        abort_s = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if constexpr (D == 0)
+        for (int i = tid; i < TAPS * STRIDE / 4; i += VS_THREADS) zeros[i] = 0.f;
+    __syncthreads();
+    volatile int *abort = &abort_s;
+    const uint32_t sbase = smem_u32(smem);
+    const uint32_t zero_rows = smem_u32(zeros);
+
+    // ---------------- the scan (warp 0) ----------------
+    // Its state lives in shared memory between chunks: in registers it would
+    // cost every warp of the CTA the same registers.
+    // per lane: step position p of the item -> (tx, rx)
+    auto step_of = [&](const VsScan &k, int p, int n_ele, int &tx, int &rx) {
+        int e = p + k.rot;
+        if (e >= k.steps) e -= k.steps;
+        const int t = e / n_ele;
+        rx = e - t * n_ele;
+        tx = k.it.tx0 + t;
+    };
+    // starts the copy of the table ranges of batch `base`
+    auto fetch_ranges = [&](const VsScan &k) {
+        const int p = k.base + lane;
+        if (p < k.steps) {
+            const FusedJob &J = prm.jobs[k.it.job];
+            int tx, rx;
+            step_of(k, p, J.g.n_ele, tx, rx);
+            cp_async<8>(&scan_rng[lane].x, &J.rx_range[((int64_t)rx * J.tiles_u + k.it.tu) * J.tiles_z + k.it.tz]);
+            cp_async<8>(&scan_rng[lane].z, &J.tx_range[((int64_t)tx * J.tiles_v + k.it.tv) * J.tiles_z + k.it.tz]);
+        }
+        cp_async_commit();
+    };
+    // takes the next item: its scan starts at its first step
+    auto scan_item = [&](VsScan &k, int item) {
+        k.item = item < (int)prm.n_items ? item : -1;
+        k.mask = 0;
+        k.base = k.steps = 0;
+        if (k.item < 0) return;
+        k.next = 0;
+        if (lane == 0) k.next = (int)atomicAdd(prm.counter, 1u);   // needed when this item's scan ends
+        k.next = __shfl_sync(0xffffffffu, k.next, 0);
+        k.it = vs_item(prm, k.item);
+        const FusedJob &J = prm.jobs[k.it.job];
+        k.steps = k.it.n_tx * J.g.n_ele;
+        // transmit order rotated per tile: a hash of the tile picks the
+        // quarter of the transmits the item starts from, so that CTAs of an
+        // SM do not run their steps in lock step; whole transmits, so a
+        // per-transmit item (n_tx = 1) is complete
+        const uint32_t tile = (uint32_t)(k.it.tz + J.tiles_z * (k.it.tu + J.tiles_u * k.it.tv));
+        const int t0 = k.it.n_tx >= 4 ? (int)(((tile * 0x9E3779B1u) >> 30) * (uint32_t)k.it.n_tx / 4u) : 0;
+        k.rot = t0 * J.g.n_ele;
+        fetch_ranges(k);
+    };
+    // fills stage st with the next chunk
+    auto issue = [&](int st) {
+        VsScan k = scan_s;
+        __syncwarp();
+        int n = 0, last = 0;
+        uint32_t bytes = 0;
+        const int item = k.item;
+        if (item >= 0) {
+            const FusedJob &J = prm.jobs[k.it.job];
+            const int n_ele = J.g.n_ele;
+            const char *S = reinterpret_cast<const char *>(J.S);
+            const uint32_t slot0 = sbase + (uint32_t)(st * krec) * slot_bytes;
+            int lo = scan_lo[lane], cnt = scan_cnt[lane];   // this lane's step of the batch before base
+            while (n < krec) {
+                int tx, rx;
+                if (k.mask == 0) {
+                    if (k.base >= k.steps) { last = 1; break; }
+                    // windows of batch `base`, from the ranges copied ahead
+                    cp_async_wait<0>();
+                    bool act = false;
+                    lo = cnt = 0;
+                    if (k.base + lane < k.steps) {
+                        step_of(k, k.base + lane, n_ele, tx, rx);
+                        const float4 q = scan_rng[lane];
+                        if (q.x <= q.y && q.z <= q.w) {
+                            const float ab = ab_value(J.g, tx, rx), fmax_n = (float)J.n_sample;
+                            float lo_f = __fadd_rn(__fadd_rn(q.z, q.x), ab);
+                            float hi_f = __fadd_rn(__fadd_rn(q.w, q.y), ab);
+                            lo_f = fminf(fmaxf(floorf(lo_f), -1.0f), fmax_n);
+                            hi_f = fminf(fmaxf(floorf(hi_f), -1.0f), fmax_n);
+                            lo = max((int)lo_f - KT::LO, 0);
+                            const int hi = min((int)hi_f - KT::LO + TAPS - 1, J.n_sample - 2);
+                            if (hi >= lo) {
+                                if (FB == 1) lo &= ~1;   // 8-byte rows: keep the copy 16-byte aligned
+                                cnt = hi + D - lo + 1;   // + shift rows
+                                act = cnt <= prm.wmax;
+                                if (!act) atomicAdd(prm.err_count, 1ull);   // never expected: the planner bounds the window
+                            }
+                        }
+                    }
+                    k.mask = __ballot_sync(0xffffffffu, act);
+                    scan_lo[lane] = lo;
+                    scan_cnt[lane] = cnt;
+                    k.base += 32;
+                    fetch_ranges(k);
+                    continue;
+                }
+                const int rank = __popc(k.mask & ((1u << lane) - 1u));
+                const bool mine = ((k.mask >> lane) & 1u) && rank < krec - n;
+                if (mine) {
+                    const int slot = n + rank;
+                    step_of(k, k.base - 32 + lane, n_ele, tx, rx);
+                    recs[st][slot] = VsRec{lo, cnt, tx, rx};
+                    const uint32_t b = ((uint32_t)(cnt * STRIDE) + 15u) & ~15u;
+                    bulk_load(slot0 + (uint32_t)slot * slot_bytes,
+                              S + (((int64_t)tx * n_ele + rx) * J.n_fb + k.it.fb) * J.slab_bytes + (int64_t)lo * STRIDE,
+                              b, &full[st]);
+                    bytes += b;
+                }
+                const unsigned took = __ballot_sync(0xffffffffu, mine);
+                n += __popc(took);
+                k.mask &= ~took;
+            }
+        }
+        bytes = __reduce_add_sync(0xffffffffu, bytes);
+        if (last) scan_item(k, k.next);
+        __syncwarp();   // the lanes' records before lane 0's arrival
+        if (lane == 0) {
+            info[st] = VsChunkInfo{item, n, last, 0};
+            scan_s = k;
+            mbar_arrive_expect_tx(&full[st], bytes);
+        }
+        __syncwarp();
+    };
+
+    if (warp == 0) {
+        int first = 0;
+        if (lane == 0) first = (int)atomicAdd(prm.counter, 1u);
+        VsScan k{};
+        scan_item(k, __shfl_sync(0xffffffffu, first, 0));
+        if (lane == 0) scan_s = k;
+        __syncwarp();
+        issue(0);
+        issue(1);
+    }
+
+    // ---------------- state of the item being computed ----------------
+    int cur = -1, cur_tx = -1, job = 0, n_pair = 0;
+    int iz = 0, iu = 0, iv0 = 0, nvv = 0;     // the thread's first voxel, and how many of its four are on the grid
+    const float4 *rxp = nullptr;              // receive table entry of element 0, and the elements' stride
+    int rx_stride = 0;
+    float lim = 0.f;                          // sample indices at or past it leave the record
+    bool has_ab = false;
+    float4 enext = make_float4(0.f, 0.f, 0.f, 0.f);   // receive table entry of the next record
+    bool have_e = false;
+    unsigned cone_bits = 0;
+    float2 txi[2], txr[2], txq[2];    // voxel pairs: index part and phasor of the current transmit
+    // FB = 1: (re, im) of voxel v in are[v][0]; else frames 2p, 2p + 1 of
+    // voxel v: re in are[v][p], im in aim[v][p]
+    float2 are[VB][NP], aim[VB][FB == 1 ? 1 : NP];
+
+    for (uint32_t c = 0;; ++c) {
+        const int st = (int)(c % VS_STAGES);
+        if (!__all_sync(0xffffffffu, mbar_wait(&full[st], (c / VS_STAGES) & 1u, abort))) break;
+        const VsChunkInfo ck = info[st];
+        if (ck.item < 0) break;
+        if (ck.item != cur) {
+            cur = ck.item;
+            cur_tx = -1;
+            const VsItem ci = vs_item(prm, cur);
+            job = ci.job;
+            const FusedJob &J = prm.jobs[job];
+            const int lu = tid % J.tu, lvb = (tid / J.tu) % J.tv, lz = tid / (J.tu * J.tv);
+            iz = ci.tz * J.tz + lz;
+            iu = ci.tu * J.tu + lu;
+            iv0 = (ci.tv * J.tv + lvb) * VB;
+            const int rem = (int)J.g.n_v - iv0;
+            nvv = !(iz < J.g.n_z && iu < J.g.n_u) || rem <= 0 ? 0 : rem >= VB ? VB : rem;
+            rxp = J.g.rx_tab + (nvv > 0 ? (int64_t)iu * J.g.n_z + iz : 0);   // off the grid: any entry, never used
+            rx_stride = (int)(J.g.n_u * J.g.n_z);
+            lim = (float)(J.n_sample - 1 - KT::HI);
+            has_ab = J.g.ab != nullptr;
+            n_pair = FB == 1 ? 1 : (min(FB, J.n_frame - ci.fb * FB) + 1) / 2;
+#pragma unroll
+            for (int v = 0; v < VB; ++v)
+#pragma unroll
+                for (int p = 0; p < NP; ++p) {
+                    are[v][p] = make_float2(0.f, 0.f);
+                    if constexpr (FB > 1) aim[v][p] = make_float2(0.f, 0.f);
+                }
+        }
+        const uint32_t slot0 = sbase + (uint32_t)(st * krec) * slot_bytes;
+        if (!have_e && ck.n > 0) enext = __ldg(rxp + (int64_t)recs[st][0].rx * rx_stride);
+        for (int i = 0; i < ck.n; ++i) {
+            const VsRec h = recs[st][i];
+            const float4 e = enext;
+            if (i + 1 < ck.n) enext = __ldg(rxp + (int64_t)recs[st][i + 1].rx * rx_stride);
+            if (h.tx != cur_tx) {
+                cur_tx = h.tx;
+                cone_bits = 0;
+                if (nvv > 0) {
+                    const DevGeom &g = prm.jobs[job].g;
+                    const float4 *txrow = g.tx_tab + (int64_t)h.tx * (g.n_v * g.n_z) + iz;
+                    const bool cu = g.cone_u == nullptr ||
+                                    g.cone_u[(int64_t)h.tx * rx_stride + (int64_t)iu * g.n_z + iz] != 0;
+                    float4 t[VB];
+#pragma unroll
+                    for (int v = 0; v < VB; ++v) {
+                        // voxels past the grid: the last one's entry, never in cone_bits
+                        t[v] = __ldg(&txrow[(int64_t)(iv0 + min(v, nvv - 1)) * g.n_z]);
+                        if (cu && v < nvv && t[v].w != 0.0f) cone_bits |= 1u << v;
+                    }
+#pragma unroll
+                    for (int j = 0; j < 2; ++j) {
+                        txi[j] = make_float2(t[2 * j].x, t[2 * j + 1].x);
+                        txr[j] = make_float2(t[2 * j].y, t[2 * j + 1].y);
+                        txq[j] = make_float2(t[2 * j].z, t[2 * j + 1].z);
+                    }
+                }
+            }
+            if (cone_bits == 0 || !(e.w > 0.0f)) continue;
+
+            // ---- sample index of each voxel: floor and fraction ----
+            float2 fl[2], dd[2];
+            float rd[VB];
+            bool ok[VB];
+            float ab = 0.0f;
+            if (has_ab) ab = ab_value(prm.jobs[job].g, h.tx, h.rx);
+            float base = 3.0e38f;
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                float2 idx = __fadd2_rn(txi[j], make_float2(e.x, e.x));
+                idx = __fadd2_rn(idx, make_float2(ab, ab));
+                rd[2 * j] = __fadd_rd(idx.x, VS_MAGIC);
+                rd[2 * j + 1] = __fadd_rd(idx.y, VS_MAGIC);
+                fl[j] = make_float2(rd[2 * j] - VS_MAGIC, rd[2 * j + 1] - VS_MAGIC);
+                dd[j] = make_float2(idx.x - fl[j].x, idx.y - fl[j].y);
+                ok[2 * j] = ((cone_bits >> (2 * j)) & 1u) && fl[j].x >= (float)KT::LO && fl[j].x < lim;
+                ok[2 * j + 1] = ((cone_bits >> (2 * j + 1)) & 1u) && fl[j].y >= (float)KT::LO && fl[j].y < lim;
+                if (ok[2 * j]) base = fminf(base, fl[j].x);
+                if (ok[2 * j + 1]) base = fminf(base, fl[j].y);
+            }
+            if (!(base < 2.0e38f)) continue;
+
+            // ---- phasor P = apod exp(j phase_tx) exp(j phase_rx) exp(j phase_ab) ----
+            float2 Px[2], Py[2];
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                const float2 ey = make_float2(e.y, e.y), ez = make_float2(e.z, e.z);
+                const float2 nq = make_float2(-txq[j].x, -txq[j].y);
+                Px[j] = __ffma2_rn(txr[j], ey, __fmul2_rn(nq, ez));
+                Py[j] = __ffma2_rn(txr[j], ez, __fmul2_rn(txq[j], ey));
+            }
+            if (has_ab) {
+                const float2 abp = ab_phasor(prm.jobs[job].g, h.tx, h.rx);
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    const float2 qx = Px[j], qy = Py[j];
+                    const float2 ax = make_float2(abp.x, abp.x), ay = make_float2(abp.y, abp.y);
+                    Px[j] = __ffma2_rn(qx, ax, __fmul2_rn(make_float2(-qy.x, -qy.y), ay));
+                    Py[j] = __ffma2_rn(qx, ay, __fmul2_rn(qy, ax));
+                }
+            }
+
+            if constexpr (D == 0) {
+                // each voxel's own rows; a voxel without a contribution reads
+                // the rows of zeros and adds exact zeros
+                float2 w[2][TAPS];
+#pragma unroll
+                for (int j = 0; j < 2; ++j) poly_weights2<KIND, DEG>(dd[j], w[j]);
+                const uint32_t slot = slot0 + (uint32_t)i * slot_bytes;
+                uint32_t a[VB];
+                bool bad = false;
+#pragma unroll
+                for (int v = 0; v < VB; ++v) {
+                    const int row = __float_as_int(rd[v]) - VS_MAGIC_BITS - KT::LO - h.lo;
+                    const bool in = (unsigned)row <= (unsigned)(h.count - TAPS);
+                    bad = bad || (ok[v] && !in);
+                    a[v] = ok[v] && in ? slot + (uint32_t)(row * STRIDE) : zero_rows;
+                }
+                if (bad) atomicAdd(prm.err_count, 1ull);   // never expected: window bound violated
+                auto wt = [&](int v, int k) { return v & 1 ? w[v >> 1][k].y : w[v >> 1][k].x; };
+                if constexpr (FB == 1) {
+                    float2 tv[VB];   // interpolated sample
+#pragma unroll
+                    for (int v = 0; v < VB; ++v) {
+                        tv[v] = make_float2(0.f, 0.f);
+#pragma unroll
+                        for (int k = 0; k < TAPS; ++k) {
+                            const float2 x = ld_shared_f2(a[v] + k * STRIDE);
+                            tv[v].x = fmaf(wt(v, k), x.x, tv[v].x);
+                            tv[v].y = fmaf(wt(v, k), x.y, tv[v].y);
+                        }
+                    }
+#pragma unroll
+                    for (int v = 0; v < VB; ++v) {
+                        const float px = v & 1 ? Px[v >> 1].y : Px[v >> 1].x, py = v & 1 ? Py[v >> 1].y : Py[v >> 1].x;
+                        float2 &q = are[v][0];
+                        q.x = fmaf(px, tv[v].x, fmaf(-py, tv[v].y, q.x));
+                        q.y = fmaf(px, tv[v].y, fmaf(py, tv[v].x, q.y));
+                    }
+                } else {
+#pragma unroll
+                    for (int p = 0; p < NP; ++p) {
+                        if (p < n_pair) {
+#pragma unroll
+                            for (int v = 0; v < VB; ++v) {
+                                const float px = v & 1 ? Px[v >> 1].y : Px[v >> 1].x;
+                                const float py = v & 1 ? Py[v >> 1].y : Py[v >> 1].x;
+                                float2 tre = make_float2(0.f, 0.f), tim = tre;
+#pragma unroll
+                                for (int k = 0; k < TAPS; ++k) {
+                                    const float4 x = ld_shared_f4(a[v] + k * STRIDE + p * 16);
+                                    const float2 w2 = make_float2(wt(v, k), wt(v, k));
+                                    tre = __ffma2_rn(w2, make_float2(x.x, x.y), tre);
+                                    tim = __ffma2_rn(w2, make_float2(x.z, x.w), tim);
+                                }
+                                are[v][p] = __ffma2_rn(make_float2(px, px), tre,
+                                                       __ffma2_rn(make_float2(-py, -py), tim, are[v][p]));
+                                aim[v][p] = __ffma2_rn(make_float2(px, px), tim,
+                                                       __ffma2_rn(make_float2(py, py), tre, aim[v][p]));
+                            }
+                        }
+                    }
+                }
+            } else {
+                // rows shared from the lowest voxel's first one
+                const int row0 = __float_as_int(base + VS_MAGIC) - VS_MAGIC_BITS - KT::LO - h.lo;
+                if (row0 < 0 || row0 + R > h.count) {
+                    atomicAdd(prm.err_count, 1ull);   // never expected: window bound violated
+                    continue;
+                }
+                float ws[VB][R];
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    float2 w[TAPS];
+                    poly_weights2<KIND, DEG>(dd[j], w);
+#pragma unroll
+                    for (int h2 = 0; h2 < 2; ++h2) {
+                        const int v = 2 * j + h2;
+                        const float sh = (h2 ? fl[j].y : fl[j].x) - base;   // rows of shift
+                        if (ok[v] && sh > (float)D + 0.5f) { atomicAdd(prm.err_count, 1ull); ok[v] = false; }
+                        const bool s1 = sh > 0.5f, s2 = sh > 1.5f;
+#pragma unroll
+                        for (int k = 0; k < R; ++k) {
+                            auto wt = [&](int q) { return q >= 0 && q < TAPS ? (h2 ? w[q].y : w[q].x) : 0.0f; };
+                            float a = wt(k);
+                            if (s1) a = wt(k - 1);
+                            if constexpr (D >= 2) { if (s2) a = wt(k - 2); }
+                            ws[v][k] = a;
+                        }
+                    }
+                }
+                float px[VB], py[VB];
+#pragma unroll
+                for (int v = 0; v < VB; ++v) {
+                    px[v] = ok[v] ? (v & 1 ? Px[v >> 1].y : Px[v >> 1].x) : 0.0f;
+                    py[v] = ok[v] ? (v & 1 ? Py[v >> 1].y : Py[v >> 1].x) : 0.0f;
+                }
+                const uint32_t a0 = slot0 + (uint32_t)i * slot_bytes + (uint32_t)(row0 * STRIDE);
+#pragma unroll
+                for (int p = 0; p < NP; ++p) {
+                    if (p < n_pair) {
+                        float2 tre[VB], tim[VB];
+#pragma unroll
+                        for (int v = 0; v < VB; ++v) { tre[v] = make_float2(0.f, 0.f); tim[v] = tre[v]; }
+#pragma unroll
+                        for (int k = 0; k < R; ++k) {
+                            const float4 x = ld_shared_f4(a0 + k * STRIDE + p * 16);
+#pragma unroll
+                            for (int v = 0; v < VB; ++v) {
+                                const float2 w2 = make_float2(ws[v][k], ws[v][k]);
+                                tre[v] = __ffma2_rn(w2, make_float2(x.x, x.y), tre[v]);
+                                tim[v] = __ffma2_rn(w2, make_float2(x.z, x.w), tim[v]);
+                            }
+                        }
+#pragma unroll
+                        for (int v = 0; v < VB; ++v) {
+                            const float2 p2 = make_float2(px[v], px[v]);
+                            are[v][p] = __ffma2_rn(p2, tre[v], __ffma2_rn(make_float2(-py[v], -py[v]), tim[v], are[v][p]));
+                            aim[v][p] = __ffma2_rn(p2, tim[v], __ffma2_rn(make_float2(py[v], py[v]), tre[v], aim[v][p]));
+                        }
+                    }
+                }
+            }
+        }
+        have_e = false;
+        if (ck.last) {
+            const FusedJob &J = prm.jobs[job];
+            const DevGeom &g = J.g;
+            // the item's outputs: the volume (or the transmit's own, when not
+            // compounded), or this transmit range's part of it
+            const VsItem ci = vs_item(prm, cur);
+            cur = -1;
+            const int64_t pix0 = iz * g.s_z + iu * g.s_u + (int64_t)iv0 * g.s_v;
+            float2 *out = J.out;
+            int64_t stride = g.n_pix, off = 0;
+            bool add = J.accumulate != 0;
+            if (!J.compound) {
+                stride = (int64_t)g.n_tx * g.n_pix;
+                off = (int64_t)ci.tx0 * g.n_pix;
+            } else if (J.n_split > 1) {
+                out = J.partial + (int64_t)ci.split * J.n_frame * g.n_pix;
+                add = false;
+            }
+#pragma unroll
+            for (int v = 0; v < VB; ++v) {
+                if (v < nvv) {
+#pragma unroll
+                    for (int f = 0; f < FB; ++f) {
+                        const int fr = ci.fb * FB + f;
+                        if (fr < J.n_frame) {
+                            float2 a;
+                            if constexpr (FB == 1) a = are[v][0];
+                            else a = f & 1 ? make_float2(are[v][f >> 1].y, aim[v][f >> 1].y)
+                                           : make_float2(are[v][f >> 1].x, aim[v][f >> 1].x);
+                            float2 *o = out + (int64_t)fr * stride + off + pix0 + v * g.s_v;
+                            if (add) { float2 q = *o; q.x += a.x; q.y += a.y; *o = q; }
+                            else *o = a;
+                        }
+                    }
+                }
+            }
+        }
+        else {
+            // the next chunk's first table entry, when the chunk has landed
+            const uint32_t nc = c + 1;
+            const int ns = (int)(nc % VS_STAGES);
+            if (__all_sync(0xffffffffu, mbar_test_wait(&full[ns], (nc / VS_STAGES) & 1u))) {
+                have_e = info[ns].n > 0;
+                if (have_e) enext = __ldg(rxp + (int64_t)recs[ns][0].rx * rx_stride);
+            }
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&empty[st]);
+        if (warp == 0) {
+            // refill the stage of the chunk before this one: the other warps
+            // had the whole of this chunk to leave it
+            if (c >= 1 && !__all_sync(0xffffffffu, mbar_wait(&empty[(c - 1) % VS_STAGES], ((c - 1) / VS_STAGES) & 1u, abort)))
+                break;
+            issue((int)((c + 2) % VS_STAGES));
+        }
+    }
+    if (abort_s) {
+        // a wait ran out: count it, and leave only when the copies this CTA
+        // issued have landed (each wait bounded)
+        if (tid == 0) {
+            atomicAdd(prm.err_count, 1ull);
+            int none = 0;
+            for (int i = 0; i < VS_STAGES; ++i)
+                for (uint32_t ph = 0; ph < 2; ++ph) mbar_wait(&full[i], ph, &none, 100000000ull);
+        }
+    }
+}
+
+}  // namespace rcabf

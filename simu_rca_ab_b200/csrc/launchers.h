@@ -27,6 +27,18 @@ struct RangeParams {
     int32_t mode, is_rx;
 };
 
+// One launch of everything the streaming voxel-blocked kernel reads
+// (aux_kernels.cu).  launch_prep fills the block counts.
+struct PrepParams {
+    IngestParams ingest;       // n_rows: slab rows, the record and its zero rows
+    RangeParams rx, tx;
+    DevGeom g;
+    float *mask;               // NULL: no mask
+    int32_t compound, accumulate;
+    uint32_t *counter;         // zeroed
+    int64_t blocks_rx, blocks_tx, blocks_mask;
+};
+
 // Inputs of the REF_COMPAT table kernels: single-precision copies of what the
 // reference wrapper hands its kernel (RCA.m:601-626), per table key.
 struct RefTableParams {
@@ -50,6 +62,7 @@ struct RefTableParams {
 };
 
 cudaError_t launch_ingest(const IngestParams &p, int store, cudaStream_t st);
+cudaError_t launch_prep(PrepParams &p, int store, cudaStream_t st);
 cudaError_t launch_range(const RangeParams &p, cudaStream_t st);
 cudaError_t launch_mask(const DevGeom &g, float *mask, int compound, int accumulate, cudaStream_t st);
 cudaError_t launch_fma_probe(float *out, int blocks, int iters, cudaStream_t st);
@@ -63,13 +76,24 @@ cudaError_t prepare_fused(int mode, int kind, int fb, int store, size_t smem);
 // Resident CTAs per SM for a variant at a given dynamic shared memory size.
 int fused_occupancy(int mode, int kind, int fb, int store, size_t smem);
 
-// Voxel-blocked fused kernel (EXACT tables): d = row shift bound (1 or 2),
-// fb in {2, 4, 8, 16}; 128 threads per CTA; tm = 1: accumulators in tensor
-// memory, occupancy capped by the SM's 512 TMEM columns.
-cudaError_t launch_fused_vb(int kind, int d, int tm, int fb, int store, const FusedParams &p, int grid,
-                            size_t smem, cudaStream_t st);
-cudaError_t prepare_fused_vb(int kind, int d, int tm, int fb, int store, size_t smem);
-int fused_vb_occupancy(int kind, int d, int tm, int fb, int store, size_t smem);
+// Voxel-blocked fused kernel with tensor-memory accumulators (EXACT tables):
+// d = row shift bound (1 or 2), fb in {2, 4, 8, 16}; 128 threads per CTA,
+// occupancy capped by the SM's 512 TMEM columns.
+cudaError_t launch_fused_vb(int kind, int d, int fb, int store, const FusedParams &p, int grid, size_t smem,
+                            cudaStream_t st);
+cudaError_t prepare_fused_vb(int kind, int d, int fb, int store, size_t smem);
+int fused_vb_occupancy(int kind, int d, int fb, int store, size_t smem);
+
+// Streaming voxel-blocked kernel with register accumulators (EXACT tables):
+// d = row shift bound 1 or 2 with fb in {2, 4, 8, 16}, or 0 (every voxel reads
+// its own rows) with fb in {1, 2, 4, 8, 16}; `store` picks the weight polynomials.
+cudaError_t launch_fused_vbs(int kind, int d, int fb, int store, const FusedParams &p, int grid, size_t smem,
+                             cudaStream_t st);
+cudaError_t prepare_fused_vbs(int kind, int d, int fb, int store, size_t smem);
+int fused_vbs_occupancy(int kind, int d, int fb, int store, size_t smem);
+// out (+)= the transmit ranges' sums, n elements each
+cudaError_t launch_vbs_reduce(float2 *out, const float2 *partial, int64_t n, int n_split, int accumulate,
+                              cudaStream_t st);
 
 // Tensor-core kernel (FP16 slabs, EXACT tables, compounded output; one CTA
 // per SM, all 512 tensor-memory columns): fb frames per block (multiple of

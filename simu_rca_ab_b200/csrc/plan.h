@@ -15,10 +15,13 @@ constexpr size_t SMEM_BUDGET = 110 * 1024;
 struct Plan {
     int kernel = 0;       // rcabf_kernel
     int pc_all = 0;       // per-channel output, every frame in one launch (pc_das_kernel)
-    int vb = 0;           // voxel-blocked kernel (fused_vb_kernel.cuh): 1 register, 2 TMEM accumulators
+    // voxel-blocked kernels: 1 register accumulators, streamed windows
+    // (fused_vbs_kernel.cuh), 2 TMEM accumulators (fused_vb_kernel.cuh)
+    int vb = 0;
+    int n_split = 1;      // vb = 1: transmit ranges, one work item each
     int tc = 0;           // tensor-core kernel (fused_tc_kernel.cuh): 1 FP16 weights, 2 hi + remainder weights
     int tc_rows = 0;      // its slab rows (the record + zero rows a window may reach past it)
-    int d = 0;            // its row shift bound
+    int d = 0;            // voxel-blocked kernels: row shift bound (0: every voxel reads its own rows)
     int store = 0;
     int fb = 1, n_fb = 1;
     TileShape ts{1, 1, 256};
@@ -26,7 +29,7 @@ struct Plan {
     int wmax = 0, row_words = 0;
     size_t smem = 0;
     int64_t slab_bytes = 0;
-    size_t off_S = 0, off_rxr = 0, off_txr = 0, total = 0;
+    size_t off_S = 0, off_rxr = 0, off_txr = 0, off_part = 0, off_ctr = 0, total = 0;
     int64_t n_items = 0;
 };
 
@@ -34,6 +37,9 @@ struct Plan {
 // without one, a choice rcabf_autotune stored for these frames and storage
 // is used.  RCABF_ERR_UNSUPPORTED when a forced choice does not fit.
 int plan_beamform(rcabf_geometry *g, const rcabf_beamform_args *a, Plan &p, const TuneChoice *force = nullptr);
+
+// Smaller-workspace replacement of a streaming-kernel plan (api.cpp).
+void plan_compact(rcabf_geometry *g, rcabf_beamform_args &a, Plan &p);
 
 // Frame-block sizes with a compiled fused-kernel variant.
 bool fb_supported(int mode, int fb);
@@ -59,6 +65,16 @@ inline size_t vb_smem_bytes(int store, int wmax, int row_words, int zero_rows = 
 {
     return (size_t)(fused_stages(store) * wmax + zero_rows) * row_words * 4;
 }
+// Steps per chunk of the streaming kernel: as many as its three chunks'
+// share of the SM's shared memory holds at the CTAs its registers allow
+// (0: not even one).
+inline int vbs_chunk_records(int fb, int wmax)
+{
+    const int ctas = fb >= 8 ? 2 : fb >= 4 ? 3 : 4;
+    const int n = (int)((224 * 1024 / ctas - 2048) / (3 * (size_t)vbs_slot_bytes(fb, wmax)));
+    return n > VBS_MAX_RECORDS ? VBS_MAX_RECORDS : n;
+}
+inline size_t vbs_smem_bytes(int fb, int wmax) { return 3 * (size_t)vbs_chunk_records(fb, wmax) * vbs_slot_bytes(fb, wmax); }
 inline int vb_stage_rows_cap(int store, int fb)
 {
     if (store == ST_F32) return 1 << 30;

@@ -86,6 +86,8 @@ struct FusedJob {
     int32_t compound, accumulate;
     int32_t tiles_z, tiles_u, tiles_v;
     int32_t tu, tv, tz;        // tile shape, tu*tv*tz = blockDim.x
+    int32_t n_split;           // streaming kernel: transmit ranges, an item each (n_tx when not compounded)
+    float2 *partial;           // its sums per range [n_split][frame][pix] when compounded and n_split > 1
 };
 
 // Tensor-core kernel (fused_tc_kernel.cuh): voxel tiles of 128 voxels, tu
@@ -100,17 +102,29 @@ constexpr int FUSED_STAGES = 3;
 constexpr int VB_BLOCK = 4;          // voxels per thread along v in the voxel-blocked kernel
 constexpr int VB_THREADS_HOST = 128; // its CTA size
 constexpr int VB_STAGE_REGS = 2;     // 16-byte staging chunks a thread holds (FP16/BF16 slabs)
-constexpr int VB_MIN_BLOCKS = 1;     // launch-bounds hint: more forces spills (~230 registers live)
-constexpr int VB_TM_MIN_BLOCKS = 4;  // the same with the accumulators in tensor memory (128 registers, no spills)
+constexpr int VB_TM_MIN_BLOCKS = 4;  // launch-bounds hint with the accumulators in tensor memory (128 registers, no spills)
 // tensor-memory columns a CTA of the voxel-blocked kernel allocates: 16 per
 // frame pair, a power of two >= 32
 constexpr RCABF_HD int vb_tmem_cols_host(int fb) { return fb * 8 <= 32 ? 32 : fb * 8; }
+
+// Streaming voxel-blocked kernel (fused_vbs_kernel.cuh): steps per chunk at
+// most, the longest record its floor() covers, FP32 slab rows in the layout
+// they are staged in (frame pairs as (re, re, im, im), rows of 4 frames or
+// more padded by 16 bytes so that 8 consecutive rows start in distinct banks).
+constexpr int VBS_MAX_RECORDS = 8;
+constexpr int VBS_MAX_SAMPLES = 1 << 21;
+constexpr int VBS_MIN_ITEMS = 8 * 148;   // work items below which a grid is split by transmits
+constexpr int VBS_PAD_ROWS = 2;      // zero rows past the record (shift rows)
+constexpr RCABF_HD int vbs_row_bytes(int fb) { return fb <= 2 ? 8 * fb : 8 * fb + 16; }
+constexpr RCABF_HD int vbs_slot_bytes(int fb, int wmax) { return (wmax * vbs_row_bytes(fb) + 15) / 16 * 16; }
 
 struct FusedParams {
     FusedJob jobs[MAX_JOBS];
     int32_t n_jobs;
     int32_t wmax;               // rows per shared-memory stage
     int32_t row_words;          // shared-memory row stride (4-byte words)
+    int32_t krec;               // streaming kernel: steps per chunk
+    uint32_t *counter;          // streaming kernel: work items handed out (zero at launch)
     int64_t n_items;
     unsigned long long *err_count;
 };
