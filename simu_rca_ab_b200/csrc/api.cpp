@@ -131,7 +131,7 @@ int choose_fb(const rcabf_geometry *g, int store, int64_t n_frame, int requested
     return best;
 }
 
-int plan_beamform(rcabf_geometry *g, const rcabf_beamform_args *a, Plan &p, const TuneChoice *force)
+int plan_beamform(rcabf_geometry *g, const rcabf_beamform_args *a, Plan &p, const TuneChoice *force, int split_req)
 {
     if (!g || !a) return RCABF_ERR_INVALID_ARGUMENT;
     if (a->struct_size != (int32_t)sizeof(rcabf_beamform_args)) return RCABF_ERR_INVALID_ARGUMENT;
@@ -170,10 +170,12 @@ int plan_beamform(rcabf_geometry *g, const rcabf_beamform_args *a, Plan &p, cons
         }
     }
     auto layout = [&](int tile_v_extent) {
-        p.n_fb = (int)((a->n_frame + p.fb - 1) / p.fb);
+        p.n_fb = (int)((a->n_frame * p.n_sym + p.fb - 1) / p.fb);
+        p.nu_t = p.mirror & VBS_MIRROR_U ? (g->n_u + 1) / 2 : g->n_u;
+        p.nv_t = p.mirror & VBS_MIRROR_V ? (g->n_v + 1) / 2 : g->n_v;
         p.tiles_z = (int)((g->n_z + p.ts.tz - 1) / p.ts.tz);
-        p.tiles_u = (int)((g->n_u + p.ts.tu - 1) / p.ts.tu);
-        p.tiles_v = (int)((g->n_v + tile_v_extent - 1) / tile_v_extent);
+        p.tiles_u = (int)((p.nu_t + p.ts.tu - 1) / p.ts.tu);
+        p.tiles_v = (int)((p.nv_t + tile_v_extent - 1) / tile_v_extent);
         p.row_words = fused_row_words(p.fb);
         p.slab_bytes = p.vb == 1 ? (a->n_sample + VBS_PAD_ROWS) * vbs_row_bytes(p.fb)
                                  : (int64_t)(p.tc ? p.tc_rows : a->n_sample) * p.fb * es;
@@ -183,7 +185,10 @@ int plan_beamform(rcabf_geometry *g, const rcabf_beamform_args *a, Plan &p, cons
         p.off_S = off;
         // (tensor-core plans: the slabs, then right after them the same
         // slabs holding (-im, re), one row range of the kernel's tensor map)
-        off += al((size_t)g->n_tx * g->n_ele * p.n_fb * p.slab_bytes * (p.tc ? 2 : 1));
+        p.compact = p.n_sym > 1 && p.fb >= p.n_sym;
+        p.slab_tx = p.compact && (p.mirror & VBS_MIRROR_V) ? (g->n_tx + 1) / 2 : g->n_tx;
+        p.slab_ele = p.compact && (p.mirror & VBS_MIRROR_U) ? (g->n_ele + 1) / 2 : g->n_ele;
+        off += al((size_t)p.slab_tx * p.slab_ele * p.n_fb * p.slab_bytes * (p.tc ? 2 : 1));
         p.off_rxr = off;
         off += al((size_t)g->n_ele * p.tiles_u * p.tiles_z * sizeof(float2));
         p.off_txr = off;
@@ -287,14 +292,27 @@ int plan_beamform(rcabf_geometry *g, const rcabf_beamform_args *a, Plan &p, cons
             vts = force->ts;
         }
         const int rows = g->window_rows(TileShape{vts.tu, vts.tv * VB_BLOCK, vts.tz});
-        // streaming kernel: a grid of few tiles is split by transmits until
-        // there are two items per resident CTA (a number that depends on the
-        // grid alone, not on frames: the split sets the order of the sums)
-        const int64_t tiles = ((g->n_z + vts.tz - 1) / vts.tz) * ((g->n_u + vts.tu - 1) / vts.tu) *
-                              ((g->n_v + vts.tv * VB_BLOCK - 1) / (vts.tv * VB_BLOCK));
-        const int split = !a->compound ? g->n_tx
-                          : named ? 1
-                                  : (int)std::min<int64_t>(g->n_tx, (VBS_MIN_ITEMS + tiles - 1) / tiles);
+        // streaming kernel: symmetric axes are mirrored where that drops about
+        // half of the tiles (the grid fills the last ones)
+        auto n_tiles = [](int64_t n, int64_t t) { return (n + t - 1) / t; };
+        const int64_t tile_v = vts.tv * VB_BLOCK;
+        int mirror = named ? 0 : g->mirror;
+        if (5 * n_tiles((g->n_u + 1) / 2, vts.tu) > 3 * n_tiles(g->n_u, vts.tu)) mirror &= ~VBS_MIRROR_U;
+        if (5 * n_tiles((g->n_v + 1) / 2, tile_v) > 3 * n_tiles(g->n_v, tile_v)) mirror &= ~VBS_MIRROR_V;
+        const int n_sym = (mirror & VBS_MIRROR_U ? 2 : 1) * (mirror & VBS_MIRROR_V ? 2 : 1);
+        const int64_t tiles = n_tiles(g->n_z, vts.tz) *
+                              n_tiles(mirror & VBS_MIRROR_U ? (g->n_u + 1) / 2 : g->n_u, vts.tu) *
+                              n_tiles(mirror & VBS_MIRROR_V ? (g->n_v + 1) / 2 : g->n_v, tile_v);
+        // few work items are split by transmits, to about two items per
+        // resident CTA (the split sets the order of the sums: a caller that
+        // cuts one acquisition into several calls passes the whole one's)
+        auto split = [&](int fb) {
+            if (!a->compound) return g->n_tx;
+            if (named) return 1;
+            if (split_req > 0) return split_req;
+            const int64_t items = tiles * n_tiles(a->n_frame * n_sym, fb);
+            return (int)std::min<int64_t>(g->n_tx, n_tiles(2 * 148 * vbs_min_ctas(fb), items));
+        };
         auto fits = [&](int vb, int d, int fb) {   // the largest window of the acquisition in its staging buffer
             const int need = (int)std::min<int64_t>(rows + std::max(d, 1), a->n_sample + d);
             if (vb == 1)
@@ -310,16 +328,17 @@ int plan_beamform(rcabf_geometry *g, const rcabf_beamform_args *a, Plan &p, cons
                 // the planner's choice: at most the frame count rounded up to a
                 // power of two (a block more than half empty costs more than
                 // the setup it saves); a store asked for by name may pad to 2x
-                const int64_t lim = want_vb ? 2 * a->n_frame : pow2_ceil(a->n_frame);
+                const int64_t lim = want_vb ? 2 * a->n_frame : pow2_ceil(a->n_frame * (vb == 1 ? n_sym : 1));
                 if (!force && fb_req == 0 && c > lim) continue;
                 // register accumulators: blocks of 8 at most (16 spill), but by name,
                 // and where every frame block has to keep one order of sums
-                if (vb == 1 && c == 16 && !want_vb && !(fb_req == 16 && (split > 1 || d == 0))) continue;
+                if (vb == 1 && c == 16 && !want_vb && !(fb_req == 16 && (split(8) > 1 || d == 0 || n_sym > 1))) continue;
                 if (fits(vb, d, c)) return c;
             }
             return 0;
         };
-        const bool single = force ? force->fb == 1 : fb_req == 1 || (fb_req == 0 && a->n_frame == 1);
+        // single frames without mirrored copies: every voxel its own rows
+        const bool single = force ? force->fb == 1 : fb_req == 1 || (fb_req == 0 && a->n_frame * n_sym == 1);
         int vb = 0, d = shift <= 2 && !single ? shift : 0, fb = 0;
         if (want_vb) {
             fb = pick(vb = want_vb, d);
@@ -334,7 +353,11 @@ int plan_beamform(rcabf_geometry *g, const rcabf_beamform_args *a, Plan &p, cons
             p.fb = fb;
             p.ts = vts;
             p.wmax = (int)std::min<int64_t>(rows + std::max(d, 1), a->n_sample + d);
-            if (vb == 1) p.n_split = split;
+            if (vb == 1) {
+                p.n_split = split(fb);
+                p.mirror = mirror;
+                p.n_sym = n_sym;
+            }
             layout(vts.tv * VB_BLOCK);
             if (p.n_items < INT32_MAX) {
                 p.smem = vb == 1 ? vbs_smem_bytes(fb, p.wmax)
@@ -394,7 +417,7 @@ static void mark(const rcabf_beamform_args *a, int i, cudaStream_t st)
 }
 
 // Fills the per-job descriptor and launches the job's ingest and range kernels.
-// (the streaming kernel's: one launch that also writes the mask.)
+// (the streaming kernel's in one launch.)
 int stage_job(rcabf_geometry *g, const rcabf_beamform_args *a, const Plan &p, FusedJob &J, cudaStream_t st,
               const rcabf_beamform_args *marks = nullptr)
 {
@@ -421,8 +444,10 @@ int stage_job(rcabf_geometry *g, const rcabf_beamform_args *a, const Plan &p, Fu
         PrepParams pp{};
         pp.ingest = ip;
         pp.ingest.n_rows = (int)a->n_sample + VBS_PAD_ROWS;
-        pp.rx = rr; pp.tx = tr; pp.g = g->dev(); pp.mask = a->mask;
-        pp.compound = a->compound ? 1 : 0; pp.accumulate = a->accumulate ? 1 : 0;
+        pp.ingest.n_sym = p.n_sym; pp.ingest.mirror = p.mirror;
+        pp.ingest.slab_tx = p.slab_tx; pp.ingest.slab_ele = p.slab_ele;
+        pp.rx = rr; pp.tx = tr;
+        pp.rx.n_lim = p.nu_t; pp.tx.n_lim = p.nv_t;
         pp.counter = reinterpret_cast<uint32_t *>(ws + p.off_ctr);
         if ((ce = launch_prep(pp, p.store, st)) != cudaSuccess) return cuda_fail(ce, "preparation launch");
         if (marks) mark(marks, 1, st);
@@ -445,6 +470,9 @@ int stage_job(rcabf_geometry *g, const rcabf_beamform_args *a, const Plan &p, Fu
     J.compound = a->compound ? 1 : 0; J.accumulate = a->accumulate ? 1 : 0;
     J.tiles_z = p.tiles_z; J.tiles_u = p.tiles_u; J.tiles_v = p.tiles_v;
     J.tu = p.ts.tu; J.tv = p.ts.tv; J.tz = p.ts.tz;
+    J.nu_t = (int)p.nu_t; J.nv_t = (int)p.nv_t;
+    J.n_sym = p.n_sym; J.mirror = p.mirror; J.n_vf = (int)(a->n_frame * p.n_sym);
+    J.compact = p.compact;
     J.n_split = p.n_split;
     J.partial = reinterpret_cast<float2 *>(ws + p.off_part);
     return RCABF_OK;
@@ -461,10 +489,10 @@ static int finish_job(const rcabf_geometry *g, const rcabf_beamform_args *a, con
     return RCABF_OK;
 }
 
-// The mask, where no earlier launch of the plan has written it.
-static int finish_mask(const rcabf_geometry *g, const rcabf_beamform_args *a, const Plan &p, cudaStream_t st)
+// The mask, last: like the volume, it is written when the launch ends.
+static int finish_mask(const rcabf_geometry *g, const rcabf_beamform_args *a, cudaStream_t st)
 {
-    if (!a->mask || p.vb == 1) return RCABF_OK;
+    if (!a->mask) return RCABF_OK;
     const cudaError_t e = launch_mask(g->dev(), a->mask, a->compound ? 1 : 0, a->accumulate ? 1 : 0, st);
     if (e != cudaSuccess) return cuda_fail(e, "mask kernel launch");
     g_launches += 1;
@@ -592,7 +620,7 @@ static int beamform_planned(rcabf_geometry *g, const rcabf_beamform_args *a, con
         if ((s = finish_job(g, a, p, prm.jobs[0], st)) != RCABF_OK) return s;
     }
     mark(a, 3, st);
-    if ((s = finish_mask(g, a, p, st)) != RCABF_OK) return s;
+    if ((s = finish_mask(g, a, st)) != RCABF_OK) return s;
     mark(a, 4, st);
     return RCABF_OK;
 }
@@ -669,7 +697,7 @@ int beamform_noalloc(rcabf_geometry *g, const rcabf_beamform_args *a, cudaStream
     if ((s = launch_fused_jobs(g, prm, p, st)) != RCABF_OK) return s;
     if ((s = finish_job(g, &b, p, prm.jobs[0], st)) != RCABF_OK) return s;
     mark(&b, 3, st);
-    if ((s = finish_mask(g, &b, p, st)) != RCABF_OK) return s;
+    if ((s = finish_mask(g, &b, st)) != RCABF_OK) return s;
     mark(&b, 4, st);
     return RCABF_OK;
 }
@@ -832,6 +860,7 @@ size_t align256(size_t x) { return (x + 255) / 256 * 256; }
 struct HostLayout {
     int64_t chunk = 0;
     size_t in_bytes = 0, out_bytes = 0, plan_bytes = 0, total = 0;
+    int n_split = 0;           // the whole call's transmit ranges (streaming kernel): every chunk sums as it does
     bool have_tuned = false;   // the autotuner's choice for the whole call, used by every chunk
     TuneChoice tuned;
 };
@@ -839,8 +868,8 @@ struct HostLayout {
 // Plan of one chunk: the whole call's tuned choice where one exists and fits.
 int chunk_plan(rcabf_geometry *g, const rcabf_beamform_args *c, const HostLayout &h, Plan &p)
 {
-    if (h.have_tuned && plan_beamform(g, c, p, &h.tuned) == RCABF_OK) return RCABF_OK;
-    return plan_beamform(g, c, p);
+    if (h.have_tuned && plan_beamform(g, c, p, &h.tuned, h.n_split) == RCABF_OK) return RCABF_OK;
+    return plan_beamform(g, c, p, nullptr, h.n_split);
 }
 
 int host_layout(rcabf_geometry *g, const rcabf_beamform_args *a, int32_t frames_per_chunk, HostLayout &h)
@@ -859,6 +888,7 @@ int host_layout(rcabf_geometry *g, const rcabf_beamform_args *a, int32_t frames_
         chunk = fb * ((n_fb + 3) / 4);
     }
     h.chunk = std::min<int64_t>(chunk, a->n_frame);
+    if (p.vb == 1) h.n_split = p.n_split;
     {
         std::lock_guard<std::mutex> lk(g->mu);
         auto it = g->tuned.find({a->n_frame, (int64_t)a->storage});
@@ -1036,7 +1066,7 @@ int rcabf_beamform_batch(int n, const rcabf_geometry *const *gs, const rcabf_bea
     if (s != RCABF_OK) return s;
     for (int i = 0; i < n; ++i) {
         if ((s = finish_job(gs[i], &as[i], plans[i], prm.jobs[i], st)) != RCABF_OK) return s;
-        if ((s = finish_mask(gs[i], &as[i], plans[i], st)) != RCABF_OK) return s;
+        if ((s = finish_mask(gs[i], &as[i], st)) != RCABF_OK) return s;
     }
     return RCABF_OK;
 }

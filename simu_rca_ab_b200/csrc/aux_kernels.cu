@@ -137,9 +137,10 @@ cudaError_t launch_range(const RangeParams &p, cudaStream_t st)
 // (pixel, tx) (RCA.cu:247-250, 301-304), summed over transmits when
 // compounding (RCA.m:696).
 // ------------------------------------------------------------------------
-__device__ __forceinline__ void mask_voxel(const DevGeom &g, float *mask, int compound, int accumulate, int64_t v)
+__global__ void mask_kernel(const DevGeom g, float *mask, int compound, int accumulate)
 {
     const int64_t n_vox = g.n_z * g.n_u * g.n_v;
+    const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= n_vox) return;
     const int64_t iz = v % g.n_z, iu = (v / g.n_z) % g.n_u, iv = v / (g.n_z * g.n_u);
     const int64_t rxkey = iu * g.n_z + iz, txkey = iv * g.n_z + iz;
@@ -164,11 +165,6 @@ __device__ __forceinline__ void mask_voxel(const DevGeom &g, float *mask, int co
     if (compound) mask[pix] = accumulate ? mask[pix] + total : total;
 }
 
-__global__ void mask_kernel(const DevGeom g, float *mask, int compound, int accumulate)
-{
-    mask_voxel(g, mask, compound, accumulate, (int64_t)blockIdx.x * blockDim.x + threadIdx.x);
-}
-
 cudaError_t launch_mask(const DevGeom &g, float *mask, int compound, int accumulate, cudaStream_t st)
 {
     const int64_t n = g.n_z * g.n_u * g.n_v;
@@ -181,7 +177,7 @@ cudaError_t launch_mask(const DevGeom &g, float *mask, int compound, int accumul
 // independent blocks: channel data -> FP32 slab rows (rounded through the
 // storage type, in the layout they are staged in: das_common.cuh's frame
 // pairs as (re, re, im, im), padded rows, zero rows past the record), the two
-// window range tables, the mask, and a zeroed work counter.  A call on a
+// window range tables, and a zeroed work counter.  A call on a
 // small grid is bound by launches and by the range kernel's few threads
 // (10-17 us each for one thread per table entry on the 64 x 64 x 128 grid);
 // here 16 lanes share an entry and all parts run at once.
@@ -197,14 +193,18 @@ __device__ __forceinline__ void prep_ingest(const IngestParams &p, int64_t i)
     const int64_t q = i / rows;                       // (tx, ele), frame block
     const int fb = (int)(q % p.n_fb);
     const int64_t te = q / p.n_fb;
-    if (te >= (int64_t)p.n_tx * p.n_ele) return;
+    if (te >= (int64_t)p.slab_tx * p.slab_ele) return;
     const int FB = p.fb;
     char *row = reinterpret_cast<char *>(p.S) + (te * p.n_fb + fb) * p.slab_bytes + (int64_t)n * vbs_row_bytes(FB);
-    const int64_t f0 = (int64_t)fb * FB, frame = (int64_t)p.n_tx * p.n_ele * p.n_sample;
-    const int64_t src = te * p.n_sample + n;
-    auto sample = [&](int64_t f) {
-        if (n >= p.n_sample || f >= p.n_frame) return make_float2(0.f, 0.f);
-        return to_f2(from_f2<STORE>(load_iq<IQ>(p.iq, f * frame + src)));
+    const int64_t f0 = (int64_t)fb * FB;
+    const int tx = (int)(te / p.slab_ele), ele = (int)(te % p.slab_ele);
+    const unsigned sh = p.n_sym == 4 ? 2 : p.n_sym == 2 ? 1 : 0;
+    auto sample = [&](int64_t f) {   // copy f mod n_sym of frame f / n_sym
+        const int64_t fr = f >> sh;
+        if (n >= p.n_sample || fr >= p.n_frame) return make_float2(0.f, 0.f);
+        const int m = vbs_mirrored(p.mirror, (int)f & (p.n_sym - 1));
+        const int t = m & VBS_MIRROR_V ? p.n_tx - 1 - tx : tx, e = m & VBS_MIRROR_U ? p.n_ele - 1 - ele : ele;
+        return to_f2(from_f2<STORE>(load_iq<IQ>(p.iq, ((fr * p.n_tx + t) * p.n_ele + e) * p.n_sample + n)));
     };
     if (FB == 1) {
         *reinterpret_cast<float2 *>(row) = sample(f0);
@@ -227,7 +227,7 @@ __device__ __forceinline__ void prep_range(const RangeParams &p, int64_t i, int 
         const int tai = (int)((i / p.tiles_z) % p.tiles_a);
         const float4 *tab = p.tab + i / ((int64_t)p.tiles_z * p.tiles_a) * p.n_a * p.n_z;
         const int nz = (int)min((int64_t)p.tz, p.n_z - (int64_t)tzi * p.tz);
-        const int na = (int)min((int64_t)p.ta, p.n_a - (int64_t)tai * p.ta);
+        const int na = (int)min((int64_t)p.ta, p.n_lim - (int64_t)tai * p.ta);
         for (int k = lane; k < na * nz; k += RANGE_LANES) {
             const float4 e = __ldg(&tab[((int64_t)tai * p.ta + k / nz) * p.n_z + (int64_t)tzi * p.tz + k % nz]);
             if (!p.is_rx || e.w > 0.0f) { lo = fminf(lo, e.x); hi = fmaxf(hi, e.x); }
@@ -253,11 +253,7 @@ __global__ void __launch_bounds__(PREP_THREADS) prep_kernel(const __grid_constan
         return;
     }
     b -= p.blocks_rx + p.blocks_tx;
-    if (b < p.blocks_mask) {
-        mask_voxel(p.g, p.mask, p.compound, p.accumulate, b * PREP_THREADS + threadIdx.x);
-        return;
-    }
-    prep_ingest<STORE, IQ>(p.ingest, (b - p.blocks_mask) * PREP_THREADS + threadIdx.x);
+    prep_ingest<STORE, IQ>(p.ingest, b * PREP_THREADS + threadIdx.x);
 }
 
 template <int STORE>
@@ -276,9 +272,8 @@ cudaError_t launch_prep(PrepParams &p, int store, cudaStream_t st)
     auto blocks = [](int64_t n) { return (n + PREP_THREADS - 1) / PREP_THREADS; };
     p.blocks_rx = blocks(p.rx.rows * p.rx.tiles_a * p.rx.tiles_z * RANGE_LANES);
     p.blocks_tx = blocks(p.tx.rows * p.tx.tiles_a * p.tx.tiles_z * RANGE_LANES);
-    p.blocks_mask = p.mask ? blocks(p.g.n_z * p.g.n_u * p.g.n_v) : 0;
-    const int64_t n = p.blocks_rx + p.blocks_tx + p.blocks_mask +
-                      blocks((int64_t)p.ingest.n_tx * p.ingest.n_ele * p.ingest.n_fb * p.ingest.n_rows);
+    const int64_t n = p.blocks_rx + p.blocks_tx +
+                      blocks((int64_t)p.ingest.slab_tx * p.ingest.slab_ele * p.ingest.n_fb * p.ingest.n_rows);
     if (n > INT32_MAX || p.ingest.iq_dtype < 0 || p.ingest.iq_dtype > 3) return cudaErrorInvalidValue;
     switch (store) {
     case ST_F32: launch_prep_store<ST_F32>(p, (unsigned)n, st); break;

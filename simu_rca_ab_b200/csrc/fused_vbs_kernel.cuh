@@ -21,12 +21,16 @@
 //     assignment leaves SMs idle at the end), and the scan runs on into the
 //     next item while the current one is computed.
 //
-// Measured (B200, against the barrier-per-step kernels it replaced): 8 frames,
-// 128 x 128 x 256, two orientations 257 -> 152 ms; 4 frames of a 256-element
-// probe 361 -> 252 ms; 20 frames, 97 x 95 x 159 47.3 -> 31.0 ms; one frame, 64 x
-// 64 x 128 9.38 -> 1.60 ms; one frame, 32 x 32 x 64, 4 transmits 455 -> 115 us.
-// What bounds it: instruction issue (64 % of the cycles for one frame, 337
-// instructions per warp and active step, about 140 of them on weights).
+// Measured (B200, against the barrier-per-step kernels it replaced; without
+// and with mirrored copies): 8 frames, 128 x 128 x 256, two orientations 257 ->
+// 152 -> 155 ms; 4 frames of a 256-element probe 361 -> 252 -> 212 ms; 20 frames,
+// 97 x 95 x 159 47.3 -> 31.0 -> 30.0 ms; one frame, 64 x 64 x 128 9.38 -> 1.60 ->
+// 0.94 ms; one frame, 32 x 32 x 64, 4 transmits 455 -> 115 -> 98 us.
+// What bounds it: instruction issue (without copies 64 % of the cycles for one
+// frame, 337 instructions per warp and active step, 140 of them on weights).
+//
+// Grids centred on the probe and symmetric transmits: the voxels of half the u
+// (v) axis carry their mirror images as further frames (VBS_MIRROR_*).
 //
 // D >= 1: the four voxels share TAPS + D staged rows (weights shifted to each
 // voxel's first row, zeros elsewhere): one 16-byte load feeds 16 FMAs.
@@ -51,14 +55,12 @@ constexpr int VS_WARPS = VS_THREADS / 32;
 constexpr float VS_MAGIC = 12582912.0f;
 constexpr int VS_MAGIC_BITS = 0x4B400000;
 
-// CTAs per SM the registers are budgeted for: 2 x 4 x FB accumulators, the
-// weights and the per-voxel transmit state.
-constexpr int vs_min_blocks(int fb) { return fb >= 8 ? 2 : fb >= 4 ? 3 : 4; }
-
-// One step of a chunk: staged rows [lo, lo + count) of (tx, rx).
+// One step of a chunk: staged rows [lo, lo + count) of (tx, rx); the top bits
+// of `count` hold the step's place m among the steps its slab serves.
 struct __align__(16) VsRec {
     int32_t lo, count, tx, rx;
 };
+constexpr int VS_M_SHIFT = 28;
 // One chunk: n records of work item `item` (-1: no more items), `last` the
 // item's last chunk.
 struct __align__(16) VsChunkInfo {
@@ -123,7 +125,7 @@ struct VsScan {
 };
 
 template <int KIND, int FB, int DEG, int D>
-__global__ void __launch_bounds__(VS_THREADS, vs_min_blocks(FB)) fused_vbs_kernel(const __grid_constant__ FusedParams prm)
+__global__ void __launch_bounds__(VS_THREADS, vbs_min_ctas(FB)) fused_vbs_kernel(const __grid_constant__ FusedParams prm)
 {
     static_assert(VB_BLOCK == 4, "weights are formed for two pairs of voxels");
     static_assert(FB == 1 || FB % 2 == 0, "frames are processed in pairs");
@@ -134,6 +136,7 @@ __global__ void __launch_bounds__(VS_THREADS, vs_min_blocks(FB)) fused_vbs_kerne
     constexpr int R = TAPS + D;                  // rows a thread reads per step and block (D = 0: per voxel)
     constexpr int STRIDE = vbs_row_bytes(FB);
     constexpr int NP = FB == 1 ? 1 : FB / 2;     // frame pairs
+    constexpr bool OWN = FB <= 4;                // a block one frame's mirrored copies fill
 
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ uint64_t full[VS_STAGES], empty[VS_STAGES];
@@ -267,11 +270,18 @@ __global__ void __launch_bounds__(VS_THREADS, vs_min_blocks(FB)) fused_vbs_kerne
                 if (mine) {
                     const int slot = n + rank;
                     step_of(k, k.base - 32 + lane, n_ele, tx, rx);
-                    recs[st][slot] = VsRec{lo, cnt, tx, rx};
+                    int m = 0, slab = tx * n_ele + rx;
+                    if (J.compact) {
+                        const bool mu = (J.mirror & VBS_MIRROR_U) && rx > n_ele - 1 - rx;
+                        const bool mv = (J.mirror & VBS_MIRROR_V) && tx > J.g.n_tx - 1 - tx;
+                        slab = (mv ? J.g.n_tx - 1 - tx : tx) * (J.mirror & VBS_MIRROR_U ? (n_ele + 1) / 2 : n_ele) +
+                               (mu ? n_ele - 1 - rx : rx);
+                        m = J.n_sym == 4 ? (mu ? 1 : 0) | (mv ? 2 : 0) : mu || mv ? 1 : 0;
+                    }
+                    recs[st][slot] = VsRec{lo, cnt | m << VS_M_SHIFT, tx, rx};
                     const uint32_t b = ((uint32_t)(cnt * STRIDE) + 15u) & ~15u;
                     bulk_load(slot0 + (uint32_t)slot * slot_bytes,
-                              S + (((int64_t)tx * n_ele + rx) * J.n_fb + k.it.fb) * J.slab_bytes + (int64_t)lo * STRIDE,
-                              b, &full[st]);
+                              S + ((int64_t)slab * J.n_fb + k.it.fb) * J.slab_bytes + (int64_t)lo * STRIDE, b, &full[st]);
                     bytes += b;
                 }
                 const unsigned took = __ballot_sync(0xffffffffu, mine);
@@ -303,6 +313,7 @@ __global__ void __launch_bounds__(VS_THREADS, vs_min_blocks(FB)) fused_vbs_kerne
 
     // ---------------- state of the item being computed ----------------
     int cur = -1, cur_tx = -1, job = 0, n_pair = 0;
+    int cur_m = 0;                            // the accumulators' slot s holds copy s ^ cur_m
     int iz = 0, iu = 0, iv0 = 0, nvv = 0;     // the thread's first voxel, and how many of its four are on the grid
     const float4 *rxp = nullptr;              // receive table entry of element 0, and the elements' stride
     int rx_stride = 0;
@@ -324,6 +335,7 @@ __global__ void __launch_bounds__(VS_THREADS, vs_min_blocks(FB)) fused_vbs_kerne
         if (ck.item != cur) {
             cur = ck.item;
             cur_tx = -1;
+            cur_m = 0;
             const VsItem ci = vs_item(prm, cur);
             job = ci.job;
             const FusedJob &J = prm.jobs[job];
@@ -331,13 +343,13 @@ __global__ void __launch_bounds__(VS_THREADS, vs_min_blocks(FB)) fused_vbs_kerne
             iz = ci.tz * J.tz + lz;
             iu = ci.tu * J.tu + lu;
             iv0 = (ci.tv * J.tv + lvb) * VB;
-            const int rem = (int)J.g.n_v - iv0;
-            nvv = !(iz < J.g.n_z && iu < J.g.n_u) || rem <= 0 ? 0 : rem >= VB ? VB : rem;
+            const int rem = J.nv_t - iv0;
+            nvv = !(iz < J.g.n_z && iu < J.nu_t) || rem <= 0 ? 0 : rem >= VB ? VB : rem;
             rxp = J.g.rx_tab + (nvv > 0 ? (int64_t)iu * J.g.n_z + iz : 0);   // off the grid: any entry, never used
             rx_stride = (int)(J.g.n_u * J.g.n_z);
             lim = (float)(J.n_sample - 1 - KT::HI);
             has_ab = J.g.ab != nullptr;
-            n_pair = FB == 1 ? 1 : (min(FB, J.n_frame - ci.fb * FB) + 1) / 2;
+            n_pair = FB == 1 ? 1 : (min(FB, J.n_vf - ci.fb * FB) + 1) / 2;
 #pragma unroll
             for (int v = 0; v < VB; ++v)
 #pragma unroll
@@ -349,7 +361,9 @@ __global__ void __launch_bounds__(VS_THREADS, vs_min_blocks(FB)) fused_vbs_kerne
         const uint32_t slot0 = sbase + (uint32_t)(st * krec) * slot_bytes;
         if (!have_e && ck.n > 0) enext = __ldg(rxp + (int64_t)recs[st][0].rx * rx_stride);
         for (int i = 0; i < ck.n; ++i) {
-            const VsRec h = recs[st][i];
+            VsRec h = recs[st][i];
+            const int m = (int)((unsigned)h.count >> VS_M_SHIFT);
+            h.count &= (1 << VS_M_SHIFT) - 1;
             const float4 e = enext;
             if (i + 1 < ck.n) enext = __ldg(rxp + (int64_t)recs[st][i + 1].rx * rx_stride);
             if (h.tx != cur_tx) {
@@ -373,6 +387,34 @@ __global__ void __launch_bounds__(VS_THREADS, vs_min_blocks(FB)) fused_vbs_kerne
                         txr[j] = make_float2(t[2 * j].y, t[2 * j + 1].y);
                         txq[j] = make_float2(t[2 * j].z, t[2 * j + 1].z);
                     }
+                }
+            }
+            if constexpr (FB >= 2) {
+                if (m != cur_m) {   // half-way through the elements (transmits): the copies' slots swap
+                    if ((m ^ cur_m) & 1) {
+#pragma unroll
+                        for (int v = 0; v < VB; ++v)
+#pragma unroll
+                            for (int p = 0; p < NP; ++p) {
+                                are[v][p] = make_float2(are[v][p].y, are[v][p].x);
+                                aim[v][p] = make_float2(aim[v][p].y, aim[v][p].x);
+                            }
+                    }
+                    if constexpr (FB >= 4) {
+                        if ((m ^ cur_m) & 2) {
+#pragma unroll
+                            for (int v = 0; v < VB; ++v)
+#pragma unroll
+                                for (int p = 0; p < NP; p += 2) {
+                                    const float2 r = are[v][p], q = aim[v][p];
+                                    are[v][p] = are[v][p + 1];
+                                    aim[v][p] = aim[v][p + 1];
+                                    are[v][p + 1] = r;
+                                    aim[v][p + 1] = q;
+                                }
+                        }
+                    }
+                    cur_m = m;
                 }
             }
             if (cone_bits == 0 || !(e.w > 0.0f)) continue;
@@ -487,7 +529,16 @@ __global__ void __launch_bounds__(VS_THREADS, vs_min_blocks(FB)) fused_vbs_kerne
                     atomicAdd(prm.err_count, 1ull);   // never expected: window bound violated
                     continue;
                 }
+                // weights shifted to each voxel's first row; rows 0 .. D-1 and
+                // TAPS .. R-1 are taken by some of the voxels only.  OWN: the
+                // others leave them out (and a voxel without a contribution
+                // leaves its sums alone), so that a NaN or infinite sample
+                // reaches no voxel whose taps do not touch it, as in the
+                // one-voxel kernel that single frames ran on.  Otherwise they
+                // add zero times the row, as the tensor-memory kernel does
+                // (leaving them out measured 11 % on 8 frames, 10 % on one)
                 float ws[VB][R];
+                bool s1[VB], s2[VB];
 #pragma unroll
                 for (int j = 0; j < 2; ++j) {
                     float2 w[TAPS];
@@ -497,22 +548,32 @@ __global__ void __launch_bounds__(VS_THREADS, vs_min_blocks(FB)) fused_vbs_kerne
                         const int v = 2 * j + h2;
                         const float sh = (h2 ? fl[j].y : fl[j].x) - base;   // rows of shift
                         if (ok[v] && sh > (float)D + 0.5f) { atomicAdd(prm.err_count, 1ull); ok[v] = false; }
-                        const bool s1 = sh > 0.5f, s2 = sh > 1.5f;
+                        s1[v] = sh > 0.5f;
+                        s2[v] = D >= 2 && sh > 1.5f;
 #pragma unroll
                         for (int k = 0; k < R; ++k) {
-                            auto wt = [&](int q) { return q >= 0 && q < TAPS ? (h2 ? w[q].y : w[q].x) : 0.0f; };
+                            auto wt = [&](int q) {   // OWN: rows the voxel leaves out may carry any weight
+                                const int c = q < 0 ? 0 : q < TAPS ? q : TAPS - 1;
+                                return OWN || c == q ? (h2 ? w[c].y : w[c].x) : 0.0f;
+                            };
                             float a = wt(k);
-                            if (s1) a = wt(k - 1);
-                            if constexpr (D >= 2) { if (s2) a = wt(k - 2); }
+                            if (s1[v]) a = wt(k - 1);
+                            if constexpr (D >= 2) { if (s2[v]) a = wt(k - 2); }
                             ws[v][k] = a;
                         }
                     }
                 }
+                auto uses = [&](int v, int k) {   // whether voxel v adds row k
+                    if (!OWN || (k >= D && k < TAPS)) return true;
+                    if constexpr (D == 1) return k == 0 ? !s1[v] : s1[v];
+                    else return k == 0 ? !s1[v] : k == 1 ? !s2[v] : k == TAPS ? s1[v] : s2[v];
+                };
                 float px[VB], py[VB];
 #pragma unroll
                 for (int v = 0; v < VB; ++v) {
-                    px[v] = ok[v] ? (v & 1 ? Px[v >> 1].y : Px[v >> 1].x) : 0.0f;
-                    py[v] = ok[v] ? (v & 1 ? Py[v >> 1].y : Py[v >> 1].x) : 0.0f;
+                    const bool use = OWN || ok[v];
+                    px[v] = use ? (v & 1 ? Px[v >> 1].y : Px[v >> 1].x) : 0.0f;
+                    py[v] = use ? (v & 1 ? Py[v >> 1].y : Py[v >> 1].x) : 0.0f;
                 }
                 const uint32_t a0 = slot0 + (uint32_t)i * slot_bytes + (uint32_t)(row0 * STRIDE);
 #pragma unroll
@@ -527,12 +588,15 @@ __global__ void __launch_bounds__(VS_THREADS, vs_min_blocks(FB)) fused_vbs_kerne
 #pragma unroll
                             for (int v = 0; v < VB; ++v) {
                                 const float2 w2 = make_float2(ws[v][k], ws[v][k]);
-                                tre[v] = __ffma2_rn(w2, make_float2(x.x, x.y), tre[v]);
-                                tim[v] = __ffma2_rn(w2, make_float2(x.z, x.w), tim[v]);
+                                if (uses(v, k)) {
+                                    tre[v] = __ffma2_rn(w2, make_float2(x.x, x.y), tre[v]);
+                                    tim[v] = __ffma2_rn(w2, make_float2(x.z, x.w), tim[v]);
+                                }
                             }
                         }
 #pragma unroll
                         for (int v = 0; v < VB; ++v) {
+                            if (OWN && !ok[v]) continue;
                             const float2 p2 = make_float2(px[v], px[v]);
                             are[v][p] = __ffma2_rn(p2, tre[v], __ffma2_rn(make_float2(-py[v], -py[v]), tim[v], are[v][p]));
                             aim[v][p] = __ffma2_rn(p2, tim[v], __ffma2_rn(make_float2(py[v], py[v]), tre[v], aim[v][p]));
@@ -549,32 +613,38 @@ __global__ void __launch_bounds__(VS_THREADS, vs_min_blocks(FB)) fused_vbs_kerne
             // compounded), or this transmit range's part of it
             const VsItem ci = vs_item(prm, cur);
             cur = -1;
-            const int64_t pix0 = iz * g.s_z + iu * g.s_u + (int64_t)iv0 * g.s_v;
             float2 *out = J.out;
-            int64_t stride = g.n_pix, off = 0;
+            int64_t stride = g.n_pix;
             bool add = J.accumulate != 0;
             if (!J.compound) {
                 stride = (int64_t)g.n_tx * g.n_pix;
-                off = (int64_t)ci.tx0 * g.n_pix;
             } else if (J.n_split > 1) {
                 out = J.partial + (int64_t)ci.split * J.n_frame * g.n_pix;
                 add = false;
             }
 #pragma unroll
-            for (int v = 0; v < VB; ++v) {
-                if (v < nvv) {
+            for (int f = 0; f < FB; ++f) {
+                const int vf = ci.fb * FB + f;
+                if (vf >= J.n_vf) continue;
+                const int fr = J.n_sym == 1 ? vf : vf / J.n_sym;
+                const int m = vbs_mirrored(J.mirror, (vf - fr * J.n_sym) ^ cur_m);
+                const int ou = m & VBS_MIRROR_U ? (int)g.n_u - 1 - iu : iu;
+                if ((m & VBS_MIRROR_U) && ou == iu) continue;   // the middle column: the unmirrored copy writes it
+                // not compounded: copy m of transmit tx0 is the mirrored transmit's
+                const int64_t off = J.compound ? 0
+                                               : (int64_t)(m & VBS_MIRROR_V ? g.n_tx - 1 - ci.tx0 : ci.tx0) * g.n_pix;
+                float2 *o0 = out + (int64_t)fr * stride + off + iz * g.s_z + ou * g.s_u;
 #pragma unroll
-                    for (int f = 0; f < FB; ++f) {
-                        const int fr = ci.fb * FB + f;
-                        if (fr < J.n_frame) {
-                            float2 a;
-                            if constexpr (FB == 1) a = are[v][0];
-                            else a = f & 1 ? make_float2(are[v][f >> 1].y, aim[v][f >> 1].y)
-                                           : make_float2(are[v][f >> 1].x, aim[v][f >> 1].x);
-                            float2 *o = out + (int64_t)fr * stride + off + pix0 + v * g.s_v;
-                            if (add) { float2 q = *o; q.x += a.x; q.y += a.y; *o = q; }
-                            else *o = a;
-                        }
+                for (int v = 0; v < VB; ++v) {
+                    const int iv = iv0 + v, ov = m & VBS_MIRROR_V ? (int)g.n_v - 1 - iv : iv;
+                    if (v < nvv && !((m & VBS_MIRROR_V) && ov == iv)) {
+                        float2 a;
+                        if constexpr (FB == 1) a = are[v][0];
+                        else a = f & 1 ? make_float2(are[v][f >> 1].y, aim[v][f >> 1].y)
+                                       : make_float2(are[v][f >> 1].x, aim[v][f >> 1].x);
+                        float2 *o = o0 + ov * g.s_v;
+                        if (add) { float2 q = *o; q.x += a.x; q.y += a.y; *o = q; }
+                        else *o = a;
                     }
                 }
             }

@@ -106,6 +106,29 @@ void free_geometry(rcabf_geometry *g)
     delete g;
 }
 
+// Axes along which the tables are mirror-symmetric: entry (row, a, z) against
+// (rows - 1 - row, n_a - 1 - a, z), the same valid entries, delays and phasors
+// equal to the rounding of the FP32 entries (positions that mirror each other
+// exactly differ in the last bits of their FP64 delays).
+static int mirror_axes(const rcabf_geometry &g, const std::vector<float4> &rx, const std::vector<float4> &tx)
+{
+    auto symmetric = [&](const std::vector<float4> &tab, int64_t rows, int64_t n_a) {
+        for (int64_t r = 0; 2 * r < rows; ++r)
+            for (int64_t a = 0; a < n_a; ++a)
+                for (int64_t z = 0; z < g.n_z; ++z) {
+                    const float4 p = tab[(size_t)((r * n_a + a) * g.n_z + z)];
+                    const float4 q = tab[(size_t)(((rows - 1 - r) * n_a + n_a - 1 - a) * g.n_z + z)];
+                    if ((p.w > 0.f) != (q.w > 0.f)) return false;
+                    if (!(p.w > 0.f)) continue;
+                    if (!(std::fabs(p.x - q.x) <= 1.2e-7f * std::fabs(p.x)) || !(std::fabs(p.y - q.y) <= 2.5e-7f) ||
+                        !(std::fabs(p.z - q.z) <= 2.5e-7f) || !(std::fabs(p.w - q.w) <= 2.5e-7f))
+                        return false;
+                }
+        return true;
+    };
+    return (symmetric(rx, g.n_ele, g.n_u) ? VBS_MIRROR_U : 0) | (symmetric(tx, g.n_tx, g.n_v) ? VBS_MIRROR_V : 0);
+}
+
 int build_geometry(const rcabf_geometry_desc *d, cudaStream_t st, rcabf_geometry **out)
 {
     if (!d || !out) return RCABF_ERR_INVALID_ARGUMENT;
@@ -315,6 +338,7 @@ int build_geometry(const rcabf_geometry_desc *d, cudaStream_t st, rcabf_geometry
                 tx_tab[t * n_txkey + k] = make_float4((float)itx, pc, ps, cone ? 1.f : 0.f);
                 g->tx_delay[t * n_txkey + k] = (float)itx;
             }
+        g->mirror = d->ab_law || d->grid_kind != RCABF_GRID_RECTILINEAR ? 0 : mirror_axes(*g, rx_tab, tx_tab);
         std::vector<float> apod_sum(apod_sum_d.begin(), apod_sum_d.end());
         if ((ce = upload(&g->rx_tab, rx_tab, st)) != cudaSuccess) goto cuda_fail;
         if ((ce = upload(&g->tx_tab, tx_tab, st)) != cudaSuccess) goto cuda_fail;
@@ -324,6 +348,13 @@ int build_geometry(const rcabf_geometry_desc *d, cudaStream_t st, rcabf_geometry
             for (int64_t t = 0; t < nt; ++t)
                 for (int64_t k = 0; k < n_rxkey; ++k)
                     cu[t * n_rxkey + k] = cone_half(vs_u[t], g->vs_z[t], half_u, g->ap_z, rk_u(k), k_z(k)) ? 1 : 0;
+            // the cone along u: the same at -u, and for the mirrored transmit
+            for (int64_t t = 0; t < nt && g->mirror; ++t)
+                for (int64_t k = 0; k < n_rxkey; ++k) {
+                    const int64_t m = (g->n_u - 1 - k / g->n_z) * g->n_z + k % g->n_z;
+                    if (cu[t * n_rxkey + k] != cu[t * n_rxkey + m]) g->mirror &= ~VBS_MIRROR_U;
+                    if (cu[t * n_rxkey + k] != cu[(nt - 1 - t) * n_rxkey + k]) g->mirror &= ~VBS_MIRROR_V;
+                }
             if ((ce = upload(&g->cone_u, cu, st)) != cudaSuccess) goto cuda_fail;
         }
         if (d->ab_law) {

@@ -69,6 +69,7 @@ struct rcabf_geometry {
     float2 *ab_ph = nullptr;
     float *wtab = nullptr;
     rcabf::RefScalars ref{};
+    int mirror = 0;               // VBS_MIRROR_*: axes along which the tables are symmetric
 
     std::mutex mu;
     std::map<rcabf::TileShape, rcabf::TileSpread> spreads;

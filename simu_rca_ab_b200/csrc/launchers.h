@@ -17,12 +17,16 @@ struct IngestParams {
     int64_t slab_bytes;
     int32_t n_rows;        // rows written per slab: n_sample, or more with zero rows past the record
     void *S2;              // NULL, or a second slab set of the same layout holding (-im, re)
+    // streaming kernel: copies of a frame and the axes they mirror
+    // (VBS_MIRROR_*), and the transmits and elements that have a slab
+    int32_t n_sym, mirror, slab_tx, slab_ele;
 };
 
 struct RangeParams {
     const float4 *tab;
     float2 *out;
     int64_t rows, n_a, n_z;
+    int64_t n_lim;             // streaming kernel: extent along a the tiles cover (at most n_a)
     int32_t ta, tz, tiles_a, tiles_z;
     int32_t mode, is_rx;
 };
@@ -32,11 +36,8 @@ struct RangeParams {
 struct PrepParams {
     IngestParams ingest;       // n_rows: slab rows, the record and its zero rows
     RangeParams rx, tx;
-    DevGeom g;
-    float *mask;               // NULL: no mask
-    int32_t compound, accumulate;
     uint32_t *counter;         // zeroed
-    int64_t blocks_rx, blocks_tx, blocks_mask;
+    int64_t blocks_rx, blocks_tx;
 };
 
 // Inputs of the REF_COMPAT table kernels: single-precision copies of what the

@@ -19,6 +19,10 @@ struct Plan {
     // (fused_vbs_kernel.cuh), 2 TMEM accumulators (fused_vb_kernel.cuh)
     int vb = 0;
     int n_split = 1;      // vb = 1: transmit ranges, one work item each
+    int mirror = 0, n_sym = 1;          // vb = 1: mirrored axes, copies of a frame (VBS_MIRROR_*)
+    int64_t nu_t = 0, nv_t = 0;         // vb = 1: tile-space extents
+    int compact = 0;                    // vb = 1: one slab for the steps that mirror each other
+    int slab_tx = 0, slab_ele = 0;      // transmits and elements that have a slab
     int tc = 0;           // tensor-core kernel (fused_tc_kernel.cuh): 1 FP16 weights, 2 hi + remainder weights
     int tc_rows = 0;      // its slab rows (the record + zero rows a window may reach past it)
     int d = 0;            // voxel-blocked kernels: row shift bound (0: every voxel reads its own rows)
@@ -36,7 +40,9 @@ struct Plan {
 // force: a launch choice to plan instead of the planner's own (autotuner);
 // without one, a choice rcabf_autotune stored for these frames and storage
 // is used.  RCABF_ERR_UNSUPPORTED when a forced choice does not fit.
-int plan_beamform(rcabf_geometry *g, const rcabf_beamform_args *a, Plan &p, const TuneChoice *force = nullptr);
+// split_req: transmit ranges of the streaming kernel (0: the planner's number).
+int plan_beamform(rcabf_geometry *g, const rcabf_beamform_args *a, Plan &p, const TuneChoice *force = nullptr,
+                  int split_req = 0);
 
 // Smaller-workspace replacement of a streaming-kernel plan (api.cpp).
 void plan_compact(rcabf_geometry *g, rcabf_beamform_args &a, Plan &p);
@@ -70,8 +76,7 @@ inline size_t vb_smem_bytes(int store, int wmax, int row_words, int zero_rows = 
 // (0: not even one).
 inline int vbs_chunk_records(int fb, int wmax)
 {
-    const int ctas = fb >= 8 ? 2 : fb >= 4 ? 3 : 4;
-    const int n = (int)((224 * 1024 / ctas - 2048) / (3 * (size_t)vbs_slot_bytes(fb, wmax)));
+    const int n = (int)((224 * 1024 / vbs_min_ctas(fb) - 2048) / (3 * (size_t)vbs_slot_bytes(fb, wmax)));
     return n > VBS_MAX_RECORDS ? VBS_MAX_RECORDS : n;
 }
 inline size_t vbs_smem_bytes(int fb, int wmax) { return 3 * (size_t)vbs_chunk_records(fb, wmax) * vbs_slot_bytes(fb, wmax); }

@@ -86,6 +86,10 @@ struct FusedJob {
     int32_t compound, accumulate;
     int32_t tiles_z, tiles_u, tiles_v;
     int32_t tu, tv, tz;        // tile shape, tu*tv*tz = blockDim.x
+    // streaming kernel: tile-space extents (halved along a mirrored axis), the
+    // copies of a frame a block holds (1, 2 or 4: see VBS_MIRROR_*), frames x copies
+    int32_t nu_t, nv_t;
+    int32_t n_sym, mirror, n_vf, compact;
     int32_t n_split;           // streaming kernel: transmit ranges, an item each (n_tx when not compounded)
     float2 *partial;           // its sums per range [n_split][frame][pix] when compounded and n_split > 1
 };
@@ -111,9 +115,30 @@ constexpr RCABF_HD int vb_tmem_cols_host(int fb) { return fb * 8 <= 32 ? 32 : fb
 // most, the longest record its floor() covers, FP32 slab rows in the layout
 // they are staged in (frame pairs as (re, re, im, im), rows of 4 frames or
 // more padded by 16 bytes so that 8 consecutive rows start in distinct banks).
+// Mirror symmetry.  On a grid centred on the probe, the voxel at -u sees
+// element E-1-r as the voxel at u sees element r, and with transmits steered
+// symmetrically the voxel at -v sees transmit T-1-t as the voxel at v sees t:
+// the same delays, weights, apodisation and phasors.  The streaming kernel then
+// covers u >= 0 (v >= 0) only and carries the mirrored voxels as further
+// "frames" of the block whose samples come from the mirrored element
+// (transmit): the per-step work is shared by 2 or 4 times the frames.
+// The steps (t, r), (t, E-1-r), (T-1-t, r), (T-1-t, E-1-r) read the same samples
+// in another order of the copies, so one slab serves all of them where a block
+// holds whole frames (`compact`): slot s of a row is copy s ^ m of step m of
+// the four, and the kernel keeps its accumulators in slot order.
+constexpr int VBS_MIRROR_U = 1, VBS_MIRROR_V = 2;
+// copy s of a frame (s < n_sym) -> the axes it mirrors
+constexpr RCABF_HD int vbs_mirrored(int mirror, int s)
+{
+    return mirror == (VBS_MIRROR_U | VBS_MIRROR_V) ? s : s ? mirror : 0;
+}
 constexpr int VBS_MAX_RECORDS = 8;
 constexpr int VBS_MAX_SAMPLES = 1 << 21;
-constexpr int VBS_MIN_ITEMS = 8 * 148;   // work items below which a grid is split by transmits
+// CTAs per SM its registers are budgeted for: 2 x 4 x FB accumulators, the
+// weights and the per-voxel transmit state.  With 8 frames a third CTA (168
+// registers, spills) measured 6 % slower than two; with 4 a fourth 4 % slower
+// than three.
+constexpr RCABF_HD int vbs_min_ctas(int fb) { return fb >= 8 ? 2 : fb >= 4 ? 3 : 4; }
 constexpr int VBS_PAD_ROWS = 2;      // zero rows past the record (shift rows)
 constexpr RCABF_HD int vbs_row_bytes(int fb) { return fb <= 2 ? 8 * fb : 8 * fb + 16; }
 constexpr RCABF_HD int vbs_slot_bytes(int fb, int wmax) { return (wmax * vbs_row_bytes(fb) + 15) / 16 * 16; }

@@ -97,3 +97,42 @@ def test_stream_kernel_interpolations_masks_and_outputs(cuda, interp, receive_x,
     for nf, ns in ((1, 150), (6, 97)):      # 97 samples: the record ends inside the grid
         case = _case(31, 12, 18, 3.0, interp, receive_x, mask_tx, n_tx=5, shift=shift)
         assert _check(case, nf, ns, compound=compound) < TOL[8]
+
+
+@pytest.mark.parametrize("nx,ny,n_tx,n_ele", [(16, 32, 4, 24), (15, 31, 5, 25), (16, 5, 3, 24), (3, 32, 4, 25),
+                                              (15, 31, 1, 24)])
+@pytest.mark.parametrize("n_frame,compound,receive_x", [(1, True, True), (2, True, False), (3, False, True),
+                                                        (5, True, True)])
+def test_mirrored_grids(cuda, nx, ny, n_tx, n_ele, n_frame, compound, receive_x):
+    """Grids centred on the probe, both axes or one mirrored, odd and even
+    counts of columns, elements and transmits (the middle ones mirror
+    themselves)."""
+    if not receive_x:
+        nx, ny = ny, nx
+    case = _case(18, nx, ny, 3.0, L3, receive_x, True, n_tx=n_tx, n_ele=n_ele)
+    assert _check(case, n_frame, 170, compound=compound) < TOL[8]
+
+
+@pytest.mark.parametrize("shift", [0.0, 0.4e-3])
+def test_a_bad_sample_stays_in_its_voxels(cuda, shift):
+    """A NaN and an infinite sample of a single frame reach the voxels whose
+    taps touch them, and no others: the plain kernel's set."""
+    import torch
+    from simu_rca_ab_b200 import _lib as L
+    from simu_rca_ab_b200 import beamformer as B
+    from simu_rca_ab_b200.params import normalize
+    G, T, P, O, n_tx, n_ele = _case(18, 15, 31, 3.0, L4, shift=shift)
+    n_frame = 1
+    eng = B.default_engine()
+    with warnings.catch_warnings():
+        warnings.simplefilter("ignore")
+        geom = eng.geometry(normalize(np.zeros(1, np.complex64), G, T, P, O))
+    g = torch.Generator(device="cuda").manual_seed(5)
+    iq = torch.randn(n_frame, n_tx, n_ele, 170, dtype=torch.complex64, device="cuda", generator=g)
+    iq[0, 1, 7, 60] = float("nan")
+    iq[-1, 0, 20, 95] = float("inf")
+    out, _ = eng.beamform(geom, iq)
+    ref, _ = eng.beamform(geom, iq, kernel=L.KERNEL_PLAIN)
+    bad, want = ~torch.isfinite(out.real + out.imag), ~torch.isfinite(ref.real + ref.imag)
+    assert torch.equal(bad, want) and 0 < int(want.sum()) < want.numel() // 2
+    assert _errcount() == 0
