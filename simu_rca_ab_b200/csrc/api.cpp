@@ -131,7 +131,7 @@ int choose_fb(const rcabf_geometry *g, int store, int64_t n_frame, int requested
     return best;
 }
 
-int plan_beamform(rcabf_geometry *g, const rcabf_beamform_args *a, Plan &p, const TuneChoice *force, int split_req)
+int plan_beamform(rcabf_geometry *g, const rcabf_beamform_args *a, Plan &p, const TuneChoice *force, const Plan *like)
 {
     if (!g || !a) return RCABF_ERR_INVALID_ARGUMENT;
     if (a->struct_size != (int32_t)sizeof(rcabf_beamform_args)) return RCABF_ERR_INVALID_ARGUMENT;
@@ -303,16 +303,24 @@ int plan_beamform(rcabf_geometry *g, const rcabf_beamform_args *a, Plan &p, cons
         const int64_t tiles = n_tiles(g->n_z, vts.tz) *
                               n_tiles(mirror & VBS_MIRROR_U ? (g->n_u + 1) / 2 : g->n_u, vts.tu) *
                               n_tiles(mirror & VBS_MIRROR_V ? (g->n_v + 1) / 2 : g->n_v, tile_v);
-        // few work items are split by transmits, to about two items per
-        // resident CTA (the split sets the order of the sums: a caller that
-        // cuts one acquisition into several calls passes the whole one's)
-        auto split = [&](int fb) {
-            if (!a->compound) return g->n_tx;
-            if (named) return 1;
-            if (split_req > 0) return split_req;
-            const int64_t items = tiles * n_tiles(a->n_frame * n_sym, fb);
-            return (int)std::min<int64_t>(g->n_tx, n_tiles(2 * 148 * vbs_min_ctas(fb), items));
-        };
+        // few work items are split into ranges of transmits, and up to 16 in all
+        // of elements, to about two items per resident CTA.  The ranges set the
+        // order of the sums: they do not depend on the frame block, and a
+        // caller that cuts one acquisition into several calls passes the whole
+        // one's plan.
+        int split = a->compound ? 1 : g->n_tx, split_rx = 1;
+        if (a->compound && !named) {
+            if (like && like->vb == 1) {
+                split = like->n_split;
+                split_rx = like->split_rx;
+            } else {
+                const int fb = std::min(8, pow2_ceil(a->n_frame * n_sym));
+                const int64_t want = n_tiles(2 * 148 * vbs_min_ctas(fb), tiles * n_tiles(a->n_frame * n_sym, fb));
+                split = (int)std::min<int64_t>(g->n_tx, want);
+                split_rx = (int)std::max<int64_t>(1, std::min<int64_t>({g->n_ele / 16, want / split, 16 / split}));
+                split *= split_rx;
+            }
+        }
         auto fits = [&](int vb, int d, int fb) {   // the largest window of the acquisition in its staging buffer
             const int need = (int)std::min<int64_t>(rows + std::max(d, 1), a->n_sample + d);
             if (vb == 1)
@@ -332,7 +340,7 @@ int plan_beamform(rcabf_geometry *g, const rcabf_beamform_args *a, Plan &p, cons
                 if (!force && fb_req == 0 && c > lim) continue;
                 // register accumulators: blocks of 8 at most (16 spill), but by name,
                 // and where every frame block has to keep one order of sums
-                if (vb == 1 && c == 16 && !want_vb && !(fb_req == 16 && (split(8) > 1 || d == 0 || n_sym > 1))) continue;
+                if (vb == 1 && c == 16 && !want_vb && !(fb_req == 16 && (split > 1 || d == 0 || n_sym > 1))) continue;
                 if (fits(vb, d, c)) return c;
             }
             return 0;
@@ -354,7 +362,8 @@ int plan_beamform(rcabf_geometry *g, const rcabf_beamform_args *a, Plan &p, cons
             p.ts = vts;
             p.wmax = (int)std::min<int64_t>(rows + std::max(d, 1), a->n_sample + d);
             if (vb == 1) {
-                p.n_split = split(fb);
+                p.n_split = split;
+                p.split_rx = split_rx;
                 p.mirror = mirror;
                 p.n_sym = n_sym;
             }
@@ -473,7 +482,7 @@ int stage_job(rcabf_geometry *g, const rcabf_beamform_args *a, const Plan &p, Fu
     J.nu_t = (int)p.nu_t; J.nv_t = (int)p.nv_t;
     J.n_sym = p.n_sym; J.mirror = p.mirror; J.n_vf = (int)(a->n_frame * p.n_sym);
     J.compact = p.compact;
-    J.n_split = p.n_split;
+    J.n_split = p.n_split; J.split_rx = p.split_rx;
     J.partial = reinterpret_cast<float2 *>(ws + p.off_part);
     return RCABF_OK;
 }
@@ -860,7 +869,7 @@ size_t align256(size_t x) { return (x + 255) / 256 * 256; }
 struct HostLayout {
     int64_t chunk = 0;
     size_t in_bytes = 0, out_bytes = 0, plan_bytes = 0, total = 0;
-    int n_split = 0;           // the whole call's transmit ranges (streaming kernel): every chunk sums as it does
+    Plan whole;                // the whole call's plan: every chunk sums in its order
     bool have_tuned = false;   // the autotuner's choice for the whole call, used by every chunk
     TuneChoice tuned;
 };
@@ -868,8 +877,8 @@ struct HostLayout {
 // Plan of one chunk: the whole call's tuned choice where one exists and fits.
 int chunk_plan(rcabf_geometry *g, const rcabf_beamform_args *c, const HostLayout &h, Plan &p)
 {
-    if (h.have_tuned && plan_beamform(g, c, p, &h.tuned, h.n_split) == RCABF_OK) return RCABF_OK;
-    return plan_beamform(g, c, p, nullptr, h.n_split);
+    if (h.have_tuned && plan_beamform(g, c, p, &h.tuned, &h.whole) == RCABF_OK) return RCABF_OK;
+    return plan_beamform(g, c, p, nullptr, &h.whole);
 }
 
 int host_layout(rcabf_geometry *g, const rcabf_beamform_args *a, int32_t frames_per_chunk, HostLayout &h)
@@ -888,7 +897,7 @@ int host_layout(rcabf_geometry *g, const rcabf_beamform_args *a, int32_t frames_
         chunk = fb * ((n_fb + 3) / 4);
     }
     h.chunk = std::min<int64_t>(chunk, a->n_frame);
-    if (p.vb == 1) h.n_split = p.n_split;
+    h.whole = p;
     {
         std::lock_guard<std::mutex> lk(g->mu);
         auto it = g->tuned.find({a->n_frame, (int64_t)a->storage});

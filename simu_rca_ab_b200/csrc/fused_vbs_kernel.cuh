@@ -76,23 +76,10 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_
                  : "memory");
 }
 
-__device__ __forceinline__ float2 ld_shared_f2(uint32_t a)
-{
-    float2 v;
-    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a));
-    return v;
-}
-__device__ __forceinline__ float4 ld_shared_f4(uint32_t a)
-{
-    float4 v;
-    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a));
-    return v;
-}
-
-// Work item -> frame block, transmit range and tile.  Tiles in depth-slowest
+// Work item -> frame block, ranges of transmits and elements, and tile.  Tiles in depth-slowest
 // order, deepest first.
 struct VsItem {
-    int job, fb, split, tu, tv, tz, tx0, n_tx;
+    int job, fb, split, tu, tv, tz, tx0, n_tx, rx0, n_rx;
 };
 __device__ __forceinline__ VsItem vs_item(const FusedParams &prm, int item)
 {
@@ -109,9 +96,29 @@ __device__ __forceinline__ VsItem vs_item(const FusedParams &prm, int item)
     r /= (uint32_t)J.n_split;
     w.fb = (int)(r % (uint32_t)J.n_fb);
     w.tz = J.tiles_z - 1 - (int)(r / (uint32_t)J.n_fb);
-    w.tx0 = (int)((int64_t)w.split * J.g.n_tx / J.n_split);
-    w.n_tx = (int)((int64_t)(w.split + 1) * J.g.n_tx / J.n_split) - w.tx0;
+    const int nst = J.n_split / J.split_rx, t = w.split / J.split_rx, e = w.split - t * J.split_rx;
+    w.tx0 = (int)((int64_t)t * J.g.n_tx / nst);
+    w.n_tx = (int)((int64_t)(t + 1) * J.g.n_tx / nst) - w.tx0;
+    w.rx0 = (int)((int64_t)e * J.g.n_ele / J.split_rx);
+    w.n_rx = (int)((int64_t)(e + 1) * J.g.n_ele / J.split_rx) - w.rx0;
     return w;
+}
+
+// A thread's first voxel (depth, receive axis, steering axis), and how many of
+// its four lie on the grid's part that is computed.
+struct __align__(16) VsVoxel {
+    int iz, iu, iv, n;
+};
+__device__ __forceinline__ VsVoxel vs_voxel(const FusedJob &J, const VsItem &w, int tid)
+{
+    VsVoxel x;
+    const unsigned q = (unsigned)tid / (unsigned)J.tu;
+    x.iu = w.tu * J.tu + tid - (int)q * J.tu;
+    x.iv = (w.tv * J.tv + (int)(q % (unsigned)J.tv)) * VB_BLOCK;
+    x.iz = w.tz * J.tz + (int)(q / (unsigned)J.tv);
+    const int rem = J.nv_t - x.iv;
+    x.n = !(x.iz < J.g.n_z && x.iu < J.nu_t) || rem <= 0 ? 0 : rem >= VB_BLOCK ? VB_BLOCK : rem;
+    return x;
 }
 
 // Scan state of a CTA, uniform over the scanning warp: the item scanned, the
@@ -143,18 +150,22 @@ __global__ void __launch_bounds__(VS_THREADS, vbs_min_ctas(FB)) fused_vbs_kernel
     __shared__ VsRec recs[VS_STAGES][VS_MAXREC];
     __shared__ VsChunkInfo info[VS_STAGES];
     __shared__ VsScan scan_s;
+    __shared__ VsItem item_s[VS_WARPS];          // per warp: the item it works on
+    __shared__ VsVoxel vox_s[FB < 8 ? VS_THREADS : 1];   // per thread: its voxels
+    __shared__ float4 tx_s[3][VS_THREADS];       // per thread: its voxels' index part and phasor of the transmit
+    __shared__ float4 e_s[2][VS_THREADS];        // per thread: receive table entries of this and the next record
     __shared__ float4 scan_rng[32];              // per lane: receive, transmit table ranges of the next batch
     __shared__ int scan_lo[32], scan_cnt[32];    // per lane: window of its step of the current batch
     __shared__ volatile int abort_s;
-    __shared__ __align__(16) float zeros[D == 0 ? TAPS * STRIDE / 4 : 4];   // TAPS rows of zeros
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t slot_bytes = (uint32_t)vbs_slot_bytes(FB, prm.wmax);
     const int krec = prm.krec;
+    const uint32_t zero_rows = VS_STAGES * (unsigned)krec * slot_bytes;   // offset of TAPS rows of zeros behind the chunks
     {
         unsigned dyn;
         asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn));
-        if (krec < 1 || krec > VS_MAXREC || dyn < VS_STAGES * (unsigned)krec * slot_bytes) {
+        if (krec < 1 || krec > VS_MAXREC || dyn < zero_rows + TAPS * STRIDE) {
             if (tid == 0) atomicAdd(prm.err_count, 1ull);
             return;
         }
@@ -168,21 +179,20 @@ __global__ void __launch_bounds__(VS_THREADS, vbs_min_ctas(FB)) fused_vbs_kernel
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if constexpr (D == 0)
-        for (int i = tid; i < TAPS * STRIDE / 4; i += VS_THREADS) zeros[i] = 0.f;
+        for (int i = tid; i < TAPS * STRIDE / 4; i += VS_THREADS) reinterpret_cast<float *>(smem + zero_rows)[i] = 0.f;
     __syncthreads();
     volatile int *abort = &abort_s;
     const uint32_t sbase = smem_u32(smem);
-    const uint32_t zero_rows = smem_u32(zeros);
 
     // ---------------- the scan (warp 0) ----------------
     // Its state lives in shared memory between chunks: in registers it would
     // cost every warp of the CTA the same registers.
     // per lane: step position p of the item -> (tx, rx)
-    auto step_of = [&](const VsScan &k, int p, int n_ele, int &tx, int &rx) {
+    auto step_of = [&](const VsScan &k, int p, int &tx, int &rx) {
         int e = p + k.rot;
         if (e >= k.steps) e -= k.steps;
-        const int t = e / n_ele;
-        rx = e - t * n_ele;
+        const int t = e / k.it.n_rx;
+        rx = k.it.rx0 + e - t * k.it.n_rx;
         tx = k.it.tx0 + t;
     };
     // starts the copy of the table ranges of batch `base`
@@ -191,7 +201,7 @@ __global__ void __launch_bounds__(VS_THREADS, vbs_min_ctas(FB)) fused_vbs_kernel
         if (p < k.steps) {
             const FusedJob &J = prm.jobs[k.it.job];
             int tx, rx;
-            step_of(k, p, J.g.n_ele, tx, rx);
+            step_of(k, p, tx, rx);
             cp_async<8>(&scan_rng[lane].x, &J.rx_range[((int64_t)rx * J.tiles_u + k.it.tu) * J.tiles_z + k.it.tz]);
             cp_async<8>(&scan_rng[lane].z, &J.tx_range[((int64_t)tx * J.tiles_v + k.it.tv) * J.tiles_z + k.it.tz]);
         }
@@ -208,14 +218,14 @@ __global__ void __launch_bounds__(VS_THREADS, vbs_min_ctas(FB)) fused_vbs_kernel
         k.next = __shfl_sync(0xffffffffu, k.next, 0);
         k.it = vs_item(prm, k.item);
         const FusedJob &J = prm.jobs[k.it.job];
-        k.steps = k.it.n_tx * J.g.n_ele;
+        k.steps = k.it.n_tx * k.it.n_rx;
         // transmit order rotated per tile: a hash of the tile picks the
         // quarter of the transmits the item starts from, so that CTAs of an
         // SM do not run their steps in lock step; whole transmits, so a
         // per-transmit item (n_tx = 1) is complete
         const uint32_t tile = (uint32_t)(k.it.tz + J.tiles_z * (k.it.tu + J.tiles_u * k.it.tv));
         const int t0 = k.it.n_tx >= 4 ? (int)(((tile * 0x9E3779B1u) >> 30) * (uint32_t)k.it.n_tx / 4u) : 0;
-        k.rot = t0 * J.g.n_ele;
+        k.rot = t0 * k.it.n_rx;
         fetch_ranges(k);
     };
     // fills stage st with the next chunk
@@ -240,7 +250,7 @@ __global__ void __launch_bounds__(VS_THREADS, vbs_min_ctas(FB)) fused_vbs_kernel
                     bool act = false;
                     lo = cnt = 0;
                     if (k.base + lane < k.steps) {
-                        step_of(k, k.base + lane, n_ele, tx, rx);
+                        step_of(k, k.base + lane, tx, rx);
                         const float4 q = scan_rng[lane];
                         if (q.x <= q.y && q.z <= q.w) {
                             const float ab = ab_value(J.g, tx, rx), fmax_n = (float)J.n_sample;
@@ -269,7 +279,7 @@ __global__ void __launch_bounds__(VS_THREADS, vbs_min_ctas(FB)) fused_vbs_kernel
                 const bool mine = ((k.mask >> lane) & 1u) && rank < krec - n;
                 if (mine) {
                     const int slot = n + rank;
-                    step_of(k, k.base - 32 + lane, n_ele, tx, rx);
+                    step_of(k, k.base - 32 + lane, tx, rx);
                     int m = 0, slab = tx * n_ele + rx;
                     if (J.compact) {
                         const bool mu = (J.mirror & VBS_MIRROR_U) && rx > n_ele - 1 - rx;
@@ -312,20 +322,27 @@ __global__ void __launch_bounds__(VS_THREADS, vbs_min_ctas(FB)) fused_vbs_kernel
     }
 
     // ---------------- state of the item being computed ----------------
-    int cur = -1, cur_tx = -1, job = 0, n_pair = 0;
+    // (what the frame sums do not need is kept in shared memory, or with 8
+    // frames worked out again: registers decide how many CTAs share an SM)
+    int cur = -1, cur_tx = -1, n_pair = 0;
     int cur_m = 0;                            // the accumulators' slot s holds copy s ^ cur_m
-    int iz = 0, iu = 0, iv0 = 0, nvv = 0;     // the thread's first voxel, and how many of its four are on the grid
     const float4 *rxp = nullptr;              // receive table entry of element 0, and the elements' stride
     int rx_stride = 0;
     float lim = 0.f;                          // sample indices at or past it leave the record
-    bool has_ab = false;
-    float4 enext = make_float4(0.f, 0.f, 0.f, 0.f);   // receive table entry of the next record
-    bool have_e = false;
+    int ab_job = -1;                          // the item's job, where it has an aberration law
+    bool have_e = false;                      // the next record's table entry is on its way
+    int e_buf = 0;
     unsigned cone_bits = 0;
-    float2 txi[2], txr[2], txq[2];    // voxel pairs: index part and phasor of the current transmit
     // FB = 1: (re, im) of voxel v in are[v][0]; else frames 2p, 2p + 1 of
     // voxel v: re in are[v][p], im in aim[v][p]
     float2 are[VB][NP], aim[VB][FB == 1 ? 1 : NP];
+
+    // starts the copy of the receive table entry of element rx
+    auto fetch_e = [&](int rx) {
+        cp_async<16>(&e_s[e_buf][tid], rxp + (int64_t)rx * rx_stride);
+        cp_async_commit();
+        e_buf ^= 1;
+    };
 
     for (uint32_t c = 0;; ++c) {
         const int st = (int)(c % VS_STAGES);
@@ -337,18 +354,18 @@ __global__ void __launch_bounds__(VS_THREADS, vbs_min_ctas(FB)) fused_vbs_kernel
             cur_tx = -1;
             cur_m = 0;
             const VsItem ci = vs_item(prm, cur);
-            job = ci.job;
-            const FusedJob &J = prm.jobs[job];
-            const int lu = tid % J.tu, lvb = (tid / J.tu) % J.tv, lz = tid / (J.tu * J.tv);
-            iz = ci.tz * J.tz + lz;
-            iu = ci.tu * J.tu + lu;
-            iv0 = (ci.tv * J.tv + lvb) * VB;
-            const int rem = J.nv_t - iv0;
-            nvv = !(iz < J.g.n_z && iu < J.nu_t) || rem <= 0 ? 0 : rem >= VB ? VB : rem;
-            rxp = J.g.rx_tab + (nvv > 0 ? (int64_t)iu * J.g.n_z + iz : 0);   // off the grid: any entry, never used
+            const FusedJob &J = prm.jobs[ci.job];
+            const VsVoxel x = vs_voxel(J, ci, tid);
+            if constexpr (FB < 8) {   // many short items: decoded once
+                vox_s[tid] = x;
+                __syncwarp();
+                if (lane == 0) item_s[warp] = ci;
+                __syncwarp();
+            }
+            rxp = J.g.rx_tab + (x.n > 0 ? (int64_t)x.iu * J.g.n_z + x.iz : 0);   // off the grid: any entry, never used
             rx_stride = (int)(J.g.n_u * J.g.n_z);
             lim = (float)(J.n_sample - 1 - KT::HI);
-            has_ab = J.g.ab != nullptr;
+            ab_job = J.g.ab != nullptr ? ci.job : -1;
             n_pair = FB == 1 ? 1 : (min(FB, J.n_vf - ci.fb * FB) + 1) / 2;
 #pragma unroll
             for (int v = 0; v < VB; ++v)
@@ -358,35 +375,36 @@ __global__ void __launch_bounds__(VS_THREADS, vbs_min_ctas(FB)) fused_vbs_kernel
                     if constexpr (FB > 1) aim[v][p] = make_float2(0.f, 0.f);
                 }
         }
-        const uint32_t slot0 = sbase + (uint32_t)(st * krec) * slot_bytes;
-        if (!have_e && ck.n > 0) enext = __ldg(rxp + (int64_t)recs[st][0].rx * rx_stride);
+        const uint32_t slot0 = (uint32_t)(st * krec) * slot_bytes;   // offset in smem
+        if (!have_e && ck.n > 0) fetch_e(recs[st][0].rx);
         for (int i = 0; i < ck.n; ++i) {
             VsRec h = recs[st][i];
             const int m = (int)((unsigned)h.count >> VS_M_SHIFT);
             h.count &= (1 << VS_M_SHIFT) - 1;
-            const float4 e = enext;
-            if (i + 1 < ck.n) enext = __ldg(rxp + (int64_t)recs[st][i + 1].rx * rx_stride);
+            cp_async_wait<0>();
+            const float4 e = e_s[e_buf ^ 1][tid];
+            if (i + 1 < ck.n) fetch_e(recs[st][i + 1].rx);
             if (h.tx != cur_tx) {
                 cur_tx = h.tx;
                 cone_bits = 0;
-                if (nvv > 0) {
-                    const DevGeom &g = prm.jobs[job].g;
-                    const float4 *txrow = g.tx_tab + (int64_t)h.tx * (g.n_v * g.n_z) + iz;
+                const VsItem ci = FB < 8 ? item_s[warp] : vs_item(prm, cur);
+                const DevGeom &g = prm.jobs[ci.job].g;
+                const VsVoxel x = FB < 8 ? vox_s[tid] : vs_voxel(prm.jobs[ci.job], ci, tid);
+                if (x.n > 0) {
+                    const float4 *txrow = g.tx_tab + (int64_t)h.tx * (g.n_v * g.n_z) + x.iz;
                     const bool cu = g.cone_u == nullptr ||
-                                    g.cone_u[(int64_t)h.tx * rx_stride + (int64_t)iu * g.n_z + iz] != 0;
+                                    g.cone_u[(int64_t)h.tx * rx_stride + (int64_t)x.iu * g.n_z + x.iz] != 0;
                     float4 t[VB];
+                    // (kept in shared memory, not in 12 registers across the frame sums)
 #pragma unroll
                     for (int v = 0; v < VB; ++v) {
                         // voxels past the grid: the last one's entry, never in cone_bits
-                        t[v] = __ldg(&txrow[(int64_t)(iv0 + min(v, nvv - 1)) * g.n_z]);
-                        if (cu && v < nvv && t[v].w != 0.0f) cone_bits |= 1u << v;
+                        t[v] = __ldg(&txrow[(int64_t)(x.iv + min(v, x.n - 1)) * g.n_z]);
+                        if (cu && v < x.n && t[v].w != 0.0f) cone_bits |= 1u << v;
                     }
-#pragma unroll
-                    for (int j = 0; j < 2; ++j) {
-                        txi[j] = make_float2(t[2 * j].x, t[2 * j + 1].x);
-                        txr[j] = make_float2(t[2 * j].y, t[2 * j + 1].y);
-                        txq[j] = make_float2(t[2 * j].z, t[2 * j + 1].z);
-                    }
+                    tx_s[0][tid] = make_float4(t[0].x, t[1].x, t[2].x, t[3].x);
+                    tx_s[1][tid] = make_float4(t[0].y, t[1].y, t[2].y, t[3].y);
+                    tx_s[2][tid] = make_float4(t[0].z, t[1].z, t[2].z, t[3].z);
                 }
             }
             if constexpr (FB >= 2) {
@@ -424,11 +442,12 @@ __global__ void __launch_bounds__(VS_THREADS, vbs_min_ctas(FB)) fused_vbs_kernel
             float rd[VB];
             bool ok[VB];
             float ab = 0.0f;
-            if (has_ab) ab = ab_value(prm.jobs[job].g, h.tx, h.rx);
+            if (ab_job >= 0) ab = ab_value(prm.jobs[ab_job].g, h.tx, h.rx);
             float base = 3.0e38f;
+            const float4 ti = tx_s[0][tid];
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
-                float2 idx = __fadd2_rn(txi[j], make_float2(e.x, e.x));
+                float2 idx = __fadd2_rn(j ? make_float2(ti.z, ti.w) : make_float2(ti.x, ti.y), make_float2(e.x, e.x));
                 idx = __fadd2_rn(idx, make_float2(ab, ab));
                 rd[2 * j] = __fadd_rd(idx.x, VS_MAGIC);
                 rd[2 * j + 1] = __fadd_rd(idx.y, VS_MAGIC);
@@ -443,15 +462,18 @@ __global__ void __launch_bounds__(VS_THREADS, vbs_min_ctas(FB)) fused_vbs_kernel
 
             // ---- phasor P = apod exp(j phase_tx) exp(j phase_rx) exp(j phase_ab) ----
             float2 Px[2], Py[2];
+            const float4 tr = tx_s[1][tid], tq = tx_s[2][tid];
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
+                const float2 txr = j ? make_float2(tr.z, tr.w) : make_float2(tr.x, tr.y);
+                const float2 txq = j ? make_float2(tq.z, tq.w) : make_float2(tq.x, tq.y);
                 const float2 ey = make_float2(e.y, e.y), ez = make_float2(e.z, e.z);
-                const float2 nq = make_float2(-txq[j].x, -txq[j].y);
-                Px[j] = __ffma2_rn(txr[j], ey, __fmul2_rn(nq, ez));
-                Py[j] = __ffma2_rn(txr[j], ez, __fmul2_rn(txq[j], ey));
+                const float2 nq = make_float2(-txq.x, -txq.y);
+                Px[j] = __ffma2_rn(txr, ey, __fmul2_rn(nq, ez));
+                Py[j] = __ffma2_rn(txr, ez, __fmul2_rn(txq, ey));
             }
-            if (has_ab) {
-                const float2 abp = ab_phasor(prm.jobs[job].g, h.tx, h.rx);
+            if (ab_job >= 0) {
+                const float2 abp = ab_phasor(prm.jobs[ab_job].g, h.tx, h.rx);
 #pragma unroll
                 for (int j = 0; j < 2; ++j) {
                     const float2 qx = Px[j], qy = Py[j];
@@ -486,7 +508,7 @@ __global__ void __launch_bounds__(VS_THREADS, vbs_min_ctas(FB)) fused_vbs_kernel
                         tv[v] = make_float2(0.f, 0.f);
 #pragma unroll
                         for (int k = 0; k < TAPS; ++k) {
-                            const float2 x = ld_shared_f2(a[v] + k * STRIDE);
+                            const float2 x = *reinterpret_cast<const float2 *>(smem + a[v] + k * STRIDE);
                             tv[v].x = fmaf(wt(v, k), x.x, tv[v].x);
                             tv[v].y = fmaf(wt(v, k), x.y, tv[v].y);
                         }
@@ -509,7 +531,7 @@ __global__ void __launch_bounds__(VS_THREADS, vbs_min_ctas(FB)) fused_vbs_kernel
                                 float2 tre = make_float2(0.f, 0.f), tim = tre;
 #pragma unroll
                                 for (int k = 0; k < TAPS; ++k) {
-                                    const float4 x = ld_shared_f4(a[v] + k * STRIDE + p * 16);
+                                    const float4 x = *reinterpret_cast<const float4 *>(smem + a[v] + k * STRIDE + p * 16);
                                     const float2 w2 = make_float2(wt(v, k), wt(v, k));
                                     tre = __ffma2_rn(w2, make_float2(x.x, x.y), tre);
                                     tim = __ffma2_rn(w2, make_float2(x.z, x.w), tim);
@@ -584,7 +606,7 @@ __global__ void __launch_bounds__(VS_THREADS, vbs_min_ctas(FB)) fused_vbs_kernel
                         for (int v = 0; v < VB; ++v) { tre[v] = make_float2(0.f, 0.f); tim[v] = tre[v]; }
 #pragma unroll
                         for (int k = 0; k < R; ++k) {
-                            const float4 x = ld_shared_f4(a0 + k * STRIDE + p * 16);
+                            const float4 x = *reinterpret_cast<const float4 *>(smem + a0 + k * STRIDE + p * 16);
 #pragma unroll
                             for (int v = 0; v < VB; ++v) {
                                 const float2 w2 = make_float2(ws[v][k], ws[v][k]);
@@ -607,11 +629,12 @@ __global__ void __launch_bounds__(VS_THREADS, vbs_min_ctas(FB)) fused_vbs_kernel
         }
         have_e = false;
         if (ck.last) {
-            const FusedJob &J = prm.jobs[job];
+            const VsItem ci = FB < 8 ? item_s[warp] : vs_item(prm, cur);
+            const FusedJob &J = prm.jobs[ci.job];
             const DevGeom &g = J.g;
+            const VsVoxel x = FB < 8 ? vox_s[tid] : vs_voxel(J, ci, tid);
             // the item's outputs: the volume (or the transmit's own, when not
             // compounded), or this transmit range's part of it
-            const VsItem ci = vs_item(prm, cur);
             cur = -1;
             float2 *out = J.out;
             int64_t stride = g.n_pix;
@@ -628,16 +651,16 @@ __global__ void __launch_bounds__(VS_THREADS, vbs_min_ctas(FB)) fused_vbs_kernel
                 if (vf >= J.n_vf) continue;
                 const int fr = J.n_sym == 1 ? vf : vf / J.n_sym;
                 const int m = vbs_mirrored(J.mirror, (vf - fr * J.n_sym) ^ cur_m);
-                const int ou = m & VBS_MIRROR_U ? (int)g.n_u - 1 - iu : iu;
-                if ((m & VBS_MIRROR_U) && ou == iu) continue;   // the middle column: the unmirrored copy writes it
+                const int ou = m & VBS_MIRROR_U ? (int)g.n_u - 1 - x.iu : x.iu;
+                if ((m & VBS_MIRROR_U) && ou == x.iu) continue;   // the middle column: the unmirrored copy writes it
                 // not compounded: copy m of transmit tx0 is the mirrored transmit's
                 const int64_t off = J.compound ? 0
                                                : (int64_t)(m & VBS_MIRROR_V ? g.n_tx - 1 - ci.tx0 : ci.tx0) * g.n_pix;
-                float2 *o0 = out + (int64_t)fr * stride + off + iz * g.s_z + ou * g.s_u;
+                float2 *o0 = out + (int64_t)fr * stride + off + x.iz * g.s_z + ou * g.s_u;
 #pragma unroll
                 for (int v = 0; v < VB; ++v) {
-                    const int iv = iv0 + v, ov = m & VBS_MIRROR_V ? (int)g.n_v - 1 - iv : iv;
-                    if (v < nvv && !((m & VBS_MIRROR_V) && ov == iv)) {
+                    const int iv = x.iv + v, ov = m & VBS_MIRROR_V ? (int)g.n_v - 1 - iv : iv;
+                    if (v < x.n && !((m & VBS_MIRROR_V) && ov == iv)) {
                         float2 a;
                         if constexpr (FB == 1) a = are[v][0];
                         else a = f & 1 ? make_float2(are[v][f >> 1].y, aim[v][f >> 1].y)
@@ -655,7 +678,7 @@ __global__ void __launch_bounds__(VS_THREADS, vbs_min_ctas(FB)) fused_vbs_kernel
             const int ns = (int)(nc % VS_STAGES);
             if (__all_sync(0xffffffffu, mbar_test_wait(&full[ns], (nc / VS_STAGES) & 1u))) {
                 have_e = info[ns].n > 0;
-                if (have_e) enext = __ldg(rxp + (int64_t)recs[ns][0].rx * rx_stride);
+                if (have_e) fetch_e(recs[ns][0].rx);
             }
         }
         __syncwarp();

@@ -18,7 +18,7 @@ struct Plan {
     // voxel-blocked kernels: 1 register accumulators, streamed windows
     // (fused_vbs_kernel.cuh), 2 TMEM accumulators (fused_vb_kernel.cuh)
     int vb = 0;
-    int n_split = 1;      // vb = 1: transmit ranges, one work item each
+    int n_split = 1, split_rx = 1;   // vb = 1: ranges of steps, one work item each; of them along the elements
     int mirror = 0, n_sym = 1;          // vb = 1: mirrored axes, copies of a frame (VBS_MIRROR_*)
     int64_t nu_t = 0, nv_t = 0;         // vb = 1: tile-space extents
     int compact = 0;                    // vb = 1: one slab for the steps that mirror each other
@@ -40,9 +40,10 @@ struct Plan {
 // force: a launch choice to plan instead of the planner's own (autotuner);
 // without one, a choice rcabf_autotune stored for these frames and storage
 // is used.  RCABF_ERR_UNSUPPORTED when a forced choice does not fit.
-// split_req: transmit ranges of the streaming kernel (0: the planner's number).
+// like: a plan whose ranges of steps to take (streaming kernel; NULL: the
+// planner's own).
 int plan_beamform(rcabf_geometry *g, const rcabf_beamform_args *a, Plan &p, const TuneChoice *force = nullptr,
-                  int split_req = 0);
+                  const Plan *like = nullptr);
 
 // Smaller-workspace replacement of a streaming-kernel plan (api.cpp).
 void plan_compact(rcabf_geometry *g, rcabf_beamform_args &a, Plan &p);
@@ -76,10 +77,14 @@ inline size_t vb_smem_bytes(int store, int wmax, int row_words, int zero_rows = 
 // (0: not even one).
 inline int vbs_chunk_records(int fb, int wmax)
 {
-    const int n = (int)((224 * 1024 / vbs_min_ctas(fb) - 2048) / (3 * (size_t)vbs_slot_bytes(fb, wmax)));
+    const int n = (int)((224 * 1024 / vbs_min_ctas(fb) - 16 * 1024) / (3 * (size_t)vbs_slot_bytes(fb, wmax)));
     return n > VBS_MAX_RECORDS ? VBS_MAX_RECORDS : n;
 }
-inline size_t vbs_smem_bytes(int fb, int wmax) { return 3 * (size_t)vbs_chunk_records(fb, wmax) * vbs_slot_bytes(fb, wmax); }
+// (three chunks, and 8 rows of zeros behind them)
+inline size_t vbs_smem_bytes(int fb, int wmax)
+{
+    return 3 * (size_t)vbs_chunk_records(fb, wmax) * vbs_slot_bytes(fb, wmax) + 8 * vbs_row_bytes(fb);
+}
 inline int vb_stage_rows_cap(int store, int fb)
 {
     if (store == ST_F32) return 1 << 30;

@@ -90,7 +90,9 @@ struct FusedJob {
     // copies of a frame a block holds (1, 2 or 4: see VBS_MIRROR_*), frames x copies
     int32_t nu_t, nv_t;
     int32_t n_sym, mirror, n_vf, compact;
-    int32_t n_split;           // streaming kernel: transmit ranges, an item each (n_tx when not compounded)
+    // streaming kernel: ranges of steps, an item each: n_split / split_rx ranges
+    // of transmits (n_tx when not compounded) x split_rx ranges of elements
+    int32_t n_split, split_rx;
     float2 *partial;           // its sums per range [n_split][frame][pix] when compounded and n_split > 1
 };
 
@@ -138,7 +140,7 @@ constexpr int VBS_MAX_SAMPLES = 1 << 21;
 // weights and the per-voxel transmit state.  With 8 frames a third CTA (168
 // registers, spills) measured 6 % slower than two; with 4 a fourth 4 % slower
 // than three.
-constexpr RCABF_HD int vbs_min_ctas(int fb) { return fb >= 8 ? 2 : fb >= 4 ? 3 : 4; }
+constexpr RCABF_HD int vbs_min_ctas(int fb) { return fb >= 16 ? 2 : fb >= 4 ? 3 : 4; }
 constexpr int VBS_PAD_ROWS = 2;      // zero rows past the record (shift rows)
 constexpr RCABF_HD int vbs_row_bytes(int fb) { return fb <= 2 ? 8 * fb : 8 * fb + 16; }
 constexpr RCABF_HD int vbs_slot_bytes(int fb, int wmax) { return (wmax * vbs_row_bytes(fb) + 15) / 16 * 16; }
