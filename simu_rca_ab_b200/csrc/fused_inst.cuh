@@ -52,8 +52,14 @@ static cudaError_t plain_do(const PlainParams &p, cudaStream_t st)
         int dev = 0, n_sm = 148;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
-        const int64_t blocks = std::min<int64_t>((n * p.g.n_ele + 255) / 256, (int64_t)n_sm * 16);
-        pc_das_kernel<MODE, KIND, IQ><<<(unsigned)blocks, 256, 0, st>>>(p);
+        // frames a thread takes: as many as leave about 4 threads per resident
+        // thread (2048 on an SM), at most 16, beyond which its setup is a small part
+        PlainParams q = p;
+        const int64_t setups = n * p.g.n_ele * p.g.n_tx, threads = (int64_t)n_sm * 8192;
+        q.frames = (int)std::min<int64_t>(16, std::max<int64_t>(1, setups * p.n_frame / threads));
+        const int64_t total = setups * ((p.n_frame + q.frames - 1) / q.frames);
+        const int64_t blocks = std::min<int64_t>((total + 255) / 256, (int64_t)n_sm * 256);
+        pc_das_kernel<MODE, KIND, IQ><<<(unsigned)blocks, 256, 0, st>>>(q);
     } else if (p.per_channel)
         plain_das_kernel<MODE, KIND, IQ, true><<<(unsigned)((n + 255) / 256), 256, 0, st>>>(p);
     else

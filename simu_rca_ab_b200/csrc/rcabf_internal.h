@@ -165,6 +165,7 @@ struct PlainParams {
     int32_t n_sample;
     int64_t frame;
     int64_t n_frame;
+    int32_t frames;             // per-channel, every frame in one launch: frames a thread takes
     int32_t compound, accumulate;
     int32_t per_channel;        // out is [element][frame][tx][pix]: one value per receive element
     float2 *out;
