@@ -157,6 +157,24 @@ int plan_beamform(rcabf_geometry *g, const rcabf_beamform_args *a, Plan &p, cons
     }
     p.store = a->storage;
     const int es = store_bytes(p.store);
+    // Few frames in the reference's arithmetic, the planner's own choice: the
+    // per-(voxel, transmit) kernel, whose transmit sums take n_tx volumes.
+    // (One frame, 6 taps: 7.5 -> 3.5 ms; the fused kernel shares a step's sine
+    // and divide work between the frames of its block, up to 16, and the gather
+    // kernel only between 4.)
+    bool has_tuned = false;
+    if (g->mode == MODE_REF) {
+        std::lock_guard<std::mutex> lk(g->mu);
+        has_tuned = g->tuned.count({a->n_frame, (int64_t)a->storage}) > 0;
+    }
+    if (g->mode == MODE_REF && !force && !has_tuned && fb_req == 0 && a->n_frame <= REF_MAX_FRAMES &&
+        (a->kernel == RCABF_KERNEL_AUTO || a->kernel == RCABF_KERNEL_FUSED) && g->n_tx <= 65535) {
+        p.ref = 1;
+        p.total = a->compound ? (size_t)g->n_tx * a->n_frame * g->n_pix * sizeof(float2) : 0;
+        if (p.total <= REF_MAX_BYTES) return RCABF_OK;
+        p.ref = 0;
+        p.total = 0;
+    }
     TuneChoice tuned;
     if (!force) {   // a choice the autotuner measured for this geometry, frames and storage
         std::lock_guard<std::mutex> lk(g->mu);
@@ -412,7 +430,7 @@ void plan_compact(rcabf_geometry *g, rcabf_beamform_args &a, Plan &p)
     for (int32_t k : {RCABF_KERNEL_FUSED_TMEM, RCABF_KERNEL_FUSED_NOBLOCK}) {
         Plan q;
         c.kernel = k;
-        if (plan_beamform(g, &c, q) == RCABF_OK && q.kernel == RCABF_KERNEL_FUSED && q.total < p.total) {
+        if (plan_beamform(g, &c, q) == RCABF_OK && q.kernel == RCABF_KERNEL_FUSED && (p.ref || q.total < p.total)) {
             p = q;
             a.kernel = k;
             return;
@@ -595,6 +613,27 @@ static int beamform_planned(rcabf_geometry *g, const rcabf_beamform_args *a, con
     if ((s = check_ptrs(a, p)) != RCABF_OK) return s;
     device_state(g->device);
     mark(a, 0, st);
+    if (p.ref) {
+        mark(a, 1, st);
+        mark(a, 2, st);
+        PlainParams pp{};
+        pp.g = g->dev(); pp.iq = a->iq; pp.iq_dtype = a->iq_dtype; pp.n_sample = (int)a->n_sample;
+        pp.n_frame = a->n_frame; pp.compound = a->compound ? 1 : 0; pp.accumulate = a->accumulate ? 1 : 0;
+        pp.out = reinterpret_cast<float2 *>(a->compound ? a->workspace : a->out);
+        cudaError_t e = launch_ref_das(g->kind, pp, st);
+        if (e != cudaSuccess) return cuda_fail(e, "reference-table kernel launch");
+        g_launches += 1;
+        if (a->compound) {   // transmits in order, as the reference adds them
+            e = launch_vbs_reduce(reinterpret_cast<float2 *>(a->out), static_cast<const float2 *>(a->workspace),
+                                  a->n_frame * g->n_pix, g->n_tx, a->accumulate ? 1 : 0, st);
+            if (e != cudaSuccess) return cuda_fail(e, "transmit sum launch");
+            g_launches += 1;
+        }
+        mark(a, 3, st);
+        if ((s = finish_mask(g, a, st)) != RCABF_OK) return s;
+        mark(a, 4, st);
+        return RCABF_OK;
+    }
     if (p.kernel == RCABF_KERNEL_PLAIN) {
         mark(a, 1, st);
         mark(a, 2, st);
@@ -681,7 +720,11 @@ int beamform_noalloc(rcabf_geometry *g, const rcabf_beamform_args *a, cudaStream
     // the streaming kernel's FP32 slabs are up to three times the channel
     // data in storage type: where they do not fit, the kernels that stage it
     rcabf_beamform_args b = *a;
-    if (p.vb == 1 && p.total > RCABF_NOALLOC_WORKSPACE_BYTES) plan_compact(g, b, p);
+    if (p.ref || (p.vb == 1 && p.total > RCABF_NOALLOC_WORKSPACE_BYTES)) plan_compact(g, b, p);
+    if (p.ref) {
+        snprintf(g_last_err, sizeof(g_last_err), "noalloc: no fused plan for these reference tables");
+        return RCABF_ERR_UNSUPPORTED;
+    }
     if (p.total > RCABF_NOALLOC_WORKSPACE_BYTES) {
         snprintf(g_last_err, sizeof(g_last_err),
                  "noalloc: the plan needs %zu workspace bytes; the static workspace holds %zu", p.total,
@@ -821,12 +864,13 @@ int rcabf_describe_plan(const rcabf_geometry *g, const rcabf_beamform_args *a, c
     int occ = 0;   // resident CTAs per SM of the fused kernel (0: plain kernel)
     if (p.tc) {
         occ = 1;
-    } else if (p.kernel == RCABF_KERNEL_FUSED) {
+    } else if (p.kernel == RCABF_KERNEL_FUSED && !p.ref) {
         s = resident_ctas(g, p, p.smem, device_state(g->device), occ);
         if (s != RCABF_OK) return s;
     }
     const char *kname = p.pc_all                         ? "per_channel_all_frames"
                         : p.kernel == RCABF_KERNEL_PLAIN ? "plain"
+                        : p.ref                         ? "reference_per_transmit"
                         : p.tc == 2                     ? "fused_tensor_core"
                         : p.tc == 1                     ? "fused_tensor_core_fp16w"
                         : p.vb == 2                     ? "fused_voxel_blocked_tmem"
@@ -1197,7 +1241,7 @@ int rcabf_autotune(const rcabf_geometry *gc, const rcabf_beamform_args *a, void 
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     if (s != RCABF_OK) return s;
-    {
+    if (!p0.ref || best_ms < default_ms) {   // the per-transmit kernel is no stored choice: it stays the planner's
         std::lock_guard<std::mutex> lk(g->mu);
         g->tuned[key] = best;
     }

@@ -125,13 +125,13 @@ __device__ __forceinline__ void ref_weights(float d, float (&w)[KindTraits<KIND>
 #pragma unroll
         for (int j = 0; j < 6; ++j) {
             const float x = __fadd_rn(d, (float)(2 - j));
-            w[j] = __fmul_rn(ref_sinc(x), ref_sinc(__fdiv_rn(x, 2.0f)));
+            w[j] = __fmul_rn(ref_sinc(x), ref_sinc(__fmul_rn(x, 0.5f)));   // x / 2: the same float
         }
     } else {  // RCA.cu:355-357
         const float dm1 = __fsub_rn(d, 1.0f), dp1 = __fadd_rn(d, 1.0f);
-        w[0] = __fdiv_rn(__fmul_rn(d, dm1), 2.0f);
+        w[0] = __fmul_rn(__fmul_rn(d, dm1), 0.5f);   // / 2: the same float
         w[1] = __fmul_rn(-dm1, dp1);
-        w[2] = __fdiv_rn(__fmul_rn(d, dp1), 2.0f);
+        w[2] = __fmul_rn(__fmul_rn(d, dp1), 0.5f);
     }
 }
 
@@ -213,7 +213,9 @@ __device__ __forceinline__ void setup_ref(const float4 t, const float4 e, float 
     const float delta = __fadd_rn(
         __fmul_rn(__fmul_rn(__fmul_rn(-2.0f, RCABF_PI_F), idx), rs.ratio),
         __fmul_rn(__fmul_rn(__fmul_rn(__fmul_rn(4.0f, RCABF_PI_F), rs.fd), t.z), rs.inv_c));
-    s.P = make_float2(cosf(delta), sinf(delta));
+    // (sincosf gives cosf's and sinf's bits for every finite argument below
+    // 1e30, compared over all floats: one argument reduction instead of two)
+    sincosf(delta, &s.P.y, &s.P.x);
     s.apod = e.y;
 }
 

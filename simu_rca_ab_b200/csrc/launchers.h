@@ -112,6 +112,10 @@ unsigned long long *current_error_counter();
 void count_launches(int64_t n);
 size_t tc_launch_smem(int fb);
 
+// Few frames on REF_COMPAT tables (ref_kernel.cuh): compounded, p.out holds
+// [transmit][frame][pix] sums for launch_vbs_reduce to add.
+cudaError_t launch_ref_das(int kind, const PlainParams &p, cudaStream_t st);
+
 // Plain kernel: one frame.
 cudaError_t launch_plain(int mode, int kind, const PlainParams &p, cudaStream_t st);
 

@@ -14,6 +14,7 @@ constexpr size_t SMEM_BUDGET = 110 * 1024;
 
 struct Plan {
     int kernel = 0;       // rcabf_kernel
+    int ref = 0;          // few frames on REF_COMPAT tables (ref_kernel.cuh)
     int pc_all = 0;       // per-channel output, every frame in one launch (pc_das_kernel)
     // voxel-blocked kernels: 1 register accumulators, streamed windows
     // (fused_vbs_kernel.cuh), 2 TMEM accumulators (fused_vb_kernel.cuh)

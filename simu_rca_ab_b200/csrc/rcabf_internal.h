@@ -103,6 +103,8 @@ struct FusedJob {
 constexpr int TC_TILE_U = 4, TC_TILE_V = 32, TC_MAX_ROWS = 32;
 
 constexpr int MAX_JOBS = 24;
+constexpr int REF_MAX_FRAMES = 4;             // the per-transmit REF_COMPAT kernel: most frames, and
+constexpr size_t REF_MAX_BYTES = 2ull << 30;  // most bytes of transmit sums
 constexpr int FUSED_THREADS = 256;
 constexpr int FUSED_STAGES = 3;
 constexpr int VB_BLOCK = 4;          // voxels per thread along v in the voxel-blocked kernel

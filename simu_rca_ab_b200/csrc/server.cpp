@@ -368,10 +368,10 @@ int rcabf_server_submit(rcabf_server *s, const rcabf_geometry *g, const rcabf_be
     r->a.stage_events = nullptr;
     int st = plan_beamform(gg, &r->a, r->plan);
     // a request whose FP32 slabs exceed the whole arena runs on storage-type slabs
-    if (st == RCABF_OK && r->plan.vb == 1 && Arena::round(r->plan.total) > s->arena.size())
+    if (st == RCABF_OK && (r->plan.vb == 1 || r->plan.ref) && Arena::round(r->plan.total) > s->arena.size())
         plan_compact(gg, r->a, r->plan);
     if (st == RCABF_OK && (!r->a.iq || !r->a.out)) st = RCABF_ERR_INVALID_ARGUMENT;
-    if (st == RCABF_OK && r->plan.kernel == RCABF_KERNEL_FUSED && r->a.frames_per_block == 0) {
+    if (st == RCABF_OK && r->plan.kernel == RCABF_KERNEL_FUSED && !r->plan.ref && r->a.frames_per_block == 0) {
         // pin the frame block the planner chose, so the request runs the same
         // kernel variant alone or fused with others; a request whose plan
         // would change under the pin is never fused
@@ -383,7 +383,7 @@ int rcabf_server_submit(rcabf_server *s, const rcabf_geometry *g, const rcabf_be
             r->a = pinned;
             r->batchable = true;
         }
-    } else if (st == RCABF_OK && r->plan.kernel == RCABF_KERNEL_FUSED) {
+    } else if (st == RCABF_OK && r->plan.kernel == RCABF_KERNEL_FUSED && !r->plan.ref) {
         r->batchable = true;
     }
     std::lock_guard<std::mutex> lk(s->mu);
