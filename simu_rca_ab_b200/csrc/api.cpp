@@ -286,8 +286,10 @@ int plan_beamform(rcabf_geometry *g, const rcabf_beamform_args *a, Plan &p, cons
     // Voxel-blocked kernels: exact tables and a steering axis to block along.
     //   vb = 1: register accumulators, windows streamed ahead by bulk copies.
     //     The four voxels of a thread share their sample rows where a block
-    //     spreads over at most 2 of them (d = 1, 2); single frames and wider
-    //     spreads have every voxel read its own (d = 0).
+    //     spreads over at most 2 of them (d = 1, 2), pairs of them where only
+    //     a pair does (d = 3, 4: half the shared-memory loads, which bound
+    //     it); single frames without mirrored copies and wider spreads have
+    //     every voxel read its own (d = 0).
     //   vb = 2: accumulators in tensor memory, for frame blocks of 16 that
     //     registers hold only with spills, at d = 1, 2.
     const int want_vb = force ? force->vb
@@ -339,15 +341,19 @@ int plan_beamform(rcabf_geometry *g, const rcabf_beamform_args *a, Plan &p, cons
                 split *= split_rx;
             }
         }
+        auto window = [&](int d) {   // staged rows: the largest window and the shift rows
+            const int ds = d >= 3 ? d - 2 : d;
+            return (int)std::min<int64_t>(rows + std::max(ds, 1), a->n_sample + ds);
+        };
         auto fits = [&](int vb, int d, int fb) {   // the largest window of the acquisition in its staging buffer
-            const int need = (int)std::min<int64_t>(rows + std::max(d, 1), a->n_sample + d);
+            const int need = window(d);
             if (vb == 1)
                 return a->n_sample <= VBS_MAX_SAMPLES && vbs_chunk_records(fb, need) >= 1;
             return need <= std::min<int>((int)(VB_SMEM_BUDGET / ((size_t)fused_stages(p.store) * fused_row_words(fb) * 4)),
                                          vb_stage_rows_cap(p.store, fb));
         };
         auto pick = [&](int vb, int d) {   // the frame block, 0: none
-            if (vb == 2 && d == 0) return 0;
+            if (vb == 2 && (d == 0 || d >= 3)) return 0;
             for (int c : {16, 8, 4, 2, 1}) {
                 if (d > 0 && c == 1) continue;
                 if (force ? c != force->fb : fb_req > 0 && c != fb_req) continue;
@@ -358,14 +364,20 @@ int plan_beamform(rcabf_geometry *g, const rcabf_beamform_args *a, Plan &p, cons
                 if (!force && fb_req == 0 && c > lim) continue;
                 // register accumulators: blocks of 8 at most (16 spill), but by name,
                 // and where every frame block has to keep one order of sums
-                if (vb == 1 && c == 16 && !want_vb && !(fb_req == 16 && (split > 1 || d == 0 || n_sym > 1))) continue;
+                if (vb == 1 && c == 16 && !want_vb && !(fb_req == 16 && (split > 1 || d == 0 || d >= 3 || n_sym > 1))) continue;
                 if (fits(vb, d, c)) return c;
             }
             return 0;
         };
         // single frames without mirrored copies: every voxel its own rows
         const bool single = force ? force->fb == 1 : fb_req == 1 || (fb_req == 0 && a->n_frame * n_sym == 1);
-        int vb = 0, d = shift <= 2 && !single ? shift : 0, fb = 0;
+        int vb = 0, d = 0, fb = 0;
+        if (!single && shift <= 2) {
+            d = shift;
+        } else if (!single) {   // pairs of voxels, where they stay within 2 rows
+            const int s2 = g->vb_shift(2);
+            d = s2 <= 2 ? 2 + s2 : 0;
+        }
         if (want_vb) {
             fb = pick(vb = want_vb, d);
             if (!fb && want_vb == 1 && a->n_sample > VBS_MAX_SAMPLES && d) fb = pick(vb = 2, d);   // the same bits
@@ -378,8 +390,12 @@ int plan_beamform(rcabf_geometry *g, const rcabf_beamform_args *a, Plan &p, cons
             p.d = d;
             p.fb = fb;
             p.ts = vts;
-            p.wmax = (int)std::min<int64_t>(rows + std::max(d, 1), a->n_sample + d);
+            p.wmax = window(d);
             if (vb == 1) {
+                // FP16 / BF16 single frames keep the weight accuracy of the
+                // one-voxel kernel that they ran on (degree 8)
+                const bool fine = fb_req == 0 && !named && a->n_frame == 1;
+                p.poly_store = like && like->vb == 1 ? like->poly_store : fine ? ST_F32 : p.store;
                 p.n_split = split;
                 p.split_rx = split_rx;
                 p.mirror = mirror;
@@ -530,14 +546,14 @@ static int finish_mask(const rcabf_geometry *g, const rcabf_beamform_args *a, cu
 // shared memory (sets the kernel's shared-memory limit on first use).
 static int resident_ctas(const rcabf_geometry *g0, const Plan &p, size_t smem, DeviceState *ds, int &occ)
 {
-    // variant: (mode, or 4 vb + row shift for the voxel-blocked kernels; kind; fb; store)
-    const std::array<int64_t, 4> var{p.vb ? 4 * p.vb + p.d : g0->mode, g0->kind, p.fb, p.store};
+    // variant: (mode, or 8 vb + row sharing for the voxel-blocked kernels; kind; fb; store)
+    const std::array<int64_t, 4> var{p.vb ? 8 * p.vb + p.d : g0->mode, g0->kind, p.fb, p.vb == 1 ? p.poly_store : p.store};
     const std::array<int64_t, 5> key{var[0], var[1], var[2], var[3], (int64_t)smem};
     std::lock_guard<std::mutex> lk(ds->mu);
     auto lim = ds->smem_limit.find(var);
     if (lim == ds->smem_limit.end() || lim->second < smem) {
         const cudaError_t pe = p.vb == 2   ? prepare_fused_vb(g0->kind, p.d, p.fb, p.store, smem)
-                               : p.vb == 1 ? prepare_fused_vbs(g0->kind, p.d, p.fb, p.store, smem)
+                               : p.vb == 1 ? prepare_fused_vbs(g0->kind, p.d, p.fb, p.poly_store, smem)
                                            : prepare_fused(g0->mode, g0->kind, p.fb, p.store, smem);
         if (pe != cudaSuccess) return cuda_fail(pe, "fused kernel shared-memory attribute");
         ds->smem_limit[var] = smem;
@@ -545,7 +561,7 @@ static int resident_ctas(const rcabf_geometry *g0, const Plan &p, size_t smem, D
     auto oc = ds->occ.find(key);
     if (oc == ds->occ.end()) {
         const int o = p.vb == 2   ? fused_vb_occupancy(g0->kind, p.d, p.fb, p.store, smem)
-                      : p.vb == 1 ? fused_vbs_occupancy(g0->kind, p.d, p.fb, p.store, smem)
+                      : p.vb == 1 ? fused_vbs_occupancy(g0->kind, p.d, p.fb, p.poly_store, smem)
                                   : fused_occupancy(g0->mode, g0->kind, p.fb, p.store, smem);
         oc = ds->occ.emplace(key, o).first;
     }
@@ -578,7 +594,7 @@ int launch_fused_jobs(rcabf_geometry *g0, FusedParams &prm, const Plan &p, cudaS
     const int64_t grid = std::min<int64_t>(prm.n_items, (int64_t)ds->n_sm * occ);
     if (grid <= 0) return RCABF_OK;
     const cudaError_t le = p.vb == 2   ? launch_fused_vb(g0->kind, p.d, p.fb, p.store, prm, (int)grid, smem, st)
-                           : p.vb == 1 ? launch_fused_vbs(g0->kind, p.d, p.fb, p.store, prm, (int)grid, smem, st)
+                           : p.vb == 1 ? launch_fused_vbs(g0->kind, p.d, p.fb, p.poly_store, prm, (int)grid, smem, st)
                                        : launch_fused(g0->mode, g0->kind, p.fb, p.store, prm, (int)grid, smem, st);
     if (le != cudaSuccess) return cuda_fail(le, "fused kernel launch");
     g_launches += 1;
@@ -1102,7 +1118,8 @@ int rcabf_beamform_batch(int n, const rcabf_geometry *const *gs, const rcabf_bea
         if (i == 0) p0 = p;
         plans[i] = p;
         // one launch = one kernel variant: every job fused, same frame block
-        if (p.kernel != RCABF_KERNEL_FUSED || p.fb != p0.fb || p.vb != p0.vb || p.d != p0.d)
+        if (p.kernel != RCABF_KERNEL_FUSED || p.fb != p0.fb || p.vb != p0.vb || p.d != p0.d ||
+            p.poly_store != p0.poly_store)
             return RCABF_ERR_UNSUPPORTED;
         wmax = std::max(wmax, p.wmax);
         if ((s = stage_job(g, &as[i], p, prm.jobs[i], st)) != RCABF_OK) return s;

@@ -198,11 +198,21 @@ static cudaError_t vbs_fb(int d, int fb, const FusedParams *p, int grid, size_t 
     }
 }
 
-// every voxel its own rows: degree-8 weights whatever the storage
+// every voxel its own rows (d = 0), or pairs sharing them (3, 4): degree-8
+// weights whatever the storage
 template <int KIND>
-static cudaError_t vbs_own_rows(int fb, const FusedParams *p, int grid, size_t smem, cudaStream_t st, int what, int *occ)
+static cudaError_t vbs_own_rows(int d, int fb, const FusedParams *p, int grid, size_t smem, cudaStream_t st, int what,
+                                int *occ)
 {
-    switch (fb) {
+    switch (d * 100 + fb) {
+    case 302: return vbs_do<KIND, 2, 8, 3>(p, grid, smem, st, what, occ);
+    case 304: return vbs_do<KIND, 4, 8, 3>(p, grid, smem, st, what, occ);
+    case 308: return vbs_do<KIND, 8, 8, 3>(p, grid, smem, st, what, occ);
+    case 316: return vbs_do<KIND, 16, 8, 3>(p, grid, smem, st, what, occ);
+    case 402: return vbs_do<KIND, 2, 8, 4>(p, grid, smem, st, what, occ);
+    case 404: return vbs_do<KIND, 4, 8, 4>(p, grid, smem, st, what, occ);
+    case 408: return vbs_do<KIND, 8, 8, 4>(p, grid, smem, st, what, occ);
+    case 416: return vbs_do<KIND, 16, 8, 4>(p, grid, smem, st, what, occ);
     case 1: return vbs_do<KIND, 1, 8, 0>(p, grid, smem, st, what, occ);
     case 2: return vbs_do<KIND, 2, 8, 0>(p, grid, smem, st, what, occ);
     case 4: return vbs_do<KIND, 4, 8, 0>(p, grid, smem, st, what, occ);
@@ -226,7 +236,7 @@ static cudaError_t vbs_own_rows(int fb, const FusedParams *p, int grid, size_t s
     cudaError_t vbs_entry_##NAME(int d, int store, int fb, const FusedParams *p, int grid,           \
                                  size_t smem, cudaStream_t st, int what, int *occ)                   \
     {                                                                                                \
-        if (d == 0) return vbs_own_rows<KIND>(fb, p, grid, smem, st, what, occ);                     \
+        if (d == 0 || d >= 3) return vbs_own_rows<KIND>(d, fb, p, grid, smem, st, what, occ);        \
         if (store == ST_F32) return vbs_fb<KIND, VbWeightDeg<ST_F32>::value>(d, fb, p, grid, smem, st, what, occ); \
         return vbs_fb<KIND, VbWeightDeg<ST_F16>::value>(d, fb, p, grid, smem, st, what, occ);        \
     }                                                                                                \

@@ -32,11 +32,12 @@
 // Grids centred on the probe and symmetric transmits: the voxels of half the u
 // (v) axis carry their mirror images as further frames (VBS_MIRROR_*).
 //
-// D >= 1: the four voxels share TAPS + D staged rows (weights shifted to each
+// D = 1, 2: the four voxels share TAPS + D staged rows (weights shifted to each
 // voxel's first row, zeros elsewhere): one 16-byte load feeds 16 FMAs.
-// D = 0: every voxel reads its own TAPS rows.  Single frames, whose two FMAs
-// per row leave the loads cheap, and grids whose steering step spreads a
-// block over more than two rows.
+// D = 3, 4: pairs of voxels share TAPS + D - 2 rows, where the steering step
+// spreads the four over more than two rows but a pair over at most two.
+// D = 0: every voxel reads its own TAPS rows: single frames without mirrored
+// copies, whose two FMAs per row leave the loads cheap, and wider spreads.
 #pragma once
 
 #include "das_common.cuh"
@@ -140,10 +141,12 @@ __global__ void __launch_bounds__(VS_THREADS, vbs_min_ctas(FB)) fused_vbs_kernel
     using KT = KindTraits<KIND>;
     constexpr int VB = VB_BLOCK;
     constexpr int TAPS = KT::TAPS;
-    constexpr int R = TAPS + D;                  // rows a thread reads per step and block (D = 0: per voxel)
+    constexpr int DS = D >= 3 ? D - 2 : D;       // shift rows of a group of voxels
+    constexpr int GV = D >= 3 ? 2 : VB_BLOCK;    // its voxels
+    constexpr int R = TAPS + DS;                 // rows it reads (D = 0: per voxel)
     constexpr int STRIDE = vbs_row_bytes(FB);
     constexpr int NP = FB == 1 ? 1 : FB / 2;     // frame pairs
-    constexpr bool OWN = FB <= 4;                // a block one frame's mirrored copies fill
+    constexpr bool OWN = FB <= 4 || D >= 3;      // (4: a block one frame's mirrored copies fill)
 
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ uint64_t full[VS_STAGES], empty[VS_STAGES];
@@ -262,7 +265,7 @@ __global__ void __launch_bounds__(VS_THREADS, vbs_min_ctas(FB)) fused_vbs_kernel
                             const int hi = min((int)hi_f - KT::LO + TAPS - 1, J.n_sample - 2);
                             if (hi >= lo) {
                                 if (FB == 1) lo &= ~1;   // 8-byte rows: keep the copy 16-byte aligned
-                                cnt = hi + D - lo + 1;   // + shift rows
+                                cnt = hi + DS - lo + 1;   // + shift rows
                                 act = cnt <= prm.wmax;
                                 if (!act) atomicAdd(prm.err_count, 1ull);   // never expected: the planner bounds the window
                             }
@@ -545,83 +548,100 @@ __global__ void __launch_bounds__(VS_THREADS, vbs_min_ctas(FB)) fused_vbs_kernel
                     }
                 }
             } else {
-                // rows shared from the lowest voxel's first one
-                const int row0 = __float_as_int(base + VS_MAGIC) - VS_MAGIC_BITS - KT::LO - h.lo;
-                if (row0 < 0 || row0 + R > h.count) {
-                    atomicAdd(prm.err_count, 1ull);   // never expected: window bound violated
-                    continue;
-                }
-                // weights shifted to each voxel's first row; rows 0 .. D-1 and
-                // TAPS .. R-1 are taken by some of the voxels only.  OWN: the
-                // others leave them out (and a voxel without a contribution
-                // leaves its sums alone), so that a NaN or infinite sample
-                // reaches no voxel whose taps do not touch it, as in the
-                // one-voxel kernel that single frames ran on.  Otherwise they
-                // add zero times the row, as the tensor-memory kernel does
-                // (leaving them out measured 11 % on 8 frames, 10 % on one)
-                float ws[VB][R];
-                bool s1[VB], s2[VB];
+                // groups of GV voxels share rows from their lowest first one.
+                // Weights are shifted to each voxel's first row; rows 0 .. DS-1
+                // and TAPS .. R-1 are taken by some of a group's voxels only.
+                // OWN: the others leave them out (and a voxel without a
+                // contribution leaves its sums alone), so that a NaN or
+                // infinite sample reaches no voxel whose taps do not touch it,
+                // as in the one-voxel kernel that single frames and wide
+                // spreads ran on.  Otherwise they add zero times the row, as
+                // the tensor-memory kernel does (leaving them out measured
+                // 11 % on 8 frames, 10 % on one).
 #pragma unroll
-                for (int j = 0; j < 2; ++j) {
-                    float2 w[TAPS];
-                    poly_weights2<KIND, DEG>(dd[j], w);
+                for (int v0 = 0; v0 < VB; v0 += GV) {
+                    float gb = base;
+                    if constexpr (GV < VB) {
+                        gb = 3.0e38f;
 #pragma unroll
-                    for (int h2 = 0; h2 < 2; ++h2) {
-                        const int v = 2 * j + h2;
-                        const float sh = (h2 ? fl[j].y : fl[j].x) - base;   // rows of shift
-                        if (ok[v] && sh > (float)D + 0.5f) { atomicAdd(prm.err_count, 1ull); ok[v] = false; }
-                        s1[v] = sh > 0.5f;
-                        s2[v] = D >= 2 && sh > 1.5f;
-#pragma unroll
-                        for (int k = 0; k < R; ++k) {
-                            auto wt = [&](int q) {   // OWN: rows the voxel leaves out may carry any weight
-                                const int c = q < 0 ? 0 : q < TAPS ? q : TAPS - 1;
-                                return OWN || c == q ? (h2 ? w[c].y : w[c].x) : 0.0f;
-                            };
-                            float a = wt(k);
-                            if (s1[v]) a = wt(k - 1);
-                            if constexpr (D >= 2) { if (s2[v]) a = wt(k - 2); }
-                            ws[v][k] = a;
-                        }
+                        for (int v = v0; v < v0 + GV; ++v)
+                            if (ok[v]) gb = fminf(gb, v & 1 ? fl[v >> 1].y : fl[v >> 1].x);
                     }
-                }
-                auto uses = [&](int v, int k) {   // whether voxel v adds row k
-                    if (!OWN || (k >= D && k < TAPS)) return true;
-                    if constexpr (D == 1) return k == 0 ? !s1[v] : s1[v];
-                    else return k == 0 ? !s1[v] : k == 1 ? !s2[v] : k == TAPS ? s1[v] : s2[v];
-                };
-                float px[VB], py[VB];
+                    const bool some = GV == VB || gb < 2.0e38f;
+                    const int row = __float_as_int(gb + VS_MAGIC) - VS_MAGIC_BITS - KT::LO - h.lo;
+                    const bool in = row >= 0 && row + R <= h.count;
+                    if (some && !in) {
+                        atomicAdd(prm.err_count, 1ull);   // never expected: window bound violated
 #pragma unroll
-                for (int v = 0; v < VB; ++v) {
-                    const bool use = OWN || ok[v];
-                    px[v] = use ? (v & 1 ? Px[v >> 1].y : Px[v >> 1].x) : 0.0f;
-                    py[v] = use ? (v & 1 ? Py[v >> 1].y : Py[v >> 1].x) : 0.0f;
-                }
-                const uint32_t a0 = slot0 + (uint32_t)i * slot_bytes + (uint32_t)(row0 * STRIDE);
+                        for (int v = v0; v < v0 + GV; ++v) ok[v] = false;
+                    }
+                    const int row0 = some && in ? row : 0;   // (0: any staged row, not added)
+                    float ws[GV][R];
+                    bool s1[GV], s2[GV];
 #pragma unroll
-                for (int p = 0; p < NP; ++p) {
-                    if (p < n_pair) {
-                        float2 tre[VB], tim[VB];
+                    for (int j = 0; j < GV / 2; ++j) {
+                        float2 w[TAPS];
+                        poly_weights2<KIND, DEG>(dd[v0 / 2 + j], w);
 #pragma unroll
-                        for (int v = 0; v < VB; ++v) { tre[v] = make_float2(0.f, 0.f); tim[v] = tre[v]; }
+                        for (int h2 = 0; h2 < 2; ++h2) {
+                            const int q = 2 * j + h2, v = v0 + q;
+                            const float sh = (h2 ? fl[v0 / 2 + j].y : fl[v0 / 2 + j].x) - gb;   // rows of shift
+                            if (ok[v] && sh > (float)DS + 0.5f) { atomicAdd(prm.err_count, 1ull); ok[v] = false; }
+                            s1[q] = sh > 0.5f;
+                            s2[q] = DS >= 2 && sh > 1.5f;
 #pragma unroll
-                        for (int k = 0; k < R; ++k) {
-                            const float4 x = *reinterpret_cast<const float4 *>(smem + a0 + k * STRIDE + p * 16);
-#pragma unroll
-                            for (int v = 0; v < VB; ++v) {
-                                const float2 w2 = make_float2(ws[v][k], ws[v][k]);
-                                if (uses(v, k)) {
-                                    tre[v] = __ffma2_rn(w2, make_float2(x.x, x.y), tre[v]);
-                                    tim[v] = __ffma2_rn(w2, make_float2(x.z, x.w), tim[v]);
-                                }
+                            for (int k = 0; k < R; ++k) {
+                                auto wt = [&](int i) {   // OWN: rows the voxel leaves out may carry any weight
+                                    const int c = i < 0 ? 0 : i < TAPS ? i : TAPS - 1;
+                                    return OWN || c == i ? (h2 ? w[c].y : w[c].x) : 0.0f;
+                                };
+                                float a = wt(k);
+                                if (s1[q]) a = wt(k - 1);
+                                if constexpr (DS >= 2) { if (s2[q]) a = wt(k - 2); }
+                                ws[q][k] = a;
                             }
                         }
+                    }
+                    auto uses = [&](int q, int k) {   // whether the group's voxel q adds row k
+                        if (!OWN || (k >= DS && k < TAPS)) return true;
+                        if constexpr (DS == 1) return k == 0 ? !s1[q] : s1[q];
+                        else return k == 0 ? !s1[q] : k == 1 ? !s2[q] : k == TAPS ? s1[q] : s2[q];
+                    };
+                    float px[GV], py[GV];
 #pragma unroll
-                        for (int v = 0; v < VB; ++v) {
-                            if (OWN && !ok[v]) continue;
-                            const float2 p2 = make_float2(px[v], px[v]);
-                            are[v][p] = __ffma2_rn(p2, tre[v], __ffma2_rn(make_float2(-py[v], -py[v]), tim[v], are[v][p]));
-                            aim[v][p] = __ffma2_rn(p2, tim[v], __ffma2_rn(make_float2(py[v], py[v]), tre[v], aim[v][p]));
+                    for (int q = 0; q < GV; ++q) {
+                        const int v = v0 + q;
+                        const bool use = OWN || ok[v];
+                        px[q] = use ? (v & 1 ? Px[v >> 1].y : Px[v >> 1].x) : 0.0f;
+                        py[q] = use ? (v & 1 ? Py[v >> 1].y : Py[v >> 1].x) : 0.0f;
+                    }
+                    const uint32_t a0 = slot0 + (uint32_t)i * slot_bytes + (uint32_t)(row0 * STRIDE);
+#pragma unroll
+                    for (int p = 0; p < NP; ++p) {
+                        if (p < n_pair) {
+                            float2 tre[GV], tim[GV];
+#pragma unroll
+                            for (int q = 0; q < GV; ++q) { tre[q] = make_float2(0.f, 0.f); tim[q] = tre[q]; }
+#pragma unroll
+                            for (int k = 0; k < R; ++k) {
+                                const float4 x = *reinterpret_cast<const float4 *>(smem + a0 + k * STRIDE + p * 16);
+#pragma unroll
+                                for (int q = 0; q < GV; ++q) {
+                                    const float2 w2 = make_float2(ws[q][k], ws[q][k]);
+                                    if (uses(q, k)) {
+                                        tre[q] = __ffma2_rn(w2, make_float2(x.x, x.y), tre[q]);
+                                        tim[q] = __ffma2_rn(w2, make_float2(x.z, x.w), tim[q]);
+                                    }
+                                }
+                            }
+#pragma unroll
+                            for (int q = 0; q < GV; ++q) {
+                                const int v = v0 + q;
+                                if (OWN && !ok[v]) continue;
+                                const float2 p2 = make_float2(px[q], px[q]);
+                                are[v][p] = __ffma2_rn(p2, tre[q], __ffma2_rn(make_float2(-py[q], -py[q]), tim[q], are[v][p]));
+                                aim[v][p] = __ffma2_rn(p2, tim[q], __ffma2_rn(make_float2(py[q], py[q]), tre[q], aim[v][p]));
+                            }
                         }
                     }
                 }

@@ -86,7 +86,8 @@ cudaError_t prepare_fused_vb(int kind, int d, int fb, int store, size_t smem);
 int fused_vb_occupancy(int kind, int d, int fb, int store, size_t smem);
 
 // Streaming voxel-blocked kernel with register accumulators (EXACT tables):
-// d = row shift bound 1 or 2 with fb in {2, 4, 8, 16}, or 0 (every voxel reads
+// d = row shift bound 1 or 2 with fb in {2, 4, 8, 16}, 3 or 4 (pairs of voxels
+// share rows, bound d - 2) with the same, or 0 (every voxel reads
 // its own rows) with fb in {1, 2, 4, 8, 16}; `store` picks the weight polynomials.
 cudaError_t launch_fused_vbs(int kind, int d, int fb, int store, const FusedParams &p, int grid, size_t smem,
                              cudaStream_t st);

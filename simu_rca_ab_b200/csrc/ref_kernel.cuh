@@ -10,7 +10,7 @@
 // step for the sake of the sample staging (one frame, 48 x 48 x 96 voxels, 16
 // transmits, 64 elements, 6 taps: 7.5 ms, 3.5 here).  Here transmits run side by side,
 // nothing synchronises, and the transmits' sums are added in the reference's
-// order afterwards (launch_ref_sum): the same bits.
+// order afterwards (launch_vbs_reduce): the same bits.
 #pragma once
 
 #include "das_common.cuh"
