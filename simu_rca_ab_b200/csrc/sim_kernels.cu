@@ -48,14 +48,6 @@ struct cpx {
 };
 __device__ __forceinline__ cpx cmul(cpx a, cpx b) { return {a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x}; }
 __device__ __forceinline__ cpx cadd(cpx a, cpx b) { return {a.x + b.x, a.y + b.y}; }
-__device__ __forceinline__ cpx cdiv(cpx a, cpx b)
-{
-    // scaled by the larger component of b (no overflow for the magnitudes here)
-    const float s = fmaxf(fabsf(b.x), fabsf(b.y));
-    const float bx = b.x / s, by = b.y / s;
-    const float d = bx * bx + by * by;
-    return {(a.x * bx + a.y * by) / (s * d), (a.y * bx - a.x * by) / (s * d)};
-}
 __device__ __forceinline__ cpx cexp(cpx a)
 {
     float sn, cs;
@@ -70,7 +62,7 @@ __device__ __forceinline__ cpx cexp(cpx a)
 // of Numerical Recipes, 2nd ed., section 5.4, "complex square root")
 __device__ __forceinline__ cpx csqrt(cpx a)
 {
-    const float m = hypotf(a.x, a.y);
+    const float m = sqrtf(fmaf(a.x, a.x, a.y * a.y));   // (the magnitudes here, pi h^2 / 4.6 to 26, square in range)
     if (!(m > 0.0f)) return {0.0f, 0.0f};
     if (a.x >= 0.0f) {
         const float u = sqrtf(0.5f * (m + a.x));
@@ -79,16 +71,29 @@ __device__ __forceinline__ cpx csqrt(cpx a)
     const float v = copysignf(sqrtf(0.5f * (m - a.x)), a.y);
     return {a.y / (2.0f * v), v};
 }
-// sin(z) / z on the main lobe (|z| < pi), 0 beyond, 1 at 0
+// sin(z) / z on the main lobe (|z| < pi), 0 beyond, 1 at 0.  The kernels are
+// bound by the instructions of a field term, so |z| is compared squared,
+// cosh and sinh of the small attenuation part come from their series (to y^6 /
+// y^7: below 2e-9 relative for |y| < 1/4), and the quotient takes one division.
 __device__ __forceinline__ cpx csinc(cpx z)
 {
-    const float az = hypotf(z.x, z.y);
-    if (!(az > 0.0f)) return {1.0f, 0.0f};
-    if (az >= 3.14159265359f) return {0.0f, 0.0f};
+    const float n2 = fmaf(z.x, z.x, z.y * z.y);
+    if (n2 < 1e-12f) return {1.0f, 0.0f};               // 1 - z^2 / 6
+    if (n2 >= 9.86960440109f) return {0.0f, 0.0f};      // pi^2
     float sn, cs;
     sincosf(z.x, &sn, &cs);
-    const cpx s = {sn * coshf(z.y), cs * sinhf(z.y)};   // sin(x + iy)
-    return cdiv(s, z);
+    float ch, sh;
+    const float y2 = z.y * z.y;
+    if (y2 < 0.0625f) {
+        ch = fmaf(y2, fmaf(y2, fmaf(y2, 1.0f / 720.0f, 1.0f / 24.0f), 0.5f), 1.0f);
+        sh = z.y * fmaf(y2, fmaf(y2, fmaf(y2, 1.0f / 5040.0f, 1.0f / 120.0f), 1.0f / 6.0f), 1.0f);
+    } else {
+        ch = coshf(z.y);
+        sh = sinhf(z.y);
+    }
+    const cpx s = {sn * ch, cs * sh};   // sin(x + iy)
+    const float inv = 1.0f / n2;
+    return {fmaf(s.x, z.x, s.y * z.y) * inv, fmaf(s.y, z.x, -s.x * z.y) * inv};
 }
 
 // 4-term multi-Gaussian expansion of a focused element's elevation aperture
@@ -110,12 +115,13 @@ __device__ cpx dir_flat(float theta, cpx k, float width, bool baffle)
     return d;
 }
 
-__device__ cpx dir_focused(float r, float y, cpx k, float height, float rfocus)
+// inv_r = 1 / r
+__device__ cpx dir_focused(float r, float inv_r, float y, cpx k, float height, float rfocus)
 {
     const cpx ik = {-k.y, k.x};                                 // i k
     const float rdn = 0.5f * (r - rfocus) / (r * rfocus);
     const cpx alpha = {ik.x * rdn, ik.y * rdn};
-    const float yr = y / r, y2r = y * y / (2.0f * r);
+    const float yr = y * inv_r, y2r = 0.5f * y * yr;
     const cpx beta = {-ik.x * yr, -ik.y * yr};                  // -i k y / r
     const cpx gam = {ik.x * y2r, ik.y * y2r};                   // i k y^2 / (2 r)
     const cpx b2 = cmul(beta, beta);
@@ -161,10 +167,11 @@ __device__ cpx element_field(float xs, float ys, float zs, cpx k, float w, const
         const float el = asinf(dy / r) - ele;
         // Green's function exp(i k r) / r
         cpx t = cexp({-k.y * r, k.x * r});
-        t = {t.x / r, t.y / r};
+        const float inv_r = 1.0f / r;
+        t = {t.x * inv_r, t.y * inv_r};
         t = cmul(t, dir_flat(az, k, P.width, P.baffle));
         t = cmul(t, P.rfocus > 10.0f ? dir_flat(el, k, P.width, P.baffle)
-                                     : dir_focused(r, r * sinf(el), k, P.height, P.rfocus));
+                                     : dir_focused(r, inv_r, r * sinf(el), k, P.height, P.rfocus));
         acc = cadd(acc, t);
     }
     acc = cmul(acc, {cl, sl});
