@@ -42,9 +42,9 @@ sys.path.insert(0, str(ROOT))
 METRIC = "DAS voxel·rx·tx/s (nominal, summed over frames)"
 UNIT = "voxel·rx·tx/s"
 # plan kernel -> CUDA kernel function
-KERNEL_NAMES = {"fused_voxel_blocked": "fused_vb_kernel", "fused_voxel_blocked_tmem": "fused_vb_kernel",
+KERNEL_NAMES = {"fused_voxel_blocked": "fused_vbs_kernel", "fused_voxel_blocked_tmem": "fused_vb_kernel",
                 "fused": "fused_das_kernel", "plain": "plain_das_kernel", "fused_tensor_core": "fused_tc_kernel",
-                "fused_tensor_core_fp16w": "fused_tc_kernel"}
+                "fused_tensor_core_fp16w": "fused_tc_kernel", "reference_per_transmit": "ref_das_kernel"}
 
 
 def parse():

@@ -115,14 +115,15 @@ typedef enum rcabf_storage {
 } rcabf_storage;
 
 typedef enum rcabf_kernel {
-    RCABF_KERNEL_AUTO = 0,  /* fused tiled kernel */
+    RCABF_KERNEL_AUTO = 0,  /* the planner's choice among the kernels below */
     RCABF_KERNEL_FUSED = 1, /* persistent voxel-tiled shared-memory gather, all frames in one launch;
                                voxel-blocked along the steering axis when the geometry allows */
     RCABF_KERNEL_PLAIN = 2, /* one launch per frame, one thread per voxel, global gathers */
     RCABF_KERNEL_FUSED_NOBLOCK = 3, /* the fused kernel with one voxel per thread */
     /* the voxel-blocked fused kernel with a given accumulator store
        (RCABF_ERR_UNSUPPORTED where the geometry allows no voxel blocking):
-       tensor memory (sm_100a TMEM) or registers */
+       tensor memory (sm_100a TMEM) or registers (with sample windows streamed
+       ahead by bulk copies: the planner's choice for few frames) */
     RCABF_KERNEL_FUSED_TMEM = 4,
     RCABF_KERNEL_FUSED_REGS = 5,
     /* the tensor-core kernel (sm_100a tcgen05.mma: each (tx, element) step of

@@ -311,6 +311,34 @@ int plan_beamform(rcabf_geometry *g, const rcabf_beamform_args *a, Plan &p, cons
             if (force->ts.tu * force->ts.tv * force->ts.tz != VB_THREADS_HOST) return RCABF_ERR_UNSUPPORTED;
             vts = force->ts;
         }
+        // 16-frame blocks of the tensor-memory kernel take about 0.9 of the
+        // streaming kernel's time a frame (mirrored or not: 0.78 to 0.97 on 12
+        // acquisitions of 13 to 106 frames) when they are full: where the
+        // frames fill 0.84 of them
+        const int64_t b16 = (a->n_frame + 15) / 16 * 16;
+        const bool full16 = !named && !force && shift <= 2 &&
+                            (like ? like->vb == 2 : fb_req == 0 && a->n_frame >= 15 && 100 * a->n_frame >= 84 * b16);
+        if (!force && !named) {
+            // on coarse grids a tile 16 deep spans long windows of which each
+            // voxel uses a few rows: a flatter shape where the time of a step,
+            // about 150 + window rows, times the tiles' padding of the grid
+            // falls by a tenth or more (16 frames, 170 -> 60 rows: 30.3 -> 18.8
+            // ms; 18 frames, 113 -> 32 rows: 12.6 -> 9.4 ms)
+            float sz, su, sv;
+            g->index_steps(sz, su, sv);
+            const int64_t nu = !full16 && (g->mirror & VBS_MIRROR_U) ? (g->n_u + 1) / 2 : g->n_u;
+            const int64_t nv = !full16 && (g->mirror & VBS_MIRROR_V) ? (g->n_v + 1) / 2 : g->n_v;
+            auto padded = [](int64_t n, int64_t t) { return (double)((n + t - 1) / t * t); };
+            auto cost = [&](const TileShape &t) {
+                const double rows = sz * (t.tz - 1) + su * (t.tu - 1) + sv * (t.tv * VB_BLOCK - 1) + kind_taps(g->kind) + 3;
+                return (150.0 + rows) * padded(g->n_z, t.tz) * padded(nu, t.tu) * padded(nv, t.tv * VB_BLOCK);
+            };
+            TileShape best = vts;
+            double least = (full16 ? 0.75 : 0.9) * cost(vts);
+            for (const TileShape &t : {TileShape{4, 4, 8}, TileShape{8, 4, 4}, TileShape{8, 8, 2}})
+                if (cost(t) < least) { least = cost(t); best = t; }
+            vts = best;
+        }
         const int rows = g->window_rows(TileShape{vts.tu, vts.tv * VB_BLOCK, vts.tz});
         // streaming kernel: symmetric axes are mirrored where that drops about
         // half of the tiles (the grid fills the last ones)
@@ -382,7 +410,8 @@ int plan_beamform(rcabf_geometry *g, const rcabf_beamform_args *a, Plan &p, cons
             fb = pick(vb = want_vb, d);
             if (!fb && want_vb == 1 && a->n_sample > VBS_MAX_SAMPLES && d) fb = pick(vb = 2, d);   // the same bits
         } else {
-            fb = pick(vb = 1, d);
+            if (full16) fb = pick(vb = 2, d);
+            if (!fb) fb = pick(vb = 1, d);
             if (!fb) fb = pick(vb = 2, d);
         }
         if (fb) {

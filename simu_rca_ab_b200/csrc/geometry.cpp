@@ -520,6 +520,32 @@ int rcabf_geometry::window_rows(const rcabf::TileShape &ts)
     return (int)std::ceil(m) + rcabf::kind_taps(kind) + 3;
 }
 
+void rcabf_geometry::index_steps(float &z, float &u, float &v)
+{
+    std::lock_guard<std::mutex> lk(mu);
+    if (steps[0] < 0.f) {
+        // |difference| along z and along a of every 5th entry of an odd stride
+        // of rows (NaN, an element outside its aperture, never wins a max)
+        auto scan = [&](const std::vector<float> &tab, int64_t rows, int64_t n_a, float &dz, float &da) {
+            dz = da = 0.f;
+            const int64_t rs = std::max<int64_t>(1, rows / 24);
+            for (int64_t r = 0; r < rows; r += rs)
+                for (int64_t i = r % 5; i < n_a * n_z; i += 5) {
+                    const float *p = &tab[(size_t)(r * n_a * n_z + i)];
+                    if (i % n_z + 1 < n_z) dz = std::max(dz, std::fabs(p[1] - p[0]));
+                    if (i / n_z + 1 < n_a) da = std::max(da, std::fabs(p[n_z] - p[0]));
+                }
+        };
+        float rz, ru, tz, tv;
+        scan(rx_delay, n_ele, n_u, rz, ru);
+        scan(tx_delay, n_tx, n_v, tz, tv);
+        steps = {rz + tz, ru, tv};
+    }
+    z = steps[0];
+    u = steps[1];
+    v = steps[2];
+}
+
 int64_t rcabf_geometry::tc_chunks(const rcabf::TileShape &ts, int64_t n_sample)
 {
     std::lock_guard<std::mutex> lk(mu);

@@ -79,6 +79,11 @@ struct rcabf_geometry {
     // (tx, ele) step: spread of the transmit delay + spread of the receive
     // delay inside the tile (in samples) + the taps + rounding slack.
     int window_rows(const rcabf::TileShape &ts);
+    // Largest change of the sample index (receive + transmit delay) from one
+    // depth, receive column and steering row to the next, from a sample of the
+    // tables: what a tile's extent along each axis adds to its windows.
+    void index_steps(float &z, float &u, float &v);
+    std::array<float, 3> steps{-1.f, 0.f, 0.f};
     // Tensor-core kernel: the 16-row window chunks its producer issues for
     // one frame block over all tiles of this shape and all (tx, element)
     // steps -- the same window arithmetic as the kernel, on the host copies

@@ -140,3 +140,11 @@ def test_a_bad_sample_stays_in_its_voxels(cuda, shift, ny, span, n_frame):
     bad, want = ~torch.isfinite(out.real + out.imag), ~torch.isfinite(ref.real + ref.imag)
     assert torch.equal(bad, want) and 0 < int(want.sum()) < want.numel() // 2
     assert _errcount() == 0
+
+
+@pytest.mark.parametrize("nz,nx,ny,span", [(6, 17, 33, 3.0), (5, 9, 16, 6.0), (9, 40, 20, 2.0)])
+@pytest.mark.parametrize("n_frame", [1, 3, 16, 31])
+def test_coarse_depths_and_full_16_frame_blocks(cuda, nz, nx, ny, span, n_frame):
+    """Depths 13 to 24 samples apart (flat tiles), and frame counts that fill
+    16-frame blocks (the tensor-memory kernel)."""
+    assert _check(_case(nz, nx, ny, span, L4), n_frame, 180) < TOL[8]
