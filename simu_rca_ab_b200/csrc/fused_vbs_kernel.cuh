@@ -21,14 +21,12 @@
 //     assignment leaves SMs idle at the end), and the scan runs on into the
 //     next item while the current one is computed.
 //
-// Measured (B200, against the barrier-per-step kernels it replaced; without
-// and with mirrored copies): 8 frames, 128 x 128 x 256, two orientations 257 ->
-// 152 -> 155 ms; 4 frames of a 256-element probe 361 -> 252 -> 212 ms; 20 frames,
-// 97 x 95 x 159 47.3 -> 31.0 -> 30.0 ms; one frame, 64 x 64 x 128 9.38 -> 1.60 ->
-// 0.94 ms; one frame, 32 x 32 x 64, 4 transmits 455 -> 115 -> 98 us.
-// What bounds it: instruction issue (without copies 64 % of the cycles for one
-// frame, 337 instructions per warp and active step, 140 of them on weights).
-//
+// Measured (B200, against the barrier-per-step kernels it replaced): 8 frames,
+// 128 x 128 x 256, two orientations 257 -> 158 ms; 4 frames of a 256-element probe
+// 361 -> 202 ms; 20 frames, 97 x 95 x 159 47.3 -> 28.5 ms; one frame, 64 x 64 x 128
+// 9.38 -> 0.88 ms; one frame, 32 x 32 x 64, 4 transmits 455 -> 87 us.
+// What bounds it: instruction issue and fixed latencies (8 frames: FMA pipe 58 %
+// busy at 8 and at 12 warps per SM alike; one frame: 48 %, issue 56 %).
 // Grids centred on the probe and symmetric transmits: the voxels of half the u
 // (v) axis carry their mirror images as further frames (VBS_MIRROR_*).
 //

@@ -139,9 +139,10 @@ constexpr RCABF_HD int vbs_mirrored(int mirror, int s)
 constexpr int VBS_MAX_RECORDS = 8;
 constexpr int VBS_MAX_SAMPLES = 1 << 21;
 // CTAs per SM its registers are budgeted for: 2 x 4 x FB accumulators, the
-// weights and the per-voxel transmit state.  With 8 frames a third CTA (168
-// registers, spills) measured 6 % slower than two; with 4 a fourth 4 % slower
-// than three.
+// weights and the row in flight.  8 frames: three CTAs of 168 registers against
+// two of 244: 28.9 against 32.3 ms (20 frames, 97 x 95 x 159), 201 against 222
+// ms (4 frames, mirrored, 256 elements).  4 frames: three against four of 128
+// registers: 0.90 against 1.00 ms (one frame, mirrored, 64 x 64 x 128).
 constexpr RCABF_HD int vbs_min_ctas(int fb) { return fb >= 16 ? 2 : fb >= 4 ? 3 : 4; }
 constexpr int VBS_PAD_ROWS = 2;      // zero rows past the record (shift rows)
 constexpr RCABF_HD int vbs_row_bytes(int fb) { return fb <= 2 ? 8 * fb : 8 * fb + 16; }
