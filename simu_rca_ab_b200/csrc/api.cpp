@@ -424,7 +424,7 @@ int plan_beamform(rcabf_geometry *g, const rcabf_beamform_args *a, Plan &p, cons
                 // FP16 / BF16 single frames keep the weight accuracy of the
                 // one-voxel kernel that they ran on (degree 8)
                 const bool fine = fb_req == 0 && !named && a->n_frame == 1;
-                p.poly_store = like && like->vb == 1 ? like->poly_store : fine ? ST_F32 : p.store;
+                p.deg = like && like->vb == 1 ? like->deg : vbs_weight_degree(d, fine ? ST_F32 : p.store);
                 p.n_split = split;
                 p.split_rx = split_rx;
                 p.mirror = mirror;
@@ -575,14 +575,15 @@ static int finish_mask(const rcabf_geometry *g, const rcabf_beamform_args *a, cu
 // shared memory (sets the kernel's shared-memory limit on first use).
 static int resident_ctas(const rcabf_geometry *g0, const Plan &p, size_t smem, DeviceState *ds, int &occ)
 {
-    // variant: (mode, or 8 vb + row sharing for the voxel-blocked kernels; kind; fb; store)
-    const std::array<int64_t, 4> var{p.vb ? 8 * p.vb + p.d : g0->mode, g0->kind, p.fb, p.vb == 1 ? p.poly_store : p.store};
+    // variant, one per kernel function: (mode, or 8 vb + row sharing for the voxel-blocked kernels; kind; fb;
+    // storage, for the streaming kernel, which is compiled per weight degree, that)
+    const std::array<int64_t, 4> var{p.vb ? 8 * p.vb + p.d : g0->mode, g0->kind, p.fb, p.vb == 1 ? p.deg : p.store};
     const std::array<int64_t, 5> key{var[0], var[1], var[2], var[3], (int64_t)smem};
     std::lock_guard<std::mutex> lk(ds->mu);
     auto lim = ds->smem_limit.find(var);
     if (lim == ds->smem_limit.end() || lim->second < smem) {
         const cudaError_t pe = p.vb == 2   ? prepare_fused_vb(g0->kind, p.d, p.fb, p.store, smem)
-                               : p.vb == 1 ? prepare_fused_vbs(g0->kind, p.d, p.fb, p.poly_store, smem)
+                               : p.vb == 1 ? prepare_fused_vbs(g0->kind, p.d, p.fb, p.deg, smem)
                                            : prepare_fused(g0->mode, g0->kind, p.fb, p.store, smem);
         if (pe != cudaSuccess) return cuda_fail(pe, "fused kernel shared-memory attribute");
         ds->smem_limit[var] = smem;
@@ -590,7 +591,7 @@ static int resident_ctas(const rcabf_geometry *g0, const Plan &p, size_t smem, D
     auto oc = ds->occ.find(key);
     if (oc == ds->occ.end()) {
         const int o = p.vb == 2   ? fused_vb_occupancy(g0->kind, p.d, p.fb, p.store, smem)
-                      : p.vb == 1 ? fused_vbs_occupancy(g0->kind, p.d, p.fb, p.poly_store, smem)
+                      : p.vb == 1 ? fused_vbs_occupancy(g0->kind, p.d, p.fb, p.deg, smem)
                                   : fused_occupancy(g0->mode, g0->kind, p.fb, p.store, smem);
         oc = ds->occ.emplace(key, o).first;
     }
@@ -623,7 +624,7 @@ int launch_fused_jobs(rcabf_geometry *g0, FusedParams &prm, const Plan &p, cudaS
     const int64_t grid = std::min<int64_t>(prm.n_items, (int64_t)ds->n_sm * occ);
     if (grid <= 0) return RCABF_OK;
     const cudaError_t le = p.vb == 2   ? launch_fused_vb(g0->kind, p.d, p.fb, p.store, prm, (int)grid, smem, st)
-                           : p.vb == 1 ? launch_fused_vbs(g0->kind, p.d, p.fb, p.poly_store, prm, (int)grid, smem, st)
+                           : p.vb == 1 ? launch_fused_vbs(g0->kind, p.d, p.fb, p.deg, prm, (int)grid, smem, st)
                                        : launch_fused(g0->mode, g0->kind, p.fb, p.store, prm, (int)grid, smem, st);
     if (le != cudaSuccess) return cuda_fail(le, "fused kernel launch");
     g_launches += 1;
@@ -1148,7 +1149,7 @@ int rcabf_beamform_batch(int n, const rcabf_geometry *const *gs, const rcabf_bea
         plans[i] = p;
         // one launch = one kernel variant: every job fused, same frame block
         if (p.kernel != RCABF_KERNEL_FUSED || p.fb != p0.fb || p.vb != p0.vb || p.d != p0.d ||
-            p.poly_store != p0.poly_store)
+            p.deg != p0.deg)
             return RCABF_ERR_UNSUPPORTED;
         wmax = std::max(wmax, p.wmax);
         if ((s = stage_job(g, &as[i], p, prm.jobs[i], st)) != RCABF_OK) return s;

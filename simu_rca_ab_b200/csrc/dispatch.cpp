@@ -23,7 +23,7 @@ cudaError_t plain_entry_ref(int kind, const PlainParams &p, cudaStream_t st);
 #define DECL_VB(NAME)                                                                                \
     cudaError_t vb_entry_##NAME(int d, int store, int fb, const FusedParams *p, int grid,            \
                                 size_t smem, cudaStream_t st, int what, int *occ);                    \
-    cudaError_t vbs_entry_##NAME(int d, int store, int fb, const FusedParams *p, int grid,           \
+    cudaError_t vbs_entry_##NAME(int d, int deg, int fb, const FusedParams *p, int grid,             \
                                  size_t smem, cudaStream_t st, int what, int *occ);
 DECL_VB(exact_quad3)
 DECL_VB(exact_ref6)
@@ -32,32 +32,33 @@ DECL_VB(exact_l3)
 DECL_VB(exact_l4)
 #undef DECL_VB
 
+// (`var`: the storage for vb, the weight degree for vbs)
 #define ROUTE_VB(WHICH)                                                                                   \
-    static cudaError_t WHICH##_route(int kind, int d, int fb, int store, const FusedParams *p, int grid,  \
+    static cudaError_t WHICH##_route(int kind, int d, int fb, int var, const FusedParams *p, int grid,    \
                                      size_t smem, cudaStream_t st, int what, int *occ)                    \
     {                                                                                                     \
         switch (kind) {                                                                                   \
-        case K_QUAD3: return WHICH##_entry_exact_quad3(d, store, fb, p, grid, smem, st, what, occ);       \
-        case K_REF6: return WHICH##_entry_exact_ref6(d, store, fb, p, grid, smem, st, what, occ);         \
-        case K_LANCZOS2: return WHICH##_entry_exact_l2(d, store, fb, p, grid, smem, st, what, occ);       \
-        case K_LANCZOS3: return WHICH##_entry_exact_l3(d, store, fb, p, grid, smem, st, what, occ);       \
-        case K_LANCZOS4: return WHICH##_entry_exact_l4(d, store, fb, p, grid, smem, st, what, occ);       \
+        case K_QUAD3: return WHICH##_entry_exact_quad3(d, var, fb, p, grid, smem, st, what, occ);         \
+        case K_REF6: return WHICH##_entry_exact_ref6(d, var, fb, p, grid, smem, st, what, occ);           \
+        case K_LANCZOS2: return WHICH##_entry_exact_l2(d, var, fb, p, grid, smem, st, what, occ);         \
+        case K_LANCZOS3: return WHICH##_entry_exact_l3(d, var, fb, p, grid, smem, st, what, occ);         \
+        case K_LANCZOS4: return WHICH##_entry_exact_l4(d, var, fb, p, grid, smem, st, what, occ);         \
         default: return cudaErrorInvalidValue;                                                            \
         }                                                                                                 \
     }                                                                                                     \
-    cudaError_t launch_fused_##WHICH(int kind, int d, int fb, int store, const FusedParams &p, int grid,  \
+    cudaError_t launch_fused_##WHICH(int kind, int d, int fb, int var, const FusedParams &p, int grid,    \
                                      size_t smem, cudaStream_t st)                                        \
     {                                                                                                     \
-        return WHICH##_route(kind, d, fb, store, &p, grid, smem, st, 0, nullptr);                         \
+        return WHICH##_route(kind, d, fb, var, &p, grid, smem, st, 0, nullptr);                           \
     }                                                                                                     \
-    cudaError_t prepare_fused_##WHICH(int kind, int d, int fb, int store, size_t smem)                    \
+    cudaError_t prepare_fused_##WHICH(int kind, int d, int fb, int var, size_t smem)                      \
     {                                                                                                     \
-        return WHICH##_route(kind, d, fb, store, nullptr, 0, smem, nullptr, 1, nullptr);                  \
+        return WHICH##_route(kind, d, fb, var, nullptr, 0, smem, nullptr, 1, nullptr);                    \
     }                                                                                                     \
-    int fused_##WHICH##_occupancy(int kind, int d, int fb, int store, size_t smem)                        \
+    int fused_##WHICH##_occupancy(int kind, int d, int fb, int var, size_t smem)                          \
     {                                                                                                     \
         int occ = 0;                                                                                      \
-        if (WHICH##_route(kind, d, fb, store, nullptr, 0, smem, nullptr, 2, &occ) != cudaSuccess) return 0; \
+        if (WHICH##_route(kind, d, fb, var, nullptr, 0, smem, nullptr, 2, &occ) != cudaSuccess) return 0; \
         return occ;                                                                                       \
     }
 ROUTE_VB(vb)

@@ -233,11 +233,12 @@ static cudaError_t vbs_own_rows(int d, int fb, const FusedParams *p, int grid, s
         if (d == 2) return vb_store<KIND, 2>(store, fb, p, grid, smem, st, what, occ);               \
         return cudaErrorInvalidValue;                                                                \
     }                                                                                                \
-    cudaError_t vbs_entry_##NAME(int d, int store, int fb, const FusedParams *p, int grid,           \
+    cudaError_t vbs_entry_##NAME(int d, int deg, int fb, const FusedParams *p, int grid,             \
                                  size_t smem, cudaStream_t st, int what, int *occ)                   \
     {                                                                                                \
-        if (d == 0 || d >= 3) return vbs_own_rows<KIND>(d, fb, p, grid, smem, st, what, occ);        \
-        if (store == ST_F32) return vbs_fb<KIND, VbWeightDeg<ST_F32>::value>(d, fb, p, grid, smem, st, what, occ); \
-        return vbs_fb<KIND, VbWeightDeg<ST_F16>::value>(d, fb, p, grid, smem, st, what, occ);        \
+        if (d == 0 || d >= 3)                                                                        \
+            return deg == 8 ? vbs_own_rows<KIND>(d, fb, p, grid, smem, st, what, occ) : cudaErrorInvalidValue; \
+        if (deg == 8) return vbs_fb<KIND, 8>(d, fb, p, grid, smem, st, what, occ);                   \
+        return deg == 6 ? vbs_fb<KIND, 6>(d, fb, p, grid, smem, st, what, occ) : cudaErrorInvalidValue; \
     }                                                                                                \
     }

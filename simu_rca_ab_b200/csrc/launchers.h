@@ -88,11 +88,12 @@ int fused_vb_occupancy(int kind, int d, int fb, int store, size_t smem);
 // Streaming voxel-blocked kernel with register accumulators (EXACT tables):
 // d = row shift bound 1 or 2 with fb in {2, 4, 8, 16}, 3 or 4 (pairs of voxels
 // share rows, bound d - 2) with the same, or 0 (every voxel reads
-// its own rows) with fb in {1, 2, 4, 8, 16}; `store` picks the weight polynomials.
-cudaError_t launch_fused_vbs(int kind, int d, int fb, int store, const FusedParams &p, int grid, size_t smem,
+// its own rows) with fb in {1, 2, 4, 8, 16}; deg = degree of the weight polynomials
+// (vbs_weight_degree): each (kind, d, fb, deg) is one kernel function.
+cudaError_t launch_fused_vbs(int kind, int d, int fb, int deg, const FusedParams &p, int grid, size_t smem,
                              cudaStream_t st);
-cudaError_t prepare_fused_vbs(int kind, int d, int fb, int store, size_t smem);
-int fused_vbs_occupancy(int kind, int d, int fb, int store, size_t smem);
+cudaError_t prepare_fused_vbs(int kind, int d, int fb, int deg, size_t smem);
+int fused_vbs_occupancy(int kind, int d, int fb, int deg, size_t smem);
 // out (+)= the transmit ranges' sums, n elements each
 cudaError_t launch_vbs_reduce(float2 *out, const float2 *partial, int64_t n, int n_split, int accumulate,
                               cudaStream_t st);

@@ -22,7 +22,7 @@ struct Plan {
     int n_split = 1, split_rx = 1;   // vb = 1: ranges of steps, one work item each; of them along the elements
     int mirror = 0, n_sym = 1;          // vb = 1: mirrored axes, copies of a frame (VBS_MIRROR_*)
     int64_t nu_t = 0, nv_t = 0;         // vb = 1: tile-space extents
-    int poly_store = 0;                 // vb = 1: the storage whose weight polynomials it takes
+    int deg = 0;                        // vb = 1: degree of its weight polynomials
     int compact = 0;                    // vb = 1: one slab for the steps that mirror each other
     int slab_tx = 0, slab_ele = 0;      // transmits and elements that have a slab
     int tc = 0;           // tensor-core kernel (fused_tc_kernel.cuh): 1 FP16 weights, 2 hi + remainder weights

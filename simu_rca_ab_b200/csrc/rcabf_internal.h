@@ -136,6 +136,9 @@ constexpr RCABF_HD int vbs_mirrored(int mirror, int s)
 {
     return mirror == (VBS_MIRROR_U | VBS_MIRROR_V) ? s : s ? mirror : 0;
 }
+// Degree of its weight polynomials: that of the storage where voxels share rows
+// (d = 1, 2; the tensor-memory kernel's), the highest where pairs do or none.
+constexpr RCABF_HD int vbs_weight_degree(int d, int store) { return (d == 1 || d == 2) && store != ST_F32 ? 6 : 8; }
 constexpr int VBS_MAX_RECORDS = 8;
 constexpr int VBS_MAX_SAMPLES = 1 << 21;
 // CTAs per SM its registers are budgeted for: 2 x 4 x FB accumulators, the

@@ -155,7 +155,7 @@ static bool same_variant(const Request *a, const Request *b)
     return a->batchable && b->batchable && a->g->device == b->g->device && a->g->mode == b->g->mode && a->g->kind == b->g->kind &&
            a->a.storage == b->a.storage && a->plan.kernel == RCABF_KERNEL_FUSED &&
            b->plan.kernel == RCABF_KERNEL_FUSED && a->plan.fb == b->plan.fb && a->plan.vb == b->plan.vb &&
-           a->plan.d == b->plan.d && a->plan.tc == b->plan.tc && a->plan.poly_store == b->plan.poly_store;
+           a->plan.d == b->plan.d && a->plan.tc == b->plan.tc && a->plan.deg == b->plan.deg;
 }
 
 static void finish_locked(rcabf_server *s, Request *r, int status, Clock::time_point now)
@@ -380,7 +380,7 @@ int rcabf_server_submit(rcabf_server *s, const rcabf_geometry *g, const rcabf_be
         Plan p2;
         if (plan_beamform(gg, &pinned, p2) == RCABF_OK && p2.vb == r->plan.vb && p2.d == r->plan.d &&
             p2.tc == r->plan.tc && p2.fb == r->plan.fb && p2.total == r->plan.total &&
-            p2.poly_store == r->plan.poly_store) {
+            p2.deg == r->plan.deg) {
             r->a = pinned;
             r->batchable = true;
         }
