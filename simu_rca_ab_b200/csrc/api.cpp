@@ -161,18 +161,20 @@ int plan_beamform(rcabf_geometry *g, const rcabf_beamform_args *a, Plan &p, cons
     // per-(voxel, transmit) kernel, whose transmit sums take n_tx volumes.
     // (One frame, 6 taps: 7.5 -> 3.5 ms; the fused kernel shares a step's sine
     // and divide work between the frames of its block, up to 16, and the gather
-    // kernel only between 4.)
+    // kernel only between 4.)  A chunk of a longer call stays with the call's kernel.
     bool has_tuned = false;
     if (g->mode == MODE_REF) {
         std::lock_guard<std::mutex> lk(g->mu);
         has_tuned = g->tuned.count({a->n_frame, (int64_t)a->storage}) > 0;
     }
-    if (g->mode == MODE_REF && !force && !has_tuned && fb_req == 0 && a->n_frame <= REF_MAX_FRAMES &&
+    if (g->mode == MODE_REF && !force && !has_tuned && fb_req == 0 && (!like || like->ref) && a->n_frame <= REF_MAX_FRAMES &&
         (a->kernel == RCABF_KERNEL_AUTO || a->kernel == RCABF_KERNEL_FUSED) && g->n_tx <= 65535) {
         p.ref = 1;
+        p.fb = a->n_frame >= 3 ? 4 : (int)a->n_frame;   // frames that share a step's work
         p.total = a->compound ? (size_t)g->n_tx * a->n_frame * g->n_pix * sizeof(float2) : 0;
         if (p.total <= REF_MAX_BYTES) return RCABF_OK;
         p.ref = 0;
+        p.fb = 1;
         p.total = 0;
     }
     TuneChoice tuned;
@@ -1006,10 +1008,15 @@ int host_layout(rcabf_geometry *g, const rcabf_beamform_args *a, int32_t frames_
     h.in_bytes = align256((size_t)h.chunk * a->n_tx * a->n_ch * a->n_sample * iq_sample_bytes(a->iq_dtype));
     h.out_bytes = align256((size_t)h.chunk * n_t * g->n_pix * 8);
     rcabf_beamform_args c = *a;
-    c.n_frame = h.chunk;
-    Plan pc;
-    if ((s = chunk_plan(g, &c, h, pc)) != RCABF_OK) return s;
-    h.plan_bytes = align256(pc.total);
+    // the last chunk may be shorter, and its plan need more (a smaller frame
+    // block, other sums than its frames')
+    const int64_t last = a->n_frame % h.chunk;
+    for (int64_t nf : {h.chunk, last ? last : h.chunk}) {
+        c.n_frame = nf;
+        Plan pc;
+        if ((s = chunk_plan(g, &c, h, pc)) != RCABF_OK) return s;
+        h.plan_bytes = std::max(h.plan_bytes, align256(pc.total));
+    }
     h.total = 2 * h.in_bytes + 2 * h.out_bytes + h.plan_bytes;
     return RCABF_OK;
 }

@@ -47,3 +47,35 @@ def test_shared_memory_limit_is_kept_per_kernel_function(built, span, stores, n_
     for k, store in enumerate(stores):
         i = big if k in (0, len(stores) - 1) else small
         assert h.beamform(g[i], h.args(g[i], n_frame, 300, storage=store)) == 0, (k, store)
+
+
+FRAMES_CHUNKS = [(n, c) for n in (2, 4, 9, 13, 16, 18, 20, 31, 36, 40) for c in (0, 1, 2, 3, 5, 7, 8)]
+
+
+@pytest.mark.parametrize("tables,shift,nz,nx,ny,stores", [
+    ("ref_compat", 0.0, 40, 24, 24, (F32,)), ("exact", 0.0, 40, 32, 32, (F32, F16)),
+    ("exact", 1e-3, 40, 32, 32, (F32, F16)), ("exact", 0.0, 6, 17, 33, (F32, BF16))])
+def test_host_buffer_call_fits_the_workspace_it_asks_for(host, tables, shift, nz, nx, ny, stores):
+    """Every chunk of a host-buffer call, the shorter last one too, fits the
+    scratch size the call reported, on grids with more voxels than channel
+    samples; reference tables keep one kernel for all chunks."""
+    g = host.geometry(*acquisition(nz, nx, ny, 2.0, shift=shift, n_ele=8, tables=tables,
+                                   interp=("ref6", 3) if tables == "ref_compat" else ("lanczos", 4)))
+    for n_frame, chunk in FRAMES_CHUNKS:
+        for store in stores:
+            for compound in (True, False):
+                a = host.args(g, n_frame, 97, storage=store, compound=compound)
+                host.log()
+                assert host.beamform_host(g, a, chunk) == 0, (n_frame, chunk, store, compound)
+                kernels = {line.split()[0] for line in host.log()}
+                if tables == "ref_compat":
+                    assert kernels == {"ref" if n_frame <= 4 else "fused"}, (n_frame, chunk)
+
+
+def test_host_buffer_call_on_few_reference_frames_is_one_launch(host):
+    """Up to 4 frames share the per-transmit kernel's work: one chunk."""
+    g = host.geometry(*acquisition(20, 12, 12, 2.0, n_ele=8, tables="ref_compat", interp=("ref6", 3)))
+    for n_frame in (1, 2, 3, 4):
+        host.log()
+        assert host.beamform_host(g, host.args(g, n_frame, 97), 0) == 0
+        assert host.log() == [f"ref 1 frames {n_frame}"]
