@@ -163,7 +163,7 @@ int plan_beamform(rcabf_geometry *g, const rcabf_beamform_args *a, Plan &p, cons
     // and divide work between the frames of its block, up to 16, and the gather
     // kernel only between 4.)  A chunk of a longer call stays with the call's kernel.
     bool has_tuned = false;
-    if (g->mode == MODE_REF) {
+    if (g->mode == MODE_REF && !like) {
         std::lock_guard<std::mutex> lk(g->mu);
         has_tuned = g->tuned.count({a->n_frame, (int64_t)a->storage}) > 0;
     }
@@ -178,7 +178,7 @@ int plan_beamform(rcabf_geometry *g, const rcabf_beamform_args *a, Plan &p, cons
         p.total = 0;
     }
     TuneChoice tuned;
-    if (!force) {   // a choice the autotuner measured for this geometry, frames and storage
+    if (!force && !like) {   // a choice the autotuner measured for this geometry, frames and storage
         std::lock_guard<std::mutex> lk(g->mu);
         auto it = g->tuned.find({a->n_frame, (int64_t)a->storage});
         const int vb_req = a->kernel == RCABF_KERNEL_FUSED_TMEM ? 2 : a->kernel == RCABF_KERNEL_FUSED_REGS ? 1 : -1;
@@ -299,7 +299,12 @@ int plan_beamform(rcabf_geometry *g, const rcabf_beamform_args *a, Plan &p, cons
                         : a->kernel == RCABF_KERNEL_FUSED_REGS ? 1
                                                                : 0;   // 0: the planner's choice
     const bool named = !force && want_vb > 0;   // by name: row-sharing blocks of 2 frames or more only
+    // a chunk of a call (`like`: that call's plan) keeps its kernel, row sharing,
+    // weights, tile and ranges, all that the order of its sums and their terms
+    // depend on; only the frame block is its own
+    const bool follow = like && like->kernel == RCABF_KERNEL_FUSED && !like->ref && !like->tc;
     const bool vb_fb_ok = force ? force->vb >= 1
+                          : follow ? like->vb >= 1
                                 : fb_req == 0 ? (!named || a->n_frame >= 2)
                                               : (fb_req == 2 || fb_req == 4 || fb_req == 8 || fb_req == 16 ||
                                                  (!named && fb_req == 1));
@@ -312,15 +317,17 @@ int plan_beamform(rcabf_geometry *g, const rcabf_beamform_args *a, Plan &p, cons
         if (force) {
             if (force->ts.tu * force->ts.tv * force->ts.tz != VB_THREADS_HOST) return RCABF_ERR_UNSUPPORTED;
             vts = force->ts;
+        } else if (follow) {
+            vts = like->ts;
         }
         // 16-frame blocks of the tensor-memory kernel take about 0.9 of the
         // streaming kernel's time a frame (mirrored or not: 0.78 to 0.97 on 12
         // acquisitions of 13 to 106 frames) when they are full: where the
         // frames fill 0.84 of them
         const int64_t b16 = (a->n_frame + 15) / 16 * 16;
-        const bool full16 = !named && !force && shift <= 2 &&
-                            (like ? like->vb == 2 : fb_req == 0 && a->n_frame >= 15 && 100 * a->n_frame >= 84 * b16);
-        if (!force && !named) {
+        const bool full16 = !named && !force && shift <= 2 && fb_req == 0 && a->n_frame >= 15 &&
+                            100 * a->n_frame >= 84 * b16;
+        if (!force && !named && !follow) {
             // on coarse grids a tile 16 deep spans long windows of which each
             // voxel uses a few rows: a flatter shape where the time of a step,
             // about 150 + window rows, times the tiles' padding of the grid
@@ -349,18 +356,17 @@ int plan_beamform(rcabf_geometry *g, const rcabf_beamform_args *a, Plan &p, cons
         int mirror = named ? 0 : g->mirror;
         if (5 * n_tiles((g->n_u + 1) / 2, vts.tu) > 3 * n_tiles(g->n_u, vts.tu)) mirror &= ~VBS_MIRROR_U;
         if (5 * n_tiles((g->n_v + 1) / 2, tile_v) > 3 * n_tiles(g->n_v, tile_v)) mirror &= ~VBS_MIRROR_V;
+        if (follow) mirror = like->mirror;
         const int n_sym = (mirror & VBS_MIRROR_U ? 2 : 1) * (mirror & VBS_MIRROR_V ? 2 : 1);
         const int64_t tiles = n_tiles(g->n_z, vts.tz) *
                               n_tiles(mirror & VBS_MIRROR_U ? (g->n_u + 1) / 2 : g->n_u, vts.tu) *
                               n_tiles(mirror & VBS_MIRROR_V ? (g->n_v + 1) / 2 : g->n_v, tile_v);
         // few work items are split into ranges of transmits, and up to 16 in all
         // of elements, to about two items per resident CTA.  The ranges set the
-        // order of the sums: they do not depend on the frame block, and a
-        // caller that cuts one acquisition into several calls passes the whole
-        // one's plan.
+        // order of the sums: they do not depend on the frame block.
         int split = a->compound ? 1 : g->n_tx, split_rx = 1;
         if (a->compound && !named) {
-            if (like && like->vb == 1) {
+            if (follow) {
                 split = like->n_split;
                 split_rx = like->split_rx;
             } else {
@@ -390,7 +396,9 @@ int plan_beamform(rcabf_geometry *g, const rcabf_beamform_args *a, Plan &p, cons
                 // the planner's choice: at most the frame count rounded up to a
                 // power of two (a block more than half empty costs more than
                 // the setup it saves); a store asked for by name may pad to 2x
-                const int64_t lim = want_vb ? 2 * a->n_frame : pow2_ceil(a->n_frame * (vb == 1 ? n_sym : 1));
+                // (and a one-frame chunk of a call whose voxels share rows, to 2)
+                const int64_t lim = want_vb ? 2 * a->n_frame
+                                            : std::max(pow2_ceil(a->n_frame * (vb == 1 ? n_sym : 1)), follow && d > 0 ? 2 : 1);
                 if (!force && fb_req == 0 && c > lim) continue;
                 // register accumulators: blocks of 8 at most (16 spill), but by name,
                 // and where every frame block has to keep one order of sums
@@ -402,13 +410,17 @@ int plan_beamform(rcabf_geometry *g, const rcabf_beamform_args *a, Plan &p, cons
         // single frames without mirrored copies: every voxel its own rows
         const bool single = force ? force->fb == 1 : fb_req == 1 || (fb_req == 0 && a->n_frame * n_sym == 1);
         int vb = 0, d = 0, fb = 0;
-        if (!single && shift <= 2) {
+        if (follow) {
+            d = like->d;
+        } else if (!single && shift <= 2) {
             d = shift;
         } else if (!single) {   // pairs of voxels, where they stay within 2 rows
             const int s2 = g->vb_shift(2);
             d = s2 <= 2 ? 2 + s2 : 0;
         }
-        if (want_vb) {
+        if (follow) {
+            fb = pick(vb = like->vb, d);
+        } else if (want_vb) {
             fb = pick(vb = want_vb, d);
             if (!fb && want_vb == 1 && a->n_sample > VBS_MAX_SAMPLES && d) fb = pick(vb = 2, d);   // the same bits
         } else {
@@ -426,7 +438,7 @@ int plan_beamform(rcabf_geometry *g, const rcabf_beamform_args *a, Plan &p, cons
                 // FP16 / BF16 single frames keep the weight accuracy of the
                 // one-voxel kernel that they ran on (degree 8)
                 const bool fine = fb_req == 0 && !named && a->n_frame == 1;
-                p.deg = like && like->vb == 1 ? like->deg : vbs_weight_degree(d, fine ? ST_F32 : p.store);
+                p.deg = follow ? like->deg : vbs_weight_degree(d, fine ? ST_F32 : p.store);
                 p.n_split = split;
                 p.split_rx = split_rx;
                 p.mirror = mirror;

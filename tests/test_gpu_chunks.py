@@ -1,0 +1,44 @@
+"""Host-buffer calls cut into chunks, a last one of one frame among them, give
+the bits of the call on device buffers: grids with and without mirror symmetry,
+steep steering, reference tables, half-precision data."""
+import warnings
+
+import numpy as np
+import pytest
+
+from tests.host_runtime import acquisition
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("span,shift,storage,tables", [
+    (2.0, 1e-3, "float16", "exact"), (2.0, 0.0, "float16", "exact"), (20.0, 0.0, "float32", "exact"),
+    (30.0, 1e-3, "float32", "exact"), (2.0, 0.0, "float32", "ref_compat")])
+@pytest.mark.parametrize("n_frame,chunks", [(9, (0, 1, 8)), (20, (0, 8, 16)), (16, (0, 5))])
+def test_chunked_host_call_gives_the_device_calls_bits(cuda, span, shift, storage, tables, n_frame, chunks):
+    import torch
+    from simu_rca_ab_b200 import _lib as L
+    from simu_rca_ab_b200 import beamformer as B
+    from simu_rca_ab_b200.params import normalize
+    ns, half = 180, storage == "float16"
+    acq = acquisition(40, 17, 21, span, shift=shift, tables=tables, n_ele=8 if tables == "ref_compat" else 24,
+                      interp=("ref6", 3) if tables == "ref_compat" else ("lanczos", 4))
+    eng = B.default_engine()
+    with warnings.catch_warnings():
+        warnings.simplefilter("ignore")
+        geom = eng.geometry(normalize(np.zeros(1, np.complex64), *acq))
+    g = torch.Generator(device="cuda").manual_seed(4)
+    iq = torch.randn(n_frame, geom.n_tx, geom.n_ele, ns, dtype=torch.complex64, device="cuda", generator=g)
+    if half:
+        iq = iq.to(torch.complex32)
+    kw = dict(iq_dtype=L.IQ_C32 if half else L.IQ_C64, n_sample=ns, n_frame=n_frame, mask=None, compound=True,
+              storage=L.STORE_F16 if half else L.STORE_F32)
+    out = torch.empty((n_frame, 1, geom.n_pix), dtype=torch.complex64, device="cuda")
+    eng.run(geom, eng.make_args(geom, iq, out=out, **kw))
+    iq_h, ref = iq.cpu().pin_memory(), out.cpu()
+    assert float(ref.abs().max()) > 0.0
+    for chunk in chunks:
+        out_h = torch.full(out.shape, float("nan"), dtype=torch.complex64).pin_memory()
+        eng.run_host(geom, eng.make_args(geom, iq_h, out=out_h, host=True, **kw), frames_per_chunk=chunk)
+        torch.cuda.synchronize()
+        assert torch.equal(out_h, ref), chunk

@@ -79,3 +79,31 @@ def test_host_buffer_call_on_few_reference_frames_is_one_launch(host):
         host.log()
         assert host.beamform_host(g, host.args(g, n_frame, 97), 0) == 0
         assert host.log() == [f"ref 1 frames {n_frame}"]
+
+
+def _sums(line):
+    """What the order and the terms of a launch's sums depend on: the kernel,
+    its row sharing and weights, tile, mirrored axes and ranges."""
+    w = line.split()
+    k = w.index("order")
+    return (w[0], w[1], w[2], w[4], w[k + 1])   # (w[3]: the frame block)
+
+
+@pytest.mark.parametrize("shift", [0.0, 1e-3])
+@pytest.mark.parametrize("nz,nx,ny,span", [(33, 9, 21, 2.0), (40, 32, 32, 2.0), (17, 5, 11, 20.0), (18, 9, 6, 30.0),
+                                           (6, 17, 33, 3.0)])
+@pytest.mark.parametrize("kernel", [L.KERNEL_AUTO, L.KERNEL_FUSED_TMEM, L.KERNEL_FUSED_REGS])
+def test_chunks_of_a_host_buffer_call_sum_as_the_whole_call(host, shift, nz, nx, ny, span, kernel):
+    """Each chunk, a last one of one frame too, runs the kernel, weights, tile
+    and ranges of the call on device buffers."""
+    g = host.geometry(*acquisition(nz, nx, ny, span, shift=shift))
+    for n_frame, chunk in FRAMES_CHUNKS:
+        for store, compound in ((F32, True), (F16, True), (BF16, False)):
+            a = host.args(g, n_frame, 180, storage=store, compound=compound, kernel=kernel)
+            host.log()
+            status = host.beamform(g, a)
+            whole = host.log()
+            assert host.beamform_host(g, a, chunk) == status, (n_frame, chunk, store)
+            chunks = host.log()
+            if status == 0 and not whole[0].startswith("tc"):
+                assert {_sums(c) for c in chunks} == {_sums(whole[0])}, (n_frame, chunk, store, compound)
