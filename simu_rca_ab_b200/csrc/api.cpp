@@ -320,35 +320,54 @@ int plan_beamform(rcabf_geometry *g, const rcabf_beamform_args *a, Plan &p, cons
         } else if (follow) {
             vts = like->ts;
         }
-        // 16-frame blocks of the tensor-memory kernel take about 0.9 of the
-        // streaming kernel's time a frame (mirrored or not: 0.78 to 0.97 on 12
-        // acquisitions of 13 to 106 frames) when they are full: where the
-        // frames fill 0.84 of them
-        const int64_t b16 = (a->n_frame + 15) / 16 * 16;
-        const bool full16 = !named && !force && shift <= 2 && fb_req == 0 && a->n_frame >= 15 &&
-                            100 * a->n_frame >= 84 * b16;
-        if (!force && !named && !follow) {
-            // on coarse grids a tile 16 deep spans long windows of which each
-            // voxel uses a few rows: a flatter shape where the time of a step,
-            // about 150 + window rows, times the tiles' padding of the grid
-            // falls by a tenth or more (16 frames, 170 -> 60 rows: 30.3 -> 18.8
-            // ms; 18 frames, 113 -> 32 rows: 12.6 -> 9.4 ms)
+        // on coarse grids a tile 16 deep spans long windows of which each
+        // voxel uses a few rows: a flatter shape where the time of a step,
+        // about 150 + window rows, times the tiles' padding of the grid
+        // falls by a tenth or more (16 frames, 170 -> 60 rows: 30.3 -> 18.8
+        // ms; 18 frames, 113 -> 32 rows: 12.6 -> 9.4 ms)
+        auto choose_tile = [&](bool full) {
             float sz, su, sv;
             g->index_steps(sz, su, sv);
-            const int64_t nu = !full16 && (g->mirror & VBS_MIRROR_U) ? (g->n_u + 1) / 2 : g->n_u;
-            const int64_t nv = !full16 && (g->mirror & VBS_MIRROR_V) ? (g->n_v + 1) / 2 : g->n_v;
+            const int64_t nu = !full && (g->mirror & VBS_MIRROR_U) ? (g->n_u + 1) / 2 : g->n_u;
+            const int64_t nv = !full && (g->mirror & VBS_MIRROR_V) ? (g->n_v + 1) / 2 : g->n_v;
             auto padded = [](int64_t n, int64_t t) { return (double)((n + t - 1) / t * t); };
             auto cost = [&](const TileShape &t) {
                 const double rows = sz * (t.tz - 1) + su * (t.tu - 1) + sv * (t.tv * VB_BLOCK - 1) + kind_taps(g->kind) + 3;
                 return (150.0 + rows) * padded(g->n_z, t.tz) * padded(nu, t.tu) * padded(nv, t.tv * VB_BLOCK);
             };
-            TileShape best = vts;
-            double least = (full16 ? 0.75 : 0.9) * cost(vts);
+            TileShape best{tu, tvb, VB_THREADS_HOST / (tu * tvb)};
+            double least = (full ? 0.75 : 0.9) * cost(best);
             for (const TileShape &t : {TileShape{4, 4, 8}, TileShape{8, 4, 4}, TileShape{8, 8, 2}})
                 if (cost(t) < least) { least = cost(t); best = t; }
-            vts = best;
+            return best;
+        };
+        auto tile_rows = [&](const TileShape &t) { return g->window_rows(TileShape{t.tu, t.tv * VB_BLOCK, t.tz}); };
+        // staged rows: the largest window of `rows` and the shift rows
+        auto staged = [&](int rows, int d) {
+            const int ds = d >= 3 ? d - 2 : d;
+            return (int)std::min<int64_t>(rows + std::max(ds, 1), a->n_sample + ds);
+        };
+        auto fits_tmem = [&](int need, int fb) {
+            return need <= std::min<int>((int)(VB_SMEM_BUDGET / ((size_t)fused_stages(p.store) * fused_row_words(fb) * 4)),
+                                         vb_stage_rows_cap(p.store, fb));
+        };
+        // 16-frame blocks of the tensor-memory kernel take about 0.9 of the
+        // streaming kernel's time a frame (mirrored or not: 0.78 to 0.97 on 12
+        // acquisitions of 13 to 106 frames) when they are full: where the
+        // frames fill 0.84 of them, and a block of 16 holds the windows (where
+        // only its blocks of 8 or 4 do it is the slower kernel: 16 FP16 frames,
+        // 48 x 48 x 80 voxels 9.4 ms against 6.6)
+        const int64_t b16 = (a->n_frame + 15) / 16 * 16;
+        bool full16 = !named && !force && !follow && shift <= 2 && fb_req == 0 && a->n_frame >= 15 &&
+                      100 * a->n_frame >= 84 * b16;
+        if (!force && !named && !follow) {
+            vts = choose_tile(full16);
+            if (full16 && !fits_tmem(staged(tile_rows(vts), shift), 16)) {
+                full16 = false;
+                vts = choose_tile(false);
+            }
         }
-        const int rows = g->window_rows(TileShape{vts.tu, vts.tv * VB_BLOCK, vts.tz});
+        const int rows = tile_rows(vts);
         // streaming kernel: symmetric axes are mirrored where that drops about
         // half of the tiles (the grid fills the last ones)
         auto n_tiles = [](int64_t n, int64_t t) { return (n + t - 1) / t; };
@@ -377,16 +396,9 @@ int plan_beamform(rcabf_geometry *g, const rcabf_beamform_args *a, Plan &p, cons
                 split *= split_rx;
             }
         }
-        auto window = [&](int d) {   // staged rows: the largest window and the shift rows
-            const int ds = d >= 3 ? d - 2 : d;
-            return (int)std::min<int64_t>(rows + std::max(ds, 1), a->n_sample + ds);
-        };
         auto fits = [&](int vb, int d, int fb) {   // the largest window of the acquisition in its staging buffer
-            const int need = window(d);
-            if (vb == 1)
-                return a->n_sample <= VBS_MAX_SAMPLES && vbs_chunk_records(fb, need) >= 1;
-            return need <= std::min<int>((int)(VB_SMEM_BUDGET / ((size_t)fused_stages(p.store) * fused_row_words(fb) * 4)),
-                                         vb_stage_rows_cap(p.store, fb));
+            const int need = staged(rows, d);
+            return vb == 1 ? a->n_sample <= VBS_MAX_SAMPLES && vbs_chunk_records(fb, need) >= 1 : fits_tmem(need, fb);
         };
         auto pick = [&](int vb, int d) {   // the frame block, 0: none
             if (vb == 2 && (d == 0 || d >= 3)) return 0;
@@ -433,7 +445,7 @@ int plan_beamform(rcabf_geometry *g, const rcabf_beamform_args *a, Plan &p, cons
             p.d = d;
             p.fb = fb;
             p.ts = vts;
-            p.wmax = window(d);
+            p.wmax = staged(rows, d);
             if (vb == 1) {
                 // FP16 / BF16 single frames keep the weight accuracy of the
                 // one-voxel kernel that they ran on (degree 8)

@@ -107,3 +107,15 @@ def test_chunks_of_a_host_buffer_call_sum_as_the_whole_call(host, shift, nz, nx,
             chunks = host.log()
             if status == 0 and not whole[0].startswith("tc"):
                 assert {_sums(c) for c in chunks} == {_sums(whole[0])}, (n_frame, chunk, store, compound)
+
+
+@pytest.mark.parametrize("store", [F32, F16, BF16])
+@pytest.mark.parametrize("nz,nx,ny", [(33, 9, 21), (40, 32, 32), (80, 48, 48), (6, 17, 33)])
+@pytest.mark.parametrize("depth_mm", [3, 9, 20])
+def test_full_16_frame_counts_take_16_frame_blocks_or_the_streaming_kernel(host, store, nz, nx, ny, depth_mm):
+    """The tensor-memory kernel's blocks of 8 are slower than the streaming
+    kernel: no call of 15 frames or more falls to them."""
+    g = host.geometry(*acquisition(nz, nx, ny, 2.0, depth=(4e-3, depth_mm * 1e-3)))
+    for n_frame in (15, 16, 27, 31):
+        p = host.plan(g, host.args(g, n_frame, 700, storage=store))
+        assert (p["kernel"], p["frames_per_block"]) in (("fused_voxel_blocked_tmem", 16), ("fused_voxel_blocked", 8)), p
