@@ -358,8 +358,16 @@ int plan_beamform(rcabf_geometry *g, const rcabf_beamform_args *a, Plan &p, cons
         // only its blocks of 8 or 4 do it is the slower kernel: 16 FP16 frames,
         // 48 x 48 x 80 voxels 9.4 ms against 6.6)
         const int64_t b16 = (a->n_frame + 15) / 16 * 16;
-        bool full16 = !named && !force && !follow && shift <= 2 && fb_req == 0 && a->n_frame >= 15 &&
-                      100 * a->n_frame >= 84 * b16;
+        // (blocks asked for by size, of which 16 on the streaming kernel carry four
+        // mirrored copies of 4 frames: where all are full, voxels share one shift
+        // row, and the tiles fill the GPU twice without ranges of transmits.
+        // Mirrored grids, tensor memory against registers: 16 / 32 FP32 frames on
+        // 97 x 95 x 159 26.2 / 51.5 against 26.5 / 52.0 ms, 16 FP16 frames 24.2
+        // against 26.0; two shift rows, 64 x 64 x 128, 11.7 / 22.7 against 10.4 /
+        // 19.9; 27 frames 51.4 against 44.7; 16 on 61 x 63 x 40 4.4 against 3.6)
+        const bool many = (b16 / 16) * (g->n_z * g->n_u * g->n_v / (VB_THREADS_HOST * VB_BLOCK)) >= 2 * 148 * 4;
+        bool full16 = !named && !force && !follow && shift <= 2 && fb_req != 1 && a->n_frame >= 15 &&
+                      (fb_req == 0 ? 100 * a->n_frame >= 84 * b16 : shift == 1 && a->n_frame == b16 && many);
         if (!force && !named && !follow) {
             vts = choose_tile(full16);
             if (full16 && !fits_tmem(staged(tile_rows(vts), shift), 16)) {
@@ -372,7 +380,11 @@ int plan_beamform(rcabf_geometry *g, const rcabf_beamform_args *a, Plan &p, cons
         // half of the tiles (the grid fills the last ones)
         auto n_tiles = [](int64_t n, int64_t t) { return (n + t - 1) / t; };
         const int64_t tile_v = vts.tv * VB_BLOCK;
-        int mirror = named ? 0 : g->mirror;
+        // every frame block of a call sums in one order, whichever kernel holds
+        // it: where blocks of 16 are the tensor-memory kernel's, those asked for
+        // by size mirror and split nothing either
+        const bool plain = named || full16;
+        int mirror = plain ? 0 : g->mirror;
         if (5 * n_tiles((g->n_u + 1) / 2, vts.tu) > 3 * n_tiles(g->n_u, vts.tu)) mirror &= ~VBS_MIRROR_U;
         if (5 * n_tiles((g->n_v + 1) / 2, tile_v) > 3 * n_tiles(g->n_v, tile_v)) mirror &= ~VBS_MIRROR_V;
         if (follow) mirror = like->mirror;
@@ -384,7 +396,7 @@ int plan_beamform(rcabf_geometry *g, const rcabf_beamform_args *a, Plan &p, cons
         // of elements, to about two items per resident CTA.  The ranges set the
         // order of the sums: they do not depend on the frame block.
         int split = a->compound ? 1 : g->n_tx, split_rx = 1;
-        if (a->compound && !named) {
+        if (a->compound && !plain) {
             if (follow) {
                 split = like->n_split;
                 split_rx = like->split_rx;
@@ -436,7 +448,7 @@ int plan_beamform(rcabf_geometry *g, const rcabf_beamform_args *a, Plan &p, cons
             fb = pick(vb = want_vb, d);
             if (!fb && want_vb == 1 && a->n_sample > VBS_MAX_SAMPLES && d) fb = pick(vb = 2, d);   // the same bits
         } else {
-            if (full16) fb = pick(vb = 2, d);
+            if (full16 && (fb_req == 0 || fb_req == 16)) fb = pick(vb = 2, d);
             if (!fb) fb = pick(vb = 1, d);
             if (!fb) fb = pick(vb = 2, d);
         }

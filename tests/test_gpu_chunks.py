@@ -42,3 +42,29 @@ def test_chunked_host_call_gives_the_device_calls_bits(cuda, span, shift, storag
         eng.run_host(geom, eng.make_args(geom, iq_h, out=out_h, host=True, **kw), frames_per_chunk=chunk)
         torch.cuda.synchronize()
         assert torch.equal(out_h, ref), chunk
+
+
+@pytest.mark.parametrize("storage", ["float32", "float16"])
+@pytest.mark.parametrize("shift,shape", [(0.0, (72, 96, 96)), (1e-3, (72, 96, 96)), (0.0, (40, 32, 32))])
+@pytest.mark.parametrize("compound", [True, False])
+def test_frame_blocks_asked_for_give_one_result(cuda, storage, shift, shape, compound):
+    """Blocks of 2 to 16 frames, of which full ones of 16 run on the
+    tensor-memory kernel on a large grid."""
+    import torch
+    from simu_rca_ab_b200 import _lib as L
+    from simu_rca_ab_b200 import beamformer as B
+    from simu_rca_ab_b200.params import normalize
+    eng = B.default_engine()
+    with warnings.catch_warnings():
+        warnings.simplefilter("ignore")
+        geom = eng.geometry(normalize(np.zeros(1, np.complex64),
+                                      *acquisition(*shape, 2.0, shift=shift, n_ele=8, n_tx=3)))
+    g = torch.Generator(device="cuda").manual_seed(6)
+    iq = torch.randn(16, geom.n_tx, geom.n_ele, 180, dtype=torch.complex64, device="cuda", generator=g)
+    st = L.STORE_F32
+    if storage == "float16":
+        iq, st = iq.to(torch.complex32), L.STORE_F16
+    outs = [eng.beamform(geom, iq, storage=st, compound=compound, frames_per_block=fb)[0].clone() for fb in (2, 4, 8, 16)]
+    assert float(outs[0].abs().max()) > 0.0
+    for o in outs[1:]:
+        assert torch.equal(o, outs[0])

@@ -119,3 +119,28 @@ def test_full_16_frame_counts_take_16_frame_blocks_or_the_streaming_kernel(host,
     for n_frame in (15, 16, 27, 31):
         p = host.plan(g, host.args(g, n_frame, 700, storage=store))
         assert (p["kernel"], p["frames_per_block"]) in (("fused_voxel_blocked_tmem", 16), ("fused_voxel_blocked", 8)), p
+
+
+@pytest.mark.parametrize("shift", [0.0, 1e-3])
+@pytest.mark.parametrize("nz,nx,ny,depth_mm", [(33, 9, 21, 3), (40, 32, 32, 9), (96, 96, 96, 9), (6, 17, 33, 3)])
+@pytest.mark.parametrize("store,compound", [(F32, True), (F16, True), (F32, False)])
+def test_frame_blocks_asked_for(host, shift, nz, nx, ny, depth_mm, store, compound):
+    """frames_per_block = 16 runs on the tensor-memory kernel as the call that
+    leaves it open does, where its blocks are full, voxels share one shift row
+    and the tiles fill the GPU, and every block size of a call sums in one order."""
+    g = host.geometry(*acquisition(nz, nx, ny, 2.0, shift=shift, depth=(4e-3, depth_mm * 1e-3)))
+    for n_frame in (2, 8, 9, 15, 16, 18, 27, 32):
+        orders, kernel = set(), {}
+        for fb in (0, 2, 4, 8, 16):
+            host.log()
+            a = host.args(g, n_frame, 700, storage=store, compound=compound, fb=fb)
+            assert host.beamform(g, a) == 0
+            words = host.log()[0].split()
+            kernel[fb] = words[0], words[-1] if words[0] == "tc" else words[3]
+            if fb and words[0] != "fused":
+                order = words[words.index("order") + 1].split(",")
+                orders.add(tuple(order if compound else order[:-2]))   # (ranges only split compounded sums)
+        assert len(orders) == 1, (n_frame, orders)
+        d = host.plan(g, host.args(g, n_frame, 700, storage=store, compound=compound))["row_shift"]
+        if kernel[0] == ("vb", "16") and n_frame % 16 == 0 and d == 1 and nz * nx * ny > 512 * 1184:
+            assert kernel[16] == kernel[0], (n_frame, kernel)
