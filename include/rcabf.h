@@ -251,8 +251,9 @@ int rcabf_describe_plan(const rcabf_geometry *g, const rcabf_beamform_args *a, c
  * `stream`; no host synchronisation, no allocation. */
 int rcabf_beamform(const rcabf_geometry *g, const rcabf_beamform_args *a, void *stream);
 
-/* Beamforms n independent acquisitions in one persistent launch (all must
- * share interp, storage and frames_per_block). */
+/* Beamforms n independent acquisitions in one persistent launch per kernel
+ * function among their plans, one where they share it (all must share interp,
+ * storage and frames_per_block), each with the results it has alone. */
 int rcabf_beamform_batch(int n, const rcabf_geometry *const *g, const rcabf_beamform_args *a,
                          void *stream);
 

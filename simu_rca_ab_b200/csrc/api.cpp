@@ -690,7 +690,7 @@ int beamform_one(rcabf_geometry *g, const rcabf_beamform_args *a, cudaStream_t s
     return beamform_planned(g, a, p, st);
 }
 
-// One beamform call with a given plan (the autotuner's candidates).
+// One beamform call with a given plan.
 static int beamform_planned(rcabf_geometry *g, const rcabf_beamform_args *a, const Plan &p, cudaStream_t st)
 {
     int s;
@@ -755,6 +755,73 @@ static int beamform_planned(rcabf_geometry *g, const rcabf_beamform_args *a, con
     if ((s = finish_mask(g, a, st)) != RCABF_OK) return s;
     mark(a, 4, st);
     return RCABF_OK;
+}
+
+// One kernel function, launched with jobs of one slab height.
+static bool same_kernel(const Plan &a, const Plan &b)
+{
+    return a.kernel == b.kernel && a.ref == b.ref && a.fb == b.fb && a.vb == b.vb && a.d == b.d && a.deg == b.deg &&
+           a.tc == b.tc && a.tc_rows == b.tc_rows;
+}
+
+// n acquisitions with plans of their own on one mode, interpolation, storage
+// and device: one launch per kernel among the plans, each job computed as it is
+// alone.
+int beamform_batch_planned(int n, rcabf_geometry *const *gs, const rcabf_beamform_args *as, const Plan *plans,
+                           cudaStream_t st)
+{
+    int s;
+    for (int i = 0; i < n; ++i)
+        if ((s = check_ptrs(&as[i], plans[i])) != RCABF_OK) return s;
+    std::vector<char> done((size_t)n, 0);
+    for (int i = 0; i < n; ++i) {
+        if (done[i]) continue;
+        const Plan &p0 = plans[i];
+        if (p0.ref || p0.kernel != RCABF_KERNEL_FUSED) {
+            if ((s = beamform_planned(gs[i], &as[i], p0, st)) != RCABF_OK) return s;
+            continue;
+        }
+        FusedParams prm{};
+        int job[MAX_JOBS];
+        for (int k = i; k < n && prm.n_jobs < MAX_JOBS; ++k) {
+            if (done[k] || !same_kernel(p0, plans[k]) || prm.n_items + plans[k].n_items >= INT32_MAX) continue;
+            if ((s = stage_job(gs[k], &as[k], plans[k], prm.jobs[prm.n_jobs], st)) != RCABF_OK) return s;
+            prm.jobs[prm.n_jobs].item_begin = prm.n_items;
+            prm.n_items += plans[k].n_items;
+            prm.wmax = std::max(prm.wmax, plans[k].wmax);
+            done[k] = 1;
+            job[prm.n_jobs++] = k;
+        }
+        if (prm.n_jobs == 0) {   // (more items than a launch with others holds)
+            if ((s = beamform_planned(gs[i], &as[i], p0, st)) != RCABF_OK) return s;
+            continue;
+        }
+        prm.row_words = p0.row_words;
+        prm.counter = reinterpret_cast<uint32_t *>(static_cast<char *>(as[i].workspace) + p0.off_ctr);
+        if ((s = launch_fused_jobs(gs[i], prm, p0, st)) != RCABF_OK) return s;
+        for (int k = 0; k < prm.n_jobs; ++k) {
+            if ((s = finish_job(gs[job[k]], &as[job[k]], plans[job[k]], prm.jobs[k], st)) != RCABF_OK) return s;
+            if ((s = finish_mask(gs[job[k]], &as[job[k]], st)) != RCABF_OK) return s;
+        }
+    }
+    return RCABF_OK;
+}
+
+// Which calls one batch takes together: (frame block, accumulator store, row
+// shift) of the voxel-blocked kernel with tensor-memory accumulators or of the
+// one-voxel-per-thread kernel, whichever would run the call, not of the
+// streaming kernel, which takes calls of either and has more variants.
+static std::array<int, 3> batch_class(rcabf_geometry *g, const rcabf_beamform_args &a, const Plan &p)
+{
+    if (p.tc || a.kernel == RCABF_KERNEL_FUSED_TMEM || a.kernel == RCABF_KERNEL_FUSED_REGS)
+        return {p.fb, p.tc ? 0 : a.kernel == RCABF_KERNEL_FUSED_TMEM ? 2 : 1, p.d};
+    rcabf_beamform_args c = a;
+    Plan q;
+    c.kernel = RCABF_KERNEL_FUSED_TMEM;
+    if (a.kernel != RCABF_KERNEL_FUSED_NOBLOCK && plan_beamform(g, &c, q) == RCABF_OK) return {q.fb, 2, q.d};
+    c.kernel = RCABF_KERNEL_FUSED_NOBLOCK;
+    if (plan_beamform(g, &c, q) == RCABF_OK) return {q.fb, 0, 0};
+    return {p.fb, p.vb, p.d};
 }
 
 // Static workspace of rcabf_beamform_noalloc, per device: looked up once with
@@ -1167,51 +1234,26 @@ int rcabf_beamform_noalloc(const rcabf_geometry *g, const rcabf_beamform_args *a
 int rcabf_beamform_batch(int n, const rcabf_geometry *const *gs, const rcabf_beamform_args *as, void *stream)
 {
     if (n < 1 || n > MAX_JOBS || !gs || !as) return RCABF_ERR_INVALID_ARGUMENT;
-    cudaStream_t st = (cudaStream_t)stream;
-    rcabf_geometry *g0 = const_cast<rcabf_geometry *>(gs[0]);
-    if (!g0) return RCABF_ERR_BAD_HANDLE;
-    FusedParams prm{};
-    Plan p0;
+    rcabf_geometry *const *g = const_cast<rcabf_geometry *const *>(gs);
+    if (!g[0]) return RCABF_ERR_BAD_HANDLE;
     std::vector<Plan> plans((size_t)n);
-    int64_t items = 0;
-    int wmax = 0;
+    std::array<int, 3> first{};
     for (int i = 0; i < n; ++i) {
-        rcabf_geometry *g = const_cast<rcabf_geometry *>(gs[i]);
-        if (!g) return RCABF_ERR_BAD_HANDLE;
+        if (!g[i]) return RCABF_ERR_BAD_HANDLE;
         if (as[i].frames_per_block <= 0 || as[i].frames_per_block != as[0].frames_per_block)
             return RCABF_ERR_INVALID_ARGUMENT;
         if (as[i].kernel == RCABF_KERNEL_PLAIN) return RCABF_ERR_INVALID_ARGUMENT;
-        if (g->mode != g0->mode || g->kind != g0->kind || g->device != g0->device ||
+        if (g[i]->mode != g[0]->mode || g[i]->kind != g[0]->kind || g[i]->device != g[0]->device ||
             as[i].storage != as[0].storage)
             return RCABF_ERR_UNSUPPORTED;
-        Plan p;
-        int s = plan_beamform(g, &as[i], p);
+        const int s = plan_beamform(g[i], &as[i], plans[i]);
         if (s != RCABF_OK) return s;
-        if ((s = check_ptrs(&as[i], p)) != RCABF_OK) return s;
-        if (i == 0) p0 = p;
-        plans[i] = p;
-        // one launch = one kernel variant: every job fused, same frame block
-        if (p.kernel != RCABF_KERNEL_FUSED || p.fb != p0.fb || p.vb != p0.vb || p.d != p0.d ||
-            p.deg != p0.deg)
-            return RCABF_ERR_UNSUPPORTED;
-        wmax = std::max(wmax, p.wmax);
-        if ((s = stage_job(g, &as[i], p, prm.jobs[i], st)) != RCABF_OK) return s;
-        prm.jobs[i].item_begin = items;
-        items += p.n_items;
+        if (plans[i].kernel != RCABF_KERNEL_FUSED) return RCABF_ERR_UNSUPPORTED;
+        const std::array<int, 3> c = batch_class(g[i], as[i], plans[i]);
+        if (i == 0) first = c;
+        else if (c != first) return RCABF_ERR_UNSUPPORTED;
     }
-    if (p0.vb == 1 && items >= INT32_MAX) return RCABF_ERR_UNSUPPORTED;
-    prm.n_jobs = n;
-    prm.wmax = wmax;
-    prm.row_words = p0.row_words;
-    prm.n_items = items;
-    prm.counter = reinterpret_cast<uint32_t *>(static_cast<char *>(as[0].workspace) + p0.off_ctr);
-    int s = launch_fused_jobs(g0, prm, p0, st);
-    if (s != RCABF_OK) return s;
-    for (int i = 0; i < n; ++i) {
-        if ((s = finish_job(gs[i], &as[i], plans[i], prm.jobs[i], st)) != RCABF_OK) return s;
-        if ((s = finish_mask(gs[i], &as[i], st)) != RCABF_OK) return s;
-    }
-    return RCABF_OK;
+    return beamform_batch_planned(n, g, as, plans.data(), (cudaStream_t)stream);
 }
 
 int rcabf_autotune(const rcabf_geometry *gc, const rcabf_beamform_args *a, void *stream, int iters,

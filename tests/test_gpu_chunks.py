@@ -68,3 +68,36 @@ def test_frame_blocks_asked_for_give_one_result(cuda, storage, shift, shape, com
     assert float(outs[0].abs().max()) > 0.0
     for o in outs[1:]:
         assert torch.equal(o, outs[0])
+
+
+@pytest.mark.parametrize("fb,which", [(1, (0, 1, 2, 3, 4, 5)), (4, (0, 1)), (4, (2, 3, 4, 5)), (16, (2, 3, 4, 5))])
+def test_batch_of_mixed_grids_gives_the_bits_of_each_alone(cuda, fb, which):
+    """Mirrored and unmirrored grids, steering spreads that share rows, pairs or
+    none, points: one batch, several kernels."""
+    import torch
+    from simu_rca_ab_b200 import _lib as L
+    from simu_rca_ab_b200 import beamformer as B
+    from simu_rca_ab_b200.params import normalize
+    eng = B.default_engine()
+    kws = [dict(span=2.0), dict(span=2.0, shift=1e-3), dict(span=20.0), dict(span=30.0), dict(span=30.0, shift=1e-3),
+           dict(span=2.0, points=True)]
+    g = torch.Generator(device="cuda").manual_seed(7)
+    geoms, args, wss, outs, refs, iqs = [], [], [], [], [], []
+    for k in which:
+        kw = dict(kws[k])
+        with warnings.catch_warnings():
+            warnings.simplefilter("ignore")
+            geom = eng.geometry(normalize(np.zeros(1, np.complex64), *acquisition(33, 9, 12, kw.pop("span"), **kw)))
+        iq = torch.randn(3, geom.n_tx, geom.n_ele, 180, dtype=torch.complex64, device="cuda", generator=g)
+        refs.append(eng.beamform(geom, iq, frames_per_block=fb)[0].clone())
+        outs.append(torch.full_like(refs[-1], float("nan")))
+        a = eng.make_args(geom, iq, iq_dtype=L.IQ_C64, n_sample=180, n_frame=3, out=outs[-1], mask=None, compound=True,
+                          frames_per_block=fb)
+        wss.append(torch.empty(max(256, eng.workspace_bytes(geom, a)), dtype=torch.uint8, device="cuda"))
+        geoms.append(geom)
+        args.append(a)
+        iqs.append(iq)
+    eng.run_batch(geoms, args, wss)
+    torch.cuda.synchronize()
+    for o, r in zip(outs, refs):
+        assert torch.equal(o, r) and float(r.abs().max()) > 0.0

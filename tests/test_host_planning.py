@@ -144,3 +144,49 @@ def test_frame_blocks_asked_for(host, shift, nz, nx, ny, depth_mm, store, compou
         d = host.plan(g, host.args(g, n_frame, 700, storage=store, compound=compound))["row_shift"]
         if kernel[0] == ("vb", "16") and n_frame % 16 == 0 and d == 1 and nz * nx * ny > 512 * 1184:
             assert kernel[16] == kernel[0], (n_frame, kernel)
+
+
+# (mirrored grids and others, steps of every steepness, points, one row)
+BATCH = [dict(), dict(shift=1e-3), dict(span=20.0), dict(span=30.0), dict(span=30.0, shift=1e-3), dict(points=True),
+         dict(ny=1), dict(nz=96, nx=96, ny=72)]
+
+
+def _batch_geometry(host, kw):
+    kw = {"nz": 33, "nx": 9, "ny": 12, "span": 2.0, **kw}
+    return host.geometry(*acquisition(kw.pop("nz"), kw.pop("nx"), kw.pop("ny"), kw.pop("span"), **kw))
+
+
+@pytest.mark.parametrize("fb,accepted", [
+    (1, [set(range(len(BATCH)))]),                  # one voxel per thread, or the streaming kernel
+    (4, [{0, 1, 7}, {2, 3, 4, 5, 6}]),              # shared rows; wider spreads and grids without a block
+    (16, [{0, 1, 7}, {2, 3, 4, 5, 6}])])
+def test_batches_take_mirrored_steep_and_other_grids_together(host, fb, accepted):
+    """One batch of two or of all grids of a class, each job with the kernel and
+    order of sums that it has alone; grids of different classes are refused."""
+    gs = [_batch_geometry(host, kw) for kw in BATCH]
+    args = [host.args(g, 16 if fb == 16 else 3, 180, fb=fb) for g in gs]
+    alone = []
+    for g, a in zip(gs, args):
+        host.log()
+        assert host.beamform(g, a) == 0
+        alone.append(host.log()[0].split(" jobs")[0])
+    for i in range(len(gs)):
+        for k in range(len(gs)):
+            ok = any({i, k} <= c for c in accepted)
+            host.log()
+            assert host.batch([gs[i], gs[k]], [args[i], args[k]]) == (0 if ok else L.ERR_UNSUPPORTED), (i, k)
+            if ok:
+                want = {alone[i], alone[k]}
+                assert sorted(line.split(" jobs")[0] for line in host.log()) == sorted(want), (i, k)
+    for c in accepted:
+        host.log()
+        assert host.batch([gs[i] for i in sorted(c)], [args[i] for i in sorted(c)]) == 0
+        assert len(host.log()) == len({alone[i] for i in c})
+
+
+def test_batch_of_tensor_core_calls_keeps_each_record_length(host):
+    """Jobs with records of two lengths have slabs of two heights: a launch each."""
+    g = _batch_geometry(host, {})
+    args = [host.args(g, 40, ns, storage=F16, kernel=L.KERNEL_FUSED_TC, fb=40) for ns in (180, 180, 300)]
+    assert host.batch([g] * 3, args) == 0
+    assert [line.split("rows ")[1] for line in host.log()] == ["212 of 180", "212 of 180", "332 of 300"]
