@@ -757,16 +757,13 @@ static int beamform_planned(rcabf_geometry *g, const rcabf_beamform_args *a, con
     return RCABF_OK;
 }
 
-// One kernel function, launched with jobs of one slab height.
-static bool same_kernel(const Plan &a, const Plan &b)
+bool same_kernel(const Plan &a, const Plan &b)
 {
     return a.kernel == b.kernel && a.ref == b.ref && a.fb == b.fb && a.vb == b.vb && a.d == b.d && a.deg == b.deg &&
            a.tc == b.tc && a.tc_rows == b.tc_rows;
 }
 
-// n acquisitions with plans of their own on one mode, interpolation, storage
-// and device: one launch per kernel among the plans, each job computed as it is
-// alone.
+// (each job is computed as it is alone)
 int beamform_batch_planned(int n, rcabf_geometry *const *gs, const rcabf_beamform_args *as, const Plan *plans,
                            cudaStream_t st)
 {

@@ -49,6 +49,14 @@ struct Plan {
 int plan_beamform(rcabf_geometry *g, const rcabf_beamform_args *a, Plan &p, const TuneChoice *force = nullptr,
                   const Plan *like = nullptr);
 
+// One kernel function, and slabs of one height: jobs that one launch can take.
+bool same_kernel(const Plan &a, const Plan &b);
+
+// n acquisitions with the plans plan_beamform gave them, on one mode,
+// interpolation, storage and device: one launch per kernel among the plans.
+int beamform_batch_planned(int n, rcabf_geometry *const *gs, const rcabf_beamform_args *as, const Plan *plans,
+                           cudaStream_t st);
+
 // Smaller-workspace replacement of a streaming-kernel plan (api.cpp).
 void plan_compact(rcabf_geometry *g, rcabf_beamform_args &a, Plan &p);
 

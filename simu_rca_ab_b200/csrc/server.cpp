@@ -9,10 +9,11 @@
 //   theirs.
 // * A scheduler thread admits queued requests in arrival order as launch
 //   slots (streams) and arena space free up.  Requests whose launch plans
-//   share one kernel variant (same table mode, interpolation, storage, frame
-//   block and voxel blocking) are fused into one persistent launch
-//   (rcabf_beamform_batch), so requests that arrive while others run are
-//   picked up by the next launch and their work overlaps on the device.
+//   share one kernel function (same table mode, interpolation, storage, frame
+//   block, voxel blocking and row sharing) are fused into one persistent launch
+//   (beamform_batch_planned), each with the plan it has alone, so requests that
+//   arrive while others run are picked up by the next launch and their work
+//   overlaps on the device.
 // * Completion is signalled by a host function enqueued behind each launch;
 //   it releases the workspace and the slot and records the request's latency
 //   (submit to completion, host clock).
@@ -99,13 +100,12 @@ struct Request {
     uint64_t ticket = 0;
     rcabf_geometry *g = nullptr;
     rcabf_beamform_args a{};
-    Plan plan;
+    Plan plan;                // made at submit; what the request runs, alone or fused
     size_t ws_off = 0, ws_bytes = 0;
     double units = 0.0;
     Clock::time_point t_submit;
     int status = RCABF_ERR_PENDING;
     bool done = false;
-    bool batchable = false;   // runs as one job of a fused multi-request launch
 };
 
 struct Launch;
@@ -149,13 +149,12 @@ struct Launch {
     std::vector<Request *> reqs;
 };
 
-// Requests fused into one launch must run one kernel variant.
+// Requests fused into one launch must run one kernel (few-frame requests on
+// reference tables: one launch slot, a kernel each).
 static bool same_variant(const Request *a, const Request *b)
 {
-    return a->batchable && b->batchable && a->g->device == b->g->device && a->g->mode == b->g->mode && a->g->kind == b->g->kind &&
-           a->a.storage == b->a.storage && a->plan.kernel == RCABF_KERNEL_FUSED &&
-           b->plan.kernel == RCABF_KERNEL_FUSED && a->plan.fb == b->plan.fb && a->plan.vb == b->plan.vb &&
-           a->plan.d == b->plan.d && a->plan.tc == b->plan.tc && a->plan.deg == b->plan.deg;
+    return a->g->device == b->g->device && a->g->mode == b->g->mode && a->g->kind == b->g->kind &&
+           a->a.storage == b->a.storage && a->plan.kernel == RCABF_KERNEL_FUSED && same_kernel(a->plan, b->plan);
 }
 
 static void finish_locked(rcabf_server *s, Request *r, int status, Clock::time_point now)
@@ -249,18 +248,16 @@ static bool dispatch_locked(rcabf_server *s)
             r->a.stage_events = nullptr;
         }
         cudaStream_t st = s->streams[slot];
-        int status;
-        if (L->reqs.size() == 1) {
-            status = rcabf_beamform(L->reqs[0]->g, &L->reqs[0]->a, st);
-        } else {
-            std::vector<const rcabf_geometry *> gs;
-            std::vector<rcabf_beamform_args> as;
-            for (Request *r : L->reqs) {
-                gs.push_back(r->g);
-                as.push_back(r->a);
-            }
-            status = rcabf_beamform_batch((int)gs.size(), gs.data(), as.data(), st);
+        // every request runs the plan it was admitted with, alone or fused
+        std::vector<rcabf_geometry *> gs;
+        std::vector<rcabf_beamform_args> as;
+        std::vector<Plan> plans;
+        for (Request *r : L->reqs) {
+            gs.push_back(r->g);
+            as.push_back(r->a);
+            plans.push_back(r->plan);
         }
+        int status = beamform_batch_planned((int)gs.size(), gs.data(), as.data(), plans.data(), st);
         if (status == RCABF_OK) status = cudaLaunchHostFunc(st, on_launch_done, L) == cudaSuccess ? RCABF_OK
                                                                                                   : RCABF_ERR_CUDA;
         if (status != RCABF_OK) {
@@ -371,22 +368,6 @@ int rcabf_server_submit(rcabf_server *s, const rcabf_geometry *g, const rcabf_be
     if (st == RCABF_OK && (r->plan.vb == 1 || r->plan.ref) && Arena::round(r->plan.total) > s->arena.size())
         plan_compact(gg, r->a, r->plan);
     if (st == RCABF_OK && (!r->a.iq || !r->a.out)) st = RCABF_ERR_INVALID_ARGUMENT;
-    if (st == RCABF_OK && r->plan.kernel == RCABF_KERNEL_FUSED && !r->plan.ref && r->a.frames_per_block == 0) {
-        // pin the frame block the planner chose, so the request runs the same
-        // kernel variant alone or fused with others; a request whose plan
-        // would change under the pin is never fused
-        rcabf_beamform_args pinned = r->a;
-        pinned.frames_per_block = r->plan.fb;
-        Plan p2;
-        if (plan_beamform(gg, &pinned, p2) == RCABF_OK && p2.vb == r->plan.vb && p2.d == r->plan.d &&
-            p2.tc == r->plan.tc && p2.fb == r->plan.fb && p2.total == r->plan.total &&
-            p2.deg == r->plan.deg) {
-            r->a = pinned;
-            r->batchable = true;
-        }
-    } else if (st == RCABF_OK && r->plan.kernel == RCABF_KERNEL_FUSED && !r->plan.ref) {
-        r->batchable = true;
-    }
     std::lock_guard<std::mutex> lk(s->mu);
     if (st == RCABF_OK && Arena::round(r->plan.total) > s->arena.size()) st = RCABF_ERR_OOM_ADMISSION;
     if (st == RCABF_OK && s->stop) st = RCABF_ERR_CANCELLED;

@@ -101,3 +101,39 @@ def test_batch_of_mixed_grids_gives_the_bits_of_each_alone(cuda, fb, which):
     torch.cuda.synchronize()
     for o, r in zip(outs, refs):
         assert torch.equal(o, r) and float(r.abs().max()) > 0.0
+
+
+@pytest.mark.parametrize("n_frame,storage,tables,shift", [
+    (16, "float32", "exact", 0.0), (16, "float32", "exact", 1e-3), (1, "float16", "exact", 0.0),
+    (5, "float16", "exact", 1e-3), (2, "float32", "ref_compat", 0.0)])
+def test_served_requests_share_a_launch_and_give_the_bits_of_each_alone(cuda, n_frame, storage, tables, shift):
+    import torch
+    from simu_rca_ab_b200 import _lib as L
+    from simu_rca_ab_b200 import beamformer as B
+    from simu_rca_ab_b200.params import normalize
+    from simu_rca_ab_b200.server import Server
+    eng = B.default_engine()
+    half = storage == "float16"
+    with warnings.catch_warnings():
+        warnings.simplefilter("ignore")
+        geom = eng.geometry(normalize(np.zeros(1, np.complex64), *acquisition(
+            40, 32, 32, 2.0, shift=shift, tables=tables, interp=("ref6", 3) if tables == "ref_compat" else ("lanczos", 4))))
+    g = torch.Generator(device="cuda").manual_seed(8)
+    kw = dict(iq_dtype=L.IQ_C32 if half else L.IQ_C64, n_sample=180, n_frame=n_frame,
+              storage=L.STORE_F16 if half else L.STORE_F32)
+    iqs = [torch.randn(n_frame, geom.n_tx, geom.n_ele, 180, dtype=torch.complex64, device="cuda", generator=g)
+           for _ in range(3)]
+    iqs = [q.to(torch.complex32) for q in iqs] if half else iqs
+    refs = []
+    for q in iqs:
+        refs.append(torch.empty((n_frame, 1, geom.n_pix), dtype=torch.complex64, device="cuda"))
+        eng.run(geom, eng.make_args(geom, q, out=refs[-1], mask=None, compound=True, **kw))
+    torch.cuda.synchronize()
+    outs = [torch.full_like(r, float("nan")) for r in refs]
+    torch.cuda.synchronize()
+    with Server(eng, 1 << 30, n_streams=2, batch_window_us=200_000) as srv:
+        for t in [srv.submit_beamform(geom, q, o, **kw) for q, o in zip(iqs, outs)]:
+            assert srv.wait(t, 60.0) == 0
+        assert srv.stats().launches == 1
+    for o, r in zip(outs, refs):
+        assert torch.equal(o, r) and float(r.abs().max()) > 0.0

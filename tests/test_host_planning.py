@@ -190,3 +190,35 @@ def test_batch_of_tensor_core_calls_keeps_each_record_length(host):
     args = [host.args(g, 40, ns, storage=F16, kernel=L.KERNEL_FUSED_TC, fb=40) for ns in (180, 180, 300)]
     assert host.batch([g] * 3, args) == 0
     assert [line.split("rows ")[1] for line in host.log()] == ["212 of 180", "212 of 180", "332 of 300"]
+
+
+SERVED = [(dict(), 16, F32), (dict(shift=1e-3), 16, F32), (dict(), 31, F32), (dict(), 1, F16), (dict(shift=1e-3), 1, BF16),
+          (dict(), 1, F32), (dict(shift=1e-3), 5, F16), (dict(span=30.0), 3, F32), (dict(), 40, F16),
+          (dict(tables="ref_compat", interp=("ref6", 3)), 1, F32), (dict(tables="ref_compat", interp=("ref6", 3)), 4, F32),
+          (dict(tables="ref_compat", interp=("ref6", 3)), 6, F32), (dict(points=True), 2, F32)]
+
+
+@pytest.mark.parametrize("kw,n_frame,store", SERVED)
+def test_server_runs_equal_requests_in_one_launch_with_the_plan_each_has_alone(host, kw, n_frame, store):
+    import ctypes as C
+    g = _batch_geometry(host, kw)
+    assert host.beamform(g, host.args(g, n_frame, 180, storage=store)) == 0
+    alone = host.log()
+    cfg, srv = L.ServerConfig(), C.c_void_p()
+    cfg.struct_size, cfg.hbm_budget_bytes = C.sizeof(cfg), 1 << 28
+    cfg.n_streams, cfg.max_queue, cfg.max_batch, cfg.batch_window_us = 1, 16, 8, 50_000
+    assert host.lib.rcabf_server_create(C.byref(cfg), C.byref(srv)) == 0
+    tickets = []
+    for k in range(3):
+        a, t = host.args(g, n_frame, 180, storage=store), C.c_uint64()
+        a.out = (k + 2) << 20        # outputs of their own: requests on one output wait for each other
+        assert host.lib.rcabf_server_submit(srv, g, C.byref(a), C.byref(t)) == 0
+        tickets.append(t)
+    st = C.c_int()
+    for t in tickets:
+        assert host.lib.rcabf_server_wait_for(srv, t, 20.0, C.byref(st)) == 0 and st.value == 0
+    stats = L.ServerStats()
+    stats.struct_size = C.sizeof(stats)
+    assert host.lib.rcabf_server_get_stats(srv, C.byref(stats)) == 0 and stats.launches == 1
+    assert host.lib.rcabf_server_destroy(srv) == 0
+    assert {line.split(" jobs")[0] for line in host.log()} == {line.split(" jobs")[0] for line in alone}
