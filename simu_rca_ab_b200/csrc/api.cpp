@@ -502,23 +502,29 @@ int plan_beamform(rcabf_geometry *g, const rcabf_beamform_args *a, Plan &p, cons
     return RCABF_OK;
 }
 
-// Replaces the planner's own choice of the streaming kernel by one with a
-// smaller workspace, where there is one: slabs in the storage type, staged by
-// the voxel-blocked kernel with tensor-memory accumulators or by the
-// one-voxel-per-thread kernel.  Sets a.kernel to it.
-void plan_compact(rcabf_geometry *g, rcabf_beamform_args &a, Plan &p)
+// Replaces a plan of the streaming kernel, or of the per-transmit kernel on
+// reference tables, by one of at most `limit` scratch bytes, where there is one:
+// slabs in the storage type, staged by the voxel-blocked kernel with
+// tensor-memory accumulators (for the register kernel by name too: the same
+// bits), in the planner's frame blocks or smaller ones, or else by the
+// one-voxel-per-thread kernel.
+void plan_compact(rcabf_geometry *g, const rcabf_beamform_args &a, size_t limit, Plan &p)
 {
-    if (a.kernel != RCABF_KERNEL_AUTO && a.kernel != RCABF_KERNEL_FUSED) return;
+    if (a.kernel != RCABF_KERNEL_AUTO && a.kernel != RCABF_KERNEL_FUSED && a.kernel != RCABF_KERNEL_FUSED_REGS) return;
     rcabf_beamform_args c = a;
-    for (int32_t k : {RCABF_KERNEL_FUSED_TMEM, RCABF_KERNEL_FUSED_NOBLOCK}) {
+    auto take = [&](int32_t kernel, int fb) {
         Plan q;
-        c.kernel = k;
-        if (plan_beamform(g, &c, q) == RCABF_OK && q.kernel == RCABF_KERNEL_FUSED && (p.ref || q.total < p.total)) {
-            p = q;
-            a.kernel = k;
-            return;
-        }
+        c.kernel = kernel;
+        c.frames_per_block = fb;
+        if (plan_beamform(g, &c, q) != RCABF_OK || q.kernel != RCABF_KERNEL_FUSED || q.total > limit) return false;
+        p = q;
+        return true;
+    };
+    for (int fb : {16, 8, 4, 2}) {
+        if (a.frames_per_block ? fb != a.frames_per_block : fb > pow2_ceil(a.n_frame)) continue;
+        if (take(RCABF_KERNEL_FUSED_TMEM, fb)) return;
     }
+    if (a.kernel != RCABF_KERNEL_FUSED_REGS) take(RCABF_KERNEL_FUSED_NOBLOCK, a.frames_per_block);
 }
 
 static void mark(const rcabf_beamform_args *a, int i, cudaStream_t st)
@@ -868,10 +874,13 @@ int beamform_noalloc(rcabf_geometry *g, const rcabf_beamform_args *a, cudaStream
     // the streaming kernel's FP32 slabs are up to three times the channel
     // data in storage type: where they do not fit, the kernels that stage it
     rcabf_beamform_args b = *a;
-    if (p.ref || (p.vb == 1 && p.total > RCABF_NOALLOC_WORKSPACE_BYTES)) plan_compact(g, b, p);
+    if (p.ref || (p.vb == 1 && p.total > RCABF_NOALLOC_WORKSPACE_BYTES))
+        plan_compact(g, b, RCABF_NOALLOC_WORKSPACE_BYTES, p);
     if (p.ref) {
-        snprintf(g_last_err, sizeof(g_last_err), "noalloc: no fused plan for these reference tables");
-        return RCABF_ERR_UNSUPPORTED;
+        snprintf(g_last_err, sizeof(g_last_err),
+                 "noalloc: no fused plan for these reference tables in the static workspace's %zu bytes",
+                 (size_t)RCABF_NOALLOC_WORKSPACE_BYTES);
+        return RCABF_ERR_WORKSPACE_TOO_SMALL;
     }
     if (p.total > RCABF_NOALLOC_WORKSPACE_BYTES) {
         snprintf(g_last_err, sizeof(g_last_err),

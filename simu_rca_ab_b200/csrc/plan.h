@@ -57,8 +57,9 @@ bool same_kernel(const Plan &a, const Plan &b);
 int beamform_batch_planned(int n, rcabf_geometry *const *gs, const rcabf_beamform_args *as, const Plan *plans,
                            cudaStream_t st);
 
-// Smaller-workspace replacement of a streaming-kernel plan (api.cpp).
-void plan_compact(rcabf_geometry *g, rcabf_beamform_args &a, Plan &p);
+// Replacement of a streaming-kernel or per-transmit plan within `limit` scratch
+// bytes, where there is one (api.cpp).
+void plan_compact(rcabf_geometry *g, const rcabf_beamform_args &a, size_t limit, Plan &p);
 
 // Frame-block sizes with a compiled fused-kernel variant.
 bool fb_supported(int mode, int fb);

@@ -366,7 +366,7 @@ int rcabf_server_submit(rcabf_server *s, const rcabf_geometry *g, const rcabf_be
     int st = plan_beamform(gg, &r->a, r->plan);
     // a request whose FP32 slabs exceed the whole arena runs on storage-type slabs
     if (st == RCABF_OK && (r->plan.vb == 1 || r->plan.ref) && Arena::round(r->plan.total) > s->arena.size())
-        plan_compact(gg, r->a, r->plan);
+        plan_compact(gg, r->a, s->arena.size(), r->plan);
     if (st == RCABF_OK && (!r->a.iq || !r->a.out)) st = RCABF_ERR_INVALID_ARGUMENT;
     std::lock_guard<std::mutex> lk(s->mu);
     if (st == RCABF_OK && Arena::round(r->plan.total) > s->arena.size()) st = RCABF_ERR_OOM_ADMISSION;

@@ -222,3 +222,35 @@ def test_server_runs_equal_requests_in_one_launch_with_the_plan_each_has_alone(h
     assert host.lib.rcabf_server_get_stats(srv, C.byref(stats)) == 0 and stats.launches == 1
     assert host.lib.rcabf_server_destroy(srv) == 0
     assert {line.split(" jobs")[0] for line in host.log()} == {line.split(" jobs")[0] for line in alone}
+
+
+@pytest.mark.parametrize("kw", [dict(), dict(shift=1e-3), dict(span=20.0), dict(tables="ref_compat", interp=("ref6", 3))])
+@pytest.mark.parametrize("kernel", [L.KERNEL_AUTO, L.KERNEL_FUSED_REGS])
+def test_calls_whose_storage_type_slabs_fit_run_in_the_static_workspace(host, kw, kernel):
+    """A plan with FP32 slabs, or with transmit sums, that exceeds the 64 MiB of
+    the call without allocation gives way to one that fits: the tensor-memory
+    kernel in the planner's frame blocks or smaller ones, or one voxel per thread."""
+    import ctypes as C
+    g = _batch_geometry(host, kw)
+    ref = "tables" in kw
+    if kernel == L.KERNEL_FUSED_REGS and (ref or "span" in kw):
+        return
+    limit, cut = 64 << 20, 0
+    for n_frame in (1, 2, 3, 4, 5, 8, 9, 12, 17, 24):
+        for store in (F32,) if ref else (F32, F16, BF16):
+            for mb in (20, 40, 60, 63):   # storage-type slabs of about mb MB: one frame block of each size
+                block = 1 << (n_frame - 1).bit_length()
+                ns = int(mb * 1e6 / (5 * 24 * (block if block <= 16 else 16 * -(-n_frame // 16)) * (8 if store == F32 else 4)))
+                fits = []
+                for k in (L.KERNEL_FUSED_TMEM,) + (() if kernel == L.KERNEL_FUSED_REGS else (L.KERNEL_FUSED_NOBLOCK,)):
+                    for fb in (min(block, 16), 0):
+                        a, n = host.args(g, n_frame, ns, storage=store, kernel=k, fb=fb), C.c_size_t()
+                        if host.lib.rcabf_beamform_workspace_size(g, C.byref(a), C.byref(n)) == 0:
+                            fits.append(n.value <= limit)
+                a = host.args(g, n_frame, ns, storage=store, kernel=kernel)
+                n = C.c_size_t()
+                if not any(fits) or host.lib.rcabf_beamform_workspace_size(g, C.byref(a), C.byref(n)) != 0:
+                    continue
+                assert host.lib.rcabf_beamform_noalloc(g, C.byref(a), None) == 0, (n_frame, store, mb)
+                cut += n.value > limit
+    assert cut > 0 or (ref and kernel == L.KERNEL_AUTO)
