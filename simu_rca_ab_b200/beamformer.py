@@ -247,14 +247,42 @@ class Engine:
         return ws
 
     def run(self, geom: GeometryHandle, a: L.BeamformArgs, stream=None, workspace=None) -> None:
-        """Launches one beamform (asynchronous on `stream`)."""
+        """Launches one beamform (asynchronous on `stream`).
+
+        The planner's own choice for few frames trades scratch memory for time
+        (FP32 slabs, transmit sums).  Where the device has no room for it, the
+        call runs on the kernels that stage the channel data in storage type."""
         sp = _stream_ptr(stream)
         need = self.workspace_bytes(geom, a)
-        ws = workspace if workspace is not None else self._workspace(need, sp)
+        try:
+            ws = workspace if workspace is not None else self._workspace(need, sp)
+        except torch.OutOfMemoryError:
+            return self._run_compact(geom, a, need, sp)
         a.workspace = ws.data_ptr() if need else None
         a.workspace_bytes = ws.numel() if need else 0
         with torch.cuda.device(self.device):
             L.check(L.lib().rcabf_beamform(C.c_void_p(geom.ptr), C.byref(a), C.c_void_p(sp)), "rcabf_beamform")
+
+    def _run_compact(self, geom: GeometryHandle, a: L.BeamformArgs, need: int, stream_ptr: int) -> None:
+        """run() on the first kernel and frame block whose smaller scratch can
+        be allocated: the planner's blocks and smaller ones of the tensor-memory
+        kernel, then one voxel per thread."""
+        kernel, fb = a.kernel, a.frames_per_block
+        block = max(2, 1 << (a.n_frame - 1).bit_length())
+        tries = [(L.KERNEL_FUSED_TMEM, b) for b in (16, 8, 4, 2) if (b == fb if fb else b <= block)]
+        tries.append((L.KERNEL_FUSED_NOBLOCK, fb))
+        try:
+            for a.kernel, a.frames_per_block in tries if kernel in (L.KERNEL_AUTO, L.KERNEL_FUSED) else ():
+                try:
+                    n = self.workspace_bytes(geom, a)
+                    ws = self._workspace(n, stream_ptr) if n < need else None
+                except (L.RcabfError, torch.OutOfMemoryError):
+                    continue
+                if ws is not None:
+                    return self.run(geom, a, stream=stream_ptr, workspace=ws)
+        finally:
+            a.kernel, a.frames_per_block = kernel, fb
+        raise torch.OutOfMemoryError(f"no device memory for {need} bytes of beamforming scratch")
 
     def run_host(self, geom: GeometryHandle, a: L.BeamformArgs, frames_per_chunk: int = 0, stream=None,
                  workspace=None) -> None:
