@@ -1346,8 +1346,10 @@ int rcabf_autotune(const rcabf_geometry *gc, const rcabf_beamform_args *a, void 
                 consider(TuneChoice{p0.vb, p0.fb, t});
             }
             const TileShape bt = best.ts;
+            // (a block of the streaming kernel holds the mirrored copies of its frames)
+            const int64_t held = a->n_frame * (p0.vb == 1 ? p0.n_sym : 1);
             for (int fb : {2, 4, 8, 16}) {
-                if (fb == p0.fb || fb > 2 * a->n_frame) continue;
+                if (fb == p0.fb || fb > 2 * held) continue;
                 consider(TuneChoice{p0.vb, fb, bt});
             }
             // the other accumulator store (registers / tensor memory) at every
@@ -1370,7 +1372,7 @@ int rcabf_autotune(const rcabf_geometry *gc, const rcabf_beamform_args *a, void 
         if (plan_beamform(g, &nb, pn) == RCABF_OK && pn.kernel == RCABF_KERNEL_FUSED) {
             for (int fb : {pn.fb, 40, 16}) {
                 if (!fb_supported(g->mode, fb) || (fb != pn.fb && fb > 2 * a->n_frame)) continue;
-                if (!p0.vb && fb == p0.fb) continue;   // the default itself
+                if (!p0.vb && !p0.tc && !p0.ref && fb == p0.fb) continue;   // the default itself
                 consider(TuneChoice{0, fb, pn.ts});
             }
         }

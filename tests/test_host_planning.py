@@ -254,3 +254,17 @@ def test_calls_whose_storage_type_slabs_fit_run_in_the_static_workspace(host, kw
                 assert host.lib.rcabf_beamform_noalloc(g, C.byref(a), None) == 0, (n_frame, store, mb)
                 cut += n.value > limit
     assert cut > 0 or (ref and kernel == L.KERNEL_AUTO)
+
+
+@pytest.mark.parametrize("kw,n_frame,want", [
+    (dict(tables="ref_compat", interp=("ref6", 3)), 1, {("fused", "1")}),
+    (dict(tables="ref_compat", interp=("ref6", 3)), 4, {("fused", "4")}),
+    (dict(ny=21), 1, {("vbs", "2"), ("vbs", "4"), ("vbs", "8")}), (dict(shift=1e-3), 2, {("vbs", "2"), ("vbs", "4")})])
+def test_autotuning_times_the_fused_kernel_and_blocks_of_mirrored_copies(host, kw, n_frame, want):
+    import ctypes as C
+    g = _batch_geometry(host, kw)
+    r = L.TuneResult()
+    r.struct_size = C.sizeof(r)
+    host.log()
+    assert host.lib.rcabf_autotune(g, C.byref(host.args(g, n_frame, 180)), None, 1, C.byref(r)) == 0
+    assert want <= {(line.split()[0], line.split()[3]) for line in host.log()}
