@@ -171,6 +171,20 @@ static void finish_locked(rcabf_server *s, Request *r, int status, Clock::time_p
     s->last_done = now;
 }
 
+// A launch leaves: its requests are done, its outputs and slot free.
+static void leave_locked(rcabf_server *s, Launch *L, int status)
+{
+    const auto now = Clock::now();
+    for (Request *r : L->reqs) {
+        s->busy_out.erase(s->busy_out.find(r->a.out));
+        if (r->a.mask) s->busy_out.erase(s->busy_out.find(r->a.mask));
+        finish_locked(s, r, status, now);
+    }
+    s->slot_busy[L->slot] = 0;
+    s->in_flight -= 1;
+    if (s->in_flight == 0) s->busy_s += std::chrono::duration<double>(now - s->busy_since).count();
+}
+
 // Host function run by CUDA when a launch's stream reaches it: no CUDA calls here.
 static void CUDART_CB on_launch_done(void *p)
 {
@@ -178,26 +192,19 @@ static void CUDART_CB on_launch_done(void *p)
     rcabf_server *s = L->srv;
     {
         std::lock_guard<std::mutex> lk(s->mu);
-        const auto now = Clock::now();
-        for (Request *r : L->reqs) {
-            finish_locked(s, r, RCABF_OK, now);
-            s->busy_out.erase(s->busy_out.find(r->a.out));
-            if (r->a.mask) s->busy_out.erase(s->busy_out.find(r->a.mask));
-        }
-        s->slot_busy[L->slot] = 0;
-        s->in_flight -= 1;
-        if (s->in_flight == 0) s->busy_s += std::chrono::duration<double>(now - s->busy_since).count();
+        leave_locked(s, L, RCABF_OK);
     }
     s->cv.notify_all();
     s->cv_done.notify_all();
     delete L;
 }
 
-// Admits queued requests while a slot and arena space are free; returns
-// whether anything was launched.  Called with the lock held.
-static bool dispatch_locked(rcabf_server *s)
+// Admits queued requests while a slot and arena space are free.  Called with
+// the lock held, which is released around the CUDA calls: the first launch of a
+// kernel may load its module and wait for the work in flight, whose completion
+// (on_launch_done) takes the lock.  Only the scheduler thread dispatches.
+static void dispatch(rcabf_server *s, std::unique_lock<std::mutex> &lk)
 {
-    bool any = false;
     while (!s->queue.empty()) {
         int slot = -1;
         for (int i = 0; i < (int)s->slot_busy.size(); ++i)
@@ -256,7 +263,15 @@ static bool dispatch_locked(rcabf_server *s)
             gs.push_back(r->g);
             as.push_back(r->a);
             plans.push_back(r->plan);
+            s->busy_out.insert(r->a.out);
+            if (r->a.mask) s->busy_out.insert(r->a.mask);
         }
+        // in flight before it is launched: it may complete before this returns
+        if (s->in_flight == 0) s->busy_since = Clock::now();
+        s->in_flight += 1;
+        s->launches += 1;
+        s->slot_busy[slot] = 1;
+        lk.unlock();
         int status = beamform_batch_planned((int)gs.size(), gs.data(), as.data(), plans.data(), st);
         if (status == RCABF_OK) status = cudaLaunchHostFunc(st, on_launch_done, L) == cudaSuccess ? RCABF_OK
                                                                                                   : RCABF_ERR_CUDA;
@@ -265,23 +280,15 @@ static bool dispatch_locked(rcabf_server *s)
             // the workspace goes back to the arena
             cudaStreamSynchronize(st);
             cudaGetLastError();
-            const auto now = Clock::now();
-            for (Request *r : L->reqs) finish_locked(s, r, status, now);
+        }
+        lk.lock();
+        if (status != RCABF_OK) {   // (else L is its completion's now)
+            s->launches -= 1;
+            leave_locked(s, L, status);
             delete L;
             s->cv_done.notify_all();
-            continue;
         }
-        for (Request *r : L->reqs) {
-            s->busy_out.insert(r->a.out);
-            if (r->a.mask) s->busy_out.insert(r->a.mask);
-        }
-        if (s->in_flight == 0) s->busy_since = Clock::now();
-        s->in_flight += 1;
-        s->launches += 1;
-        s->slot_busy[slot] = 1;
-        any = true;
     }
-    return any;
 }
 
 static void scheduler(rcabf_server *s)
@@ -299,7 +306,7 @@ static void scheduler(rcabf_server *s)
                 continue;
             }
         }
-        dispatch_locked(s);
+        dispatch(s, lk);
         s->cv.wait_for(lk, std::chrono::milliseconds(5));
     }
 }

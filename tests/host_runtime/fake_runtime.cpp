@@ -5,6 +5,7 @@
 // checked as the device would (a kernel function's shared-memory limit).
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <chrono>
 #include <cmath>
 #include <cstdio>
@@ -12,6 +13,7 @@
 #include <cstring>
 #include <map>
 #include <mutex>
+#include <set>
 #include <string>
 #include <thread>
 #include <vector>
@@ -24,6 +26,8 @@ namespace {
 std::mutex g_mu;
 std::string g_log;
 std::map<std::vector<int>, size_t> g_smem;   // kernel function -> its dynamic shared-memory limit
+std::set<std::vector<int>> g_loaded;         // kernel functions launched so far
+std::atomic<int> g_pending{0};               // host functions enqueued and not yet returned
 int g_copies = 1;
 
 void note(const std::string &s)
@@ -71,9 +75,11 @@ cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
 cudaError_t cudaEventElapsedTime(float *ms, cudaEvent_t, cudaEvent_t) { *ms = 1.0f; return cudaSuccess; }
 cudaError_t cudaLaunchHostFunc(cudaStream_t, cudaHostFn_t fn, void *p)
 {
+    ++g_pending;
     std::thread([fn, p] {
         std::this_thread::sleep_for(std::chrono::milliseconds(20));
         fn(p);
+        --g_pending;
     }).detach();
     return cudaSuccess;
 }
@@ -98,6 +104,13 @@ static cudaError_t launch(const char *name, std::vector<int> f, size_t smem, con
         std::lock_guard<std::mutex> lk(g_mu);
         const auto it = g_smem.find(f);
         if (smem > (it == g_smem.end() ? 48 * 1024 : it->second)) return cudaErrorInvalidValue;
+        if (!g_loaded.insert(f).second) f.clear();
+    }
+    // the first launch of a function may load its module, which waits for all
+    // work in flight, host functions too (here 3 s at most)
+    for (int i = 0; !f.empty() && g_pending.load() > 0; ++i) {
+        if (i == 3000) return cudaErrorLaunchTimeout;
+        std::this_thread::sleep_for(std::chrono::milliseconds(1));
     }
     s += " jobs " + std::to_string(p.n_jobs);
     const FusedJob &J = p.jobs[0];   // what sets the order of its sums

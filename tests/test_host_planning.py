@@ -192,6 +192,15 @@ def test_batch_of_tensor_core_calls_keeps_each_record_length(host):
     assert [line.split("rows ")[1] for line in host.log()] == ["212 of 180", "212 of 180", "332 of 300"]
 
 
+def _server(host, n_streams, batch_window_us):
+    import ctypes as C
+    cfg, srv = L.ServerConfig(), C.c_void_p()
+    cfg.struct_size, cfg.hbm_budget_bytes = C.sizeof(cfg), 1 << 28
+    cfg.n_streams, cfg.max_queue, cfg.max_batch, cfg.batch_window_us = n_streams, 16, 8, batch_window_us
+    assert host.lib.rcabf_server_create(C.byref(cfg), C.byref(srv)) == 0
+    return srv
+
+
 SERVED = [(dict(), 16, F32), (dict(shift=1e-3), 16, F32), (dict(), 31, F32), (dict(), 1, F16), (dict(shift=1e-3), 1, BF16),
           (dict(), 1, F32), (dict(shift=1e-3), 5, F16), (dict(span=30.0), 3, F32), (dict(), 40, F16),
           (dict(tables="ref_compat", interp=("ref6", 3)), 1, F32), (dict(tables="ref_compat", interp=("ref6", 3)), 4, F32),
@@ -204,10 +213,7 @@ def test_server_runs_equal_requests_in_one_launch_with_the_plan_each_has_alone(h
     g = _batch_geometry(host, kw)
     assert host.beamform(g, host.args(g, n_frame, 180, storage=store)) == 0
     alone = host.log()
-    cfg, srv = L.ServerConfig(), C.c_void_p()
-    cfg.struct_size, cfg.hbm_budget_bytes = C.sizeof(cfg), 1 << 28
-    cfg.n_streams, cfg.max_queue, cfg.max_batch, cfg.batch_window_us = 1, 16, 8, 50_000
-    assert host.lib.rcabf_server_create(C.byref(cfg), C.byref(srv)) == 0
+    srv = _server(host, n_streams=1, batch_window_us=50_000)
     tickets = []
     for k in range(3):
         a, t = host.args(g, n_frame, 180, storage=store), C.c_uint64()
@@ -268,3 +274,20 @@ def test_autotuning_times_the_fused_kernel_and_blocks_of_mirrored_copies(host, k
     host.log()
     assert host.lib.rcabf_autotune(g, C.byref(host.args(g, n_frame, 180)), None, 1, C.byref(r)) == 0
     assert want <= {(line.split()[0], line.split()[3]) for line in host.log()}
+
+
+def test_server_launches_kernels_for_the_first_time_while_others_run(host):
+    """The first launch of a kernel waits for the work in flight, whose completion
+    takes the server's lock: the scheduler does not hold it meanwhile."""
+    import ctypes as C
+    g = _batch_geometry(host, {})
+    srv = _server(host, n_streams=4, batch_window_us=0)
+    tickets, st = [], C.c_int()
+    for k, (n_frame, store) in enumerate([(1, F32), (2, F32), (5, F16), (16, F32), (40, F16), (9, BF16)]):
+        a, t = host.args(g, n_frame, 180, storage=store), C.c_uint64()
+        a.out = (k + 2) << 20
+        assert host.lib.rcabf_server_submit(srv, g, C.byref(a), C.byref(t)) == 0
+        tickets.append(t)
+    for t in tickets:
+        assert host.lib.rcabf_server_wait_for(srv, t, 30.0, C.byref(st)) == 0 and st.value == 0
+    assert host.lib.rcabf_server_destroy(srv) == 0
