@@ -150,11 +150,14 @@ struct Launch {
 };
 
 // Requests fused into one launch must run one kernel (few-frame requests on
-// reference tables: one launch slot, a kernel each).
+// reference tables: one launch slot, a kernel each).  Tensor-core requests, which
+// are launched one by one, keep slots of their own: in one slot they would all
+// complete with the last.
 static bool same_variant(const Request *a, const Request *b)
 {
     return a->g->device == b->g->device && a->g->mode == b->g->mode && a->g->kind == b->g->kind &&
-           a->a.storage == b->a.storage && a->plan.kernel == RCABF_KERNEL_FUSED && same_kernel(a->plan, b->plan);
+           a->a.storage == b->a.storage && a->plan.kernel == RCABF_KERNEL_FUSED && !a->plan.tc &&
+           same_kernel(a->plan, b->plan);
 }
 
 static void finish_locked(rcabf_server *s, Request *r, int status, Clock::time_point now)
@@ -170,6 +173,14 @@ static void finish_locked(rcabf_server *s, Request *r, int status, Clock::time_p
     }
     s->last_done = now;
 }
+
+// Work (voxel x element x transmit x frame) that one launch takes of several
+// requests: they complete together, so a launch of large ones holds each back for
+// all.  3e10 is some 25 ms.  The mixed stream of bench.py at 60 requests/s: p50 / p99
+// 0.84 / 1.58 s in 39 launches; without a bound 0.87 / 2.28 s in 27; 2e9 0.94 / 1.63
+// s in 46.  96 equal single-frame FP16 requests (1.7e7 each) on one stream: 0.065 ms
+// a request, 0.23 launched one by one.
+constexpr double FUSED_UNITS = 3e10;
 
 // A launch leaves: its requests are done, its outputs and slot free.
 static void leave_locked(rcabf_server *s, Launch *L, int status)
@@ -233,13 +244,15 @@ static void dispatch(rcabf_server *s, std::unique_lock<std::mutex> &lk)
         // fuse later arrivals that run the same kernel variant and fit
         if (head->plan.kernel == RCABF_KERNEL_FUSED) {
             before.push_back(head);
+            double units = head->units;
             for (auto it = s->queue.begin(); it != s->queue.end() && (int)L->reqs.size() < s->cfg.max_batch;) {
                 Request *r = *it;
                 size_t off = 0;
-                if (same_variant(head, r) && !conflicts(r, before) &&
+                if (same_variant(head, r) && units + r->units <= FUSED_UNITS && !conflicts(r, before) &&
                     s->arena.alloc(r->ws_bytes ? r->ws_bytes : 1, off)) {
                     r->ws_off = off;
                     L->reqs.push_back(r);
+                    units += r->units;
                     before.push_back(r);
                     it = s->queue.erase(it);
                 } else {
