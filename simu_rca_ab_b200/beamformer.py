@@ -302,7 +302,8 @@ class Engine:
                     "rcabf_beamform_host")
 
     def run_batch(self, geoms: list, args: list, workspaces: list, stream=None) -> None:
-        """One persistent fused launch over several acquisitions."""
+        """Several acquisitions: one persistent fused launch per kernel among their
+        plans."""
         n = len(geoms)
         arr = (L.BeamformArgs * n)()
         for i, (g, a, w) in enumerate(zip(geoms, args, workspaces)):

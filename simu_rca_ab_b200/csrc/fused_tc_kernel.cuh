@@ -616,8 +616,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1) fused_tc_kernel(const __grid_co
                 ok = false;
                 o = 0;
             }
-            // a warp none of whose voxels has a tap in this record stores
-            // zero rows without forming weights
+            // a warp none of whose voxels contributes to the record's step
+            // stores zero rows without forming weights (the two records of a
+            // long window are two builds of the same weights)
             const bool warp_any = __any_sync(0xffffffffu, ok);
             float w[TAPS];
             if (warp_any) poly_weights<KIND, 6>(ok ? idx - fl : 0.0f, w);

@@ -25,8 +25,9 @@
 // 128 x 128 x 256, two orientations 257 -> 158 ms; 4 frames of a 256-element probe
 // 361 -> 202 ms; 20 frames, 97 x 95 x 159 47.3 -> 28.5 ms; one frame, 64 x 64 x 128
 // 9.38 -> 0.88 ms; one frame, 32 x 32 x 64, 4 transmits 455 -> 87 us.
-// What bounds it: instruction issue and fixed latencies (8 frames: FMA pipe 58 %
-// busy at 8 and at 12 warps per SM alike; one frame: 48 %, issue 56 %).
+// What bounds it: the FMA pipe with the shared-memory loads that feed it, and
+// fixed latencies (8 frames: FMA pipe 58 % busy at 8 and at 12 warps per SM alike,
+// issue slots 49 %; one frame: 49 % and 52 %).
 // Grids centred on the probe and symmetric transmits: the voxels of half the u
 // (v) axis carry their mirror images as further frames (VBS_MIRROR_*).
 //

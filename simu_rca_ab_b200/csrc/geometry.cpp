@@ -524,8 +524,8 @@ void rcabf_geometry::index_steps(float &z, float &u, float &v)
 {
     std::lock_guard<std::mutex> lk(mu);
     if (steps[0] < 0.f) {
-        // |difference| along z and along a of every 5th entry of an odd stride
-        // of rows (NaN, an element outside its aperture, never wins a max)
+        // |difference| along z and along a of every 5th entry of about 24 to 48
+        // evenly spaced rows (NaN, an element outside its aperture, never wins a max)
         auto scan = [&](const std::vector<float> &tab, int64_t rows, int64_t n_a, float &dz, float &da) {
             dz = da = 0.f;
             const int64_t rs = std::max<int64_t>(1, rows / 24);

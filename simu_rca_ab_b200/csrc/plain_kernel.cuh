@@ -142,10 +142,10 @@ __global__ void __launch_bounds__(256) plain_das_kernel(const __grid_constant__ 
 // kernel's, in its order: the same bits.
 // The data set's call (17 depths, 64 elements, 16 transmits, 100 frames) has
 // 17408 setups: one thread per (voxel, element) filled 5 CTAs and took 2.0 ms;
-// with every transmit and frame on a thread of its own (ranges form on calls of
-// twice its size) the kernel takes 53 us, the call 0.13 ms.  It touches the taps
-// only: 1.7 M reads of 48 bytes, 84 MB of the 0.43 GB of channel data, in
-// sectors of 32 bytes 110 to 170 MB, 2 to 3 TB/s.
+// with every transmit and frame on a thread of its own (ranges of frames form
+// from 1.4 times its size on) the kernel takes 53 to 72 us, the call 0.13 ms.  It
+// touches the taps only: 1.7 M reads of 48 bytes, 84 MB of the 0.43 GB of channel data,
+// in sectors of 32 bytes 110 to 170 MB, 2 to 3 TB/s.
 template <int MODE, int KIND, int IQ>
 __global__ void __launch_bounds__(256) pc_das_kernel(const __grid_constant__ PlainParams prm)
 {
