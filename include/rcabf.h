@@ -340,8 +340,9 @@ int rcabf_autotune(const rcabf_geometry *g, const rcabf_beamform_args *a, void *
  * caller-owned device buffers and a geometry handle, which must stay valid
  * until the request completes; their workspace comes from the arena.
  * Requests are admitted in arrival order as slots and arena space free up;
- * queued requests whose plans run the same kernel variant are fused into one
- * persistent launch.  A request whose output or mask is written by a launch
+ * queued requests whose plans run one kernel function are fused into one
+ * persistent launch, up to a bounded amount of work since they complete
+ * together; each gives the bits that it gives alone.  A request whose output or mask is written by a launch
  * in flight, or by an earlier queued request, waits for it, so requests that
  * accumulate into one buffer apply in arrival order. */
 typedef struct rcabf_server rcabf_server;
